@@ -67,7 +67,7 @@ def build_oracle(reference_dir: str | None = None) -> None:
     PERFT_REFERENCE_DIR environment variable)."""
     subprocess.run(["make", "-s", "-C", os.path.join(ROOT, "oracle")], check=True)
     ref = reference_dir or os.environ.get("PERFT_REFERENCE_DIR")
-    if ref and os.path.isdir(ref):
+    if ref and os.path.exists(os.path.join(ref, "perft.cu")):  # an empty directory holds no sources
         subprocess.run(["make", "-s", "-C", os.path.join(ROOT, "oracle"), "ref", "REF=" + ref], check=True)
 
 

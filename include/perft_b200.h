@@ -129,6 +129,13 @@ int pb_u128_text(const pb_u128 *v, char *buf, size_t len);
  * *mismatches = disagreements. */
 int pb_selftest_listed_counts(const pb_pos *pos, int n, uint64_t *checked, uint64_t *mismatches);
 
+/* Self-test of the folded counting (leaf kernel 6), on the host: perft(2) of
+ * each position by folding against making and counting every move, both
+ * counting conventions.  No counterpart in the reference.  *checked = moves
+ * of the positions, *made = those that folding leaves to be made and counted,
+ * *mismatches = positions whose sums or move numbers differ. */
+int pb_selftest_fold(const pb_pos *pos, int n, uint64_t *checked, uint64_t *made, uint64_t *mismatches);
+
 /* Replaces perft_cpu_dispatch (launcher.cu:807-816): host-only perft. */
 int pb_perft_cpu(pb_ctx *ctx, const pb_pos *pos, int depth, uint64_t *count);
 
@@ -167,7 +174,7 @@ typedef struct {
     uint64_t leaf_edges;       /* edges the leaf kernel took (one perft(2) each) */
     uint64_t leaf_positions;   /* positions the leaf kernel counted (move-count calls) */
     uint64_t nodes;            /* the perft result of the call */
-    uint32_t kernels;          /* kernel launches of the call */
+    uint32_t kernels;          /* kernel launches of the call (a leaf counts once) */
     uint32_t levels;           /* BFS expand levels */
     uint64_t level_sizes[16];  /* edges per level, level 0 = root moves */
     uint64_t h2d_bytes;        /* host-to-device bytes copied */
@@ -180,16 +187,18 @@ typedef struct {
  * 2 = cooperative (grandchildren spread over the CTA), 3 = in-check children
  * deferred to a second pass, 4 = one edge per thread with the CTA's children
  * ranked by move count first, 5 = as 4 with each child's own-piece squares
- * listed once for all of its grandchild counts, 6 = as 5 with four children
- * per thread ranked across the CTA and dealt to the warps in light/heavy
- * chunk pairs (default, with 1024-thread CTAs); batched, planned and table
+ * listed once for all of its grandchild counts, 6 = folded counting: most
+ * grandchildren are summed by set arithmetic, the rest made and counted one
+ * per thread from a queue in the BFS arena (default; an arena without room for
+ * the queue runs 5 instead); batched and planned leaves follow 4 to 6, table
  * leaves rank their children for 4 to 6 and list pieces for 5 and 6;
  * leaf_blocks_per_sm: persistent grid of the cooperative leaf. */
 typedef struct {
     int leaf_kernel;
     int leaf_blocks_per_sm;
-    int leaf_threads;   /* CTA size of leaf kernels 1, 3 to 6: 128, 256, 512 (not 3) or, with leaf
-                           kernel 6 only, 1024 (default; other kernels then run 256) */
+    int leaf_threads;   /* CTA size of leaf kernels 1, 3 to 5: 128, 256, 512 (not 3); leaf kernel 6
+                           sizes its own CTAs and also takes 1024 (default; other kernels then run
+                           256) */
     int gen_threads;    /* CTA size of the staged generator: 64 or 128 (default); stages 64 moves per thread */
     int leaf_fuse;      /* plies fused in the leaf kernel: 2 (default) or 1 (one more BFS level) */
     int tt_replace;     /* device TT replacement: 1 = always overwrite (default, tt.h:60-70),

@@ -133,6 +133,8 @@ def _load() -> ctypes.CDLL:
         "pb_random_playouts": (ctypes.c_int, [ctypes.c_uint64, ctypes.c_int, ctypes.c_int, ctypes.c_int, P(Pos),
                                                P(ctypes.c_int)]),
         "pb_selftest_listed_counts": (ctypes.c_int, [P(Pos), ctypes.c_int, P(ctypes.c_uint64), P(ctypes.c_uint64)]),
+        "pb_selftest_fold": (ctypes.c_int, [P(Pos), ctypes.c_int, P(ctypes.c_uint64), P(ctypes.c_uint64),
+                                            P(ctypes.c_uint64)]),
         "pb_u128_add": (None, [P(U128), P(U128)]),
         "pb_u128_text": (ctypes.c_int, [P(U128), ctypes.c_char_p, ctypes.c_size_t]),
         "pb_device_count": (ctypes.c_int, []),
@@ -252,6 +254,18 @@ def selftest_listed_counts(positions: Sequence[Pos]) -> Tuple[int, int]:
     if rc != PB_OK:
         raise PerftError(rc, "listed-count self-test")
     return checked.value, bad.value
+
+
+def selftest_fold(positions: Sequence[Pos]) -> Tuple[int, int, int]:
+    """(moves, moves made and counted, mismatches) of the folded perft(2)
+    against the counted one, on the host, over the positions and both
+    counting conventions."""
+    arr = pack_positions(positions)
+    checked, made, bad = ctypes.c_uint64(0), ctypes.c_uint64(0), ctypes.c_uint64(0)
+    rc = lib.pb_selftest_fold(arr, len(arr), ctypes.byref(checked), ctypes.byref(made), ctypes.byref(bad))
+    if rc != PB_OK:
+        raise PerftError(rc, "folded-count self-test")
+    return checked.value, made.value, bad.value
 
 
 def u128_add(acc: int, v: int) -> int:
@@ -481,9 +495,9 @@ class Engine:
         leaf_kernel 1 = one edge per thread, 2 = cooperative, 3 = in-check
         children deferred, 4 = children ranked by move count,
         5 = ranked with each child's own-piece squares listed once,
-        6 = as 5 with four children per thread balanced across the warps
-        (default); leaf_threads 128/256/512, or 1024 with leaf kernel 6
-        (default); gen_threads 64/128; leaf_fuse 1/2;
+        6 = folded counting (default); leaf_threads 128/256/512, or 1024 with
+        leaf kernel 6, which sizes its own CTAs (default); gen_threads 64/128;
+        leaf_fuse 1/2;
         tt_replace 1 = always overwrite, 2 = two-slot size priority;
         planned_leaf 1 = grid over the planned capacity (default),
         2 = persistent work-queue leaf; host_driver 1 = depth-first tree

@@ -2,9 +2,8 @@
 
 Candidates: leaf kernel (one edge per thread / cooperative / one edge per
 thread with the CTA's children ranked by move count / ranked with each
-child's own-piece squares listed once / the same with four children per
-thread balanced across the warps), the leaf's CTA size
-(128/256/512), the staged generator's CTA size and tile (64 or 128
+child's own-piece squares listed once / folded counting), the leaf's CTA size
+(128/256/512; folded counting sizes its own), the staged generator's CTA size and tile (64 or 128
 threads, 64 moves staged per thread) and the leaf fuse depth (two plies fused
 in the leaf, or one with an extra BFS level).  Each candidate runs perft 7
 of the bench position on the GPU (device time from the engine's CUDA events, median of 3);
@@ -47,9 +46,8 @@ def candidates() -> List[Dict[str, int]]:
     for lk in (4, 5):
         for gt in (64, 128):
             out.append({"leaf_kernel": lk, "leaf_threads": 256, "gen_threads": gt, "leaf_fuse": 2})
-    for lt in (512, 1024):
-        for gt in (64, 128):
-            out.append({"leaf_kernel": 6, "leaf_threads": lt, "gen_threads": gt, "leaf_fuse": 2})
+    for gt in (64, 128):
+        out.append({"leaf_kernel": 6, "leaf_threads": 1024, "gen_threads": gt, "leaf_fuse": 2})
     return out
 
 

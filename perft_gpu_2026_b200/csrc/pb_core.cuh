@@ -76,6 +76,7 @@ struct Tables {
     u64 bishop_empty[64];
     u64 between[64][64];
     u64 line[64][64];
+    u64 beyond[64][64];  // [s][t]: the squares past t on the ray from s through t
     // Squares from which a rook / bishop on an empty board attacks the zone
     // of a king on that square: its 3x3 block and, for e1/e8, the castling
     // squares c..g of its back rank.

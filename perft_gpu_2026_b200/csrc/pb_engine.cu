@@ -27,6 +27,7 @@
 #include "pb_tables.cuh"
 #include "pb_util.cuh"
 #include "pb_kernels.cuh"
+#include "pb_fold_leaf.cuh"
 #include "pb_tt.cuh"
 #include "pb_devtt.cuh"
 #include "pb_mlp_host.cuh"
@@ -175,33 +176,84 @@ struct Arena {
         off += bytes;
         return p;
     }
+    // what is left, as one array (nothing is taken)
+    template <class T> T *rest(u64 *n) const
+    {
+        *n = (cap - std::min(off, cap)) / sizeof(T);
+        return reinterpret_cast<T *>(base + off);
+    }
 };
 
 inline unsigned grid_for(u64 n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
-// Leaf mode of the batched, planned and table leaves (grandchild_counts):
-// 3 for leaf kernel 6 (ranked, listed pieces, balanced warps), 2 for 5
-// (ranked, listed pieces), 1 for 4 (ranked), else 0.
+// Leaf mode of the batched, planned and table leaves: 3 for leaf kernel 6
+// (folded counting), 2 for 5 (ranked, listed pieces), 1 for 4 (ranked), else 0.
 inline int leaf_mode(const pb_ctx *ctx)
 {
     return ctx->tuning.leaf_kernel == 6 ? 3 : ctx->tuning.leaf_kernel == 5 ? 2 : ctx->tuning.leaf_kernel == 4 ? 1 : 0;
 }
 
-// CTA size of a balanced leaf over n edges (PB_BALANCED_K per thread): the
-// tuned size, halved down to 256 while the grid would have fewer than 8 CTAs
-// per SM (a small launch of big CTAs leaves its last wave half empty).
-inline int balanced_threads(const pb_ctx *ctx, u64 n, int tuned)
+// The folded leaf's queue is what the arena has left behind the levels.
+// Without this much (a few full chunks even at 256 queued moves per edge) the
+// leaf counts every move on the spot (the listed leaf), which needs no memory.
+constexpr u64 FOLD_MIN_ITEMS = 256 * 1024;
+inline FoldQueue fold_queue(const pb_ctx *ctx, const Arena &ar)
 {
-    int t = tuned;
-    while (t > 256 && n < (u64)PB_BALANCED_K * (u64)t * 8u * (u64)ctx->num_sms) t /= 2;
-    return t;
+    FoldQueue q{};
+    q.items = ar.rest<u64>(&q.cap);
+    q.cursor = ctx->d_counter + 4;
+    return q;
 }
-// Below this many edges even 256-thread balanced CTAs would not give every SM
-// 8 of them: such small leaves run one edge per thread (the listed leaf) so
-// the launch still covers the GPU (one perft-5 root has about 3e4 edges).
-inline bool balanced_fits(const pb_ctx *ctx, u64 n)
+inline bool fold_fits(const FoldQueue &q) { return q.cap >= FOLD_MIN_ITEMS; }
+
+// Edges per chunk: all of them if the queue holds 64 moves per edge (2 to 12
+// are queued on playouts, 24 in endgames of pieces alone), else that many, but
+// at 16 per edge still chunks that fill the GPU.  A chunk whose queue turns
+// out too short makes the leaf run again with `careful`: 256 moves per edge,
+// the size of every move list, always fit.
+inline u64 fold_chunk(const FoldQueue &q, u64 n, bool careful)
 {
-    return n >= (u64)PB_BALANCED_K * 256u * 8u * (u64)ctx->num_sms;
+    if (careful) return q.cap / MAX_MOVES;
+    return std::min(n, std::max(q.cap / 64, std::min<u64>(q.cap / 16, 1u << 20)));
+}
+
+// Zeroes the counters and the first chunk's queue cursor (one 64-byte block).
+inline cudaError_t reset_counters(pb_ctx *ctx) { return cudaMemsetAsync(ctx->d_counter, 0, 64, ctx->stream); }
+
+// The folded leaf over e.n edges; `overflow` is the error bit of a queue that
+// was too short.  The caller has reset the counters.
+template <int C, bool S, bool ROOTED>
+cudaError_t launch_fold_t(pb_ctx *ctx, const LeafEdges &e, const FoldQueue &q, bool careful, unsigned long long *rc,
+                          u32 overflow)
+{
+    cudaStream_t s = ctx->stream;
+    const u64 chunk = fold_chunk(q, e.n, careful);
+    for (u64 first = 0; first < e.n; first += chunk) {
+        if (first) {
+            cudaError_t me = cudaMemsetAsync(q.cursor, 0, sizeof(unsigned long long), s);
+            if (me != cudaSuccess) return me;
+        }
+        const u64 m = std::min(chunk, e.n - first);
+        if (m < (u64)ctx->num_sms * FOLD_THREADS_PER_SM)
+            k_fold<C, S, FOLD_SMALL_THREADS, ROOTED><<<grid_for(m, FOLD_SMALL_THREADS), FOLD_SMALL_THREADS, 0, s>>>(
+                e, first, m, q, rc, ctx->d_counter, ctx->d_err);
+        else
+            k_fold<C, S, FOLD_THREADS, ROOTED><<<grid_for(m, FOLD_THREADS), FOLD_THREADS, 0, s>>>(
+                e, first, m, q, rc, ctx->d_counter, ctx->d_err);
+        // at most a few queued moves per thread of a small launch
+        const unsigned g = (unsigned)std::min<u64>((u64)ctx->num_sms * 4, grid_for(m * 16, 256));
+        k_fold_count<C, S, ROOTED><<<g, 256, 0, s>>>(e, q, rc, ctx->d_counter, overflow, ctx->d_err);
+    }
+    return cudaGetLastError();
+}
+template <bool ROOTED>
+cudaError_t launch_fold(pb_ctx *ctx, int c, bool strict, const LeafEdges &e, const FoldQueue &q, bool careful,
+                        unsigned long long *rc, u32 overflow)
+{
+    if (c == WHITE) return strict ? launch_fold_t<WHITE, true, ROOTED>(ctx, e, q, careful, rc, overflow)
+                                  : launch_fold_t<WHITE, false, ROOTED>(ctx, e, q, careful, rc, overflow);
+    return strict ? launch_fold_t<BLACK, true, ROOTED>(ctx, e, q, careful, rc, overflow)
+                  : launch_fold_t<BLACK, false, ROOTED>(ctx, e, q, careful, rc, overflow);
 }
 
 // NVTX range for profilers (header-only NVTX v3: free unless a tool attaches):
@@ -233,21 +285,7 @@ int launch_leaf_t(pb_ctx *ctx, const Board *b, const uint8_t *st, const u32 *pi,
         PB_CUDA(cudaGetLastError());
         return PB_OK;
     }
-    if (ctx->tuning.leaf_kernel == 6 && balanced_fits(ctx, n)) {
-        // PB_BALANCED_K edges per thread
-        const int lt = balanced_threads(ctx, n, ctx->tuning.leaf_threads);
-        const u64 per = (u64)PB_BALANCED_K * (u64)lt;
-        const unsigned g = (unsigned)((n + per - 1) / per);
-        switch (lt) {
-        case 128: k_leaf2_balanced<C, S, 128><<<g, 128, 0, s>>>(b, st, pi, mv, n, npar, ctx->d_counter); break;
-        case 512: k_leaf2_balanced<C, S, 512><<<g, 512, 0, s>>>(b, st, pi, mv, n, npar, ctx->d_counter); break;
-        case 1024: k_leaf2_balanced<C, S, 1024><<<g, 1024, 0, s>>>(b, st, pi, mv, n, npar, ctx->d_counter); break;
-        default: k_leaf2_balanced<C, S, 256><<<g, 256, 0, s>>>(b, st, pi, mv, n, npar, ctx->d_counter); break;
-        }
-        PB_CUDA(cudaGetLastError());
-        return PB_OK;
-    }
-    if (ctx->tuning.leaf_kernel == 5 || ctx->tuning.leaf_kernel == 6) {
+    if (ctx->tuning.leaf_kernel == 5 || ctx->tuning.leaf_kernel == 6) {  // 6: an arena without room for its queue
         switch (ctx->tuning.leaf_kernel == 6 ? 256 : ctx->tuning.leaf_threads) {
         case 128: k_leaf2_listed<C, S, 128><<<grid_for(n, 128), 128, 0, s>>>(b, st, pi, mv, n, npar, ctx->d_counter); break;
         case 512: k_leaf2_listed<C, S, 512><<<grid_for(n, 512), 512, 0, s>>>(b, st, pi, mv, n, npar, ctx->d_counter); break;
@@ -407,22 +445,32 @@ int bfs_perft(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth,
         n = next;
         c = 1 - c;
     }
-    PB_CUDA(cudaMemsetAsync(ctx->d_counter, 0, 2 * sizeof(unsigned long long), s));
-    if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[1], s));
-    int rc;
-    {
-        NvtxRange nvtx_leaf("leaf");
-        rc = launch_leaf(ctx, c, strict, cur_b, cur_s, epi, emv, n, n_par);
+    const FoldQueue queue = fold_queue(ctx, ar);
+    const bool fold = ctx->tuning.leaf_kernel == 6 && fuse == 2 && fold_fits(queue);
+    for (int attempt = 0;; attempt++) {
+        PB_CUDA(reset_counters(ctx));
+        if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[1], s));
+        {
+            NvtxRange nvtx_leaf("leaf");
+            if (fold) {
+                const LeafEdges e{cur_b, cur_s, nullptr, epi, emv, n, n_par, nullptr, nullptr};
+                PB_CUDA(launch_fold<false>(ctx, c, strict, e, queue, attempt > 0, nullptr, DEVERR_QUEUE));
+            } else {
+                int rc = launch_leaf(ctx, c, strict, cur_b, cur_s, epi, emv, n, n_par);
+                if (rc != PB_OK) return rc;
+            }
+        }
+        PB_CUDA(cudaGetLastError());
+        if (ctx->timing) {
+            PB_CUDA(cudaEventRecord(ctx->ev[2], s));
+            PB_CUDA(cudaEventRecord(ctx->ev[3], s));
+        }
+        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, 2 * sizeof(u64), cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned + 2, ctx->d_err, sizeof(u32), cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaStreamSynchronize(s));
+        if ((u32)ctx->h_pinned[2] != DEVERR_QUEUE || attempt > 0) break;
+        PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));  // a queue was too short
     }
-    if (rc != PB_OK) return rc;
-    PB_CUDA(cudaGetLastError());
-    if (ctx->timing) {
-        PB_CUDA(cudaEventRecord(ctx->ev[2], s));
-        PB_CUDA(cudaEventRecord(ctx->ev[3], s));
-    }
-    PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, 2 * sizeof(u64), cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaMemcpyAsync(ctx->h_pinned + 2, ctx->d_err, sizeof(u32), cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaStreamSynchronize(s));
     if ((u32)ctx->h_pinned[2]) return fail(ctx, PB_ERR_DEVICE, "kernel reported a device error");
     *out = ctx->h_pinned[0];
     stats.kernels += 1;
@@ -866,7 +914,6 @@ int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth,
     PB_CUDA(cudaMemcpyAsync(r0, iota.data(), sizeof(u32) * n, cudaMemcpyHostToDevice, s));
     PB_CUDA(cudaMemsetAsync(rc, 0, sizeof(unsigned long long) * n, s));
     PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));
-    PB_CUDA(cudaMemsetAsync(ctx->d_counter, 0, 2 * sizeof(unsigned long long), s));
     stats.h2d_bytes += (sizeof(Board) + 1 + 4) * n;
     if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[0], s));
     if (depth == 1) {
@@ -972,69 +1019,70 @@ int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth,
         epi = npi;
         ne = next;
     }
-    if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[1], s));
-    if (ne) {
-        if (depth == 2) {
-            unsigned g = grid_for(ne, 256);
-            if (c == WHITE) {
-                if (strict) k_leaf1_rooted<WHITE, true><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
-                else k_leaf1_rooted<WHITE, false><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
-            } else {
-                if (strict) k_leaf1_rooted<BLACK, true><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
-                else k_leaf1_rooted<BLACK, false><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
-            }
-        } else {
-            unsigned g = grid_for(ne, PB_LEAF_THREADS);
-            const int mode = (leaf_mode(ctx) == 3 && !balanced_fits(ctx, ne)) ? 2 : leaf_mode(ctx);
-            const int bt = balanced_threads(ctx, ne, 1024);
-            const unsigned gb = (unsigned)((ne + (u64)PB_BALANCED_K * bt - 1) / ((u64)PB_BALANCED_K * bt));
-#define PB_ROOTED_LEAF(CC, SS)                                                                                   \
-    if (mode == 3 && bt == 1024)                                                                                 \
-        k_leaf2_rooted_balanced<CC, SS, 1024><<<gb, 1024, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc,  \
-                                                                  ctx->d_counter);                               \
-    else if (mode == 3 && bt == 512)                                                                             \
-        k_leaf2_rooted_balanced<CC, SS, 512><<<gb, 512, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc,    \
-                                                                ctx->d_counter);                                 \
-    else if (mode == 3)                                                                                          \
-        k_leaf2_rooted_balanced<CC, SS, 256><<<gb, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc,    \
-                                                                ctx->d_counter);                                 \
-    else if (mode == 2)                                                                                          \
-        k_leaf2_rooted<CC, SS, 2><<<g, PB_LEAF_THREADS, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc,    \
-                                                                ctx->d_counter);                                 \
-    else if (mode == 1)                                                                                          \
-        k_leaf2_rooted<CC, SS, 1><<<g, PB_LEAF_THREADS, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc,    \
-                                                                ctx->d_counter);                                 \
-    else                                                                                                         \
-        k_leaf2_rooted<CC, SS, 0><<<g, PB_LEAF_THREADS, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc,    \
-                                                                ctx->d_counter);
-            if (c == WHITE) {
-                if (strict) {
-                    PB_ROOTED_LEAF(WHITE, true)
-                } else {
-                    PB_ROOTED_LEAF(WHITE, false)
-                }
-            } else {
-                if (strict) {
-                    PB_ROOTED_LEAF(BLACK, true)
-                } else {
-                    PB_ROOTED_LEAF(BLACK, false)
-                }
-            }
-#undef PB_ROOTED_LEAF
-        }
-        PB_CUDA(cudaGetLastError());
-        stats.kernels += 1;
-    }
-    if (ctx->timing) {
-        PB_CUDA(cudaEventRecord(ctx->ev[2], s));
-        PB_CUDA(cudaEventRecord(ctx->ev[3], s));
-    }
+    const FoldQueue queue = fold_queue(ctx, ar);
+    const bool fold = leaf_mode(ctx) == 3 && depth > 2 && fold_fits(queue);
     std::vector<unsigned long long> tmp(n);
-    PB_CUDA(cudaMemcpyAsync(tmp.data(), rc, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, 2 * sizeof(u64), cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaMemcpyAsync(ctx->h_pinned + 2, ctx->d_err, sizeof(u32), cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaStreamSynchronize(s));
+    for (int attempt = 0;; attempt++) {
+        PB_CUDA(reset_counters(ctx));
+        if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[1], s));
+        if (ne) {
+            if (depth == 2) {
+                unsigned g = grid_for(ne, 256);
+                if (c == WHITE) {
+                    if (strict) k_leaf1_rooted<WHITE, true><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
+                    else k_leaf1_rooted<WHITE, false><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
+                } else {
+                    if (strict) k_leaf1_rooted<BLACK, true><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
+                    else k_leaf1_rooted<BLACK, false><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
+                }
+            } else if (fold) {
+                const LeafEdges e{cur_b, cur_s, cur_r, epi, emv, ne, n_par, nullptr, nullptr};
+                PB_CUDA(launch_fold<true>(ctx, c, strict, e, queue, attempt > 0, rc, DEVERR_QUEUE));
+            } else {
+                unsigned g = grid_for(ne, PB_LEAF_THREADS);
+                const int mode = std::min(leaf_mode(ctx), 2);
+#define PB_ROOTED_LEAF(CC, SS)                                                                                   \
+        if (mode == 2)                                                                                               \
+            k_leaf2_rooted<CC, SS, 2><<<g, PB_LEAF_THREADS, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc,    \
+                                                                    ctx->d_counter);                                 \
+        else if (mode == 1)                                                                                          \
+            k_leaf2_rooted<CC, SS, 1><<<g, PB_LEAF_THREADS, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc,    \
+                                                                    ctx->d_counter);                                 \
+        else                                                                                                         \
+            k_leaf2_rooted<CC, SS, 0><<<g, PB_LEAF_THREADS, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc,    \
+                                                                    ctx->d_counter);
+                if (c == WHITE) {
+                    if (strict) {
+                        PB_ROOTED_LEAF(WHITE, true)
+                    } else {
+                        PB_ROOTED_LEAF(WHITE, false)
+                    }
+                } else {
+                    if (strict) {
+                        PB_ROOTED_LEAF(BLACK, true)
+                    } else {
+                        PB_ROOTED_LEAF(BLACK, false)
+                    }
+                }
+#undef PB_ROOTED_LEAF
+            }
+            PB_CUDA(cudaGetLastError());
+        }
+        if (ctx->timing) {
+            PB_CUDA(cudaEventRecord(ctx->ev[2], s));
+            PB_CUDA(cudaEventRecord(ctx->ev[3], s));
+        }
+        PB_CUDA(cudaMemcpyAsync(tmp.data(), rc, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, 2 * sizeof(u64), cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned + 2, ctx->d_err, sizeof(u32), cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaStreamSynchronize(s));
+        if ((u32)ctx->h_pinned[2] != DEVERR_QUEUE || attempt > 0) break;
+        // a queue was too short: the leaf again, in chunks that always fit
+        PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));
+        PB_CUDA(cudaMemsetAsync(rc, 0, sizeof(unsigned long long) * n, s));
+    }
     if ((u32)ctx->h_pinned[2]) return fail(ctx, PB_ERR_DEVICE, "batched leaf reported a device error");
+    if (ne) stats.kernels += 1;
     for (u64 i = 0; i < n; i++) out[i] = tmp[i];
     stats.leaf_edges += ne;
     stats.leaf_positions += ctx->h_pinned[1];
@@ -1106,22 +1154,6 @@ void launch_leaf_grid_t(cudaStream_t s, const Board *b, const uint8_t *st, const
 }
 // Leaf of a planned batch: the grid leaf over the planned capacity, or the
 // persistent work-queue leaf (queue).
-// Balanced leaf over a planned level: the grid covers the capacity.
-template <int C, bool S>
-void launch_leaf_balanced_dev(cudaStream_t s, int sms, const Board *b, const uint8_t *st, const u32 *r,
-                              const u32 *pi, const uint16_t *mv, const u64 *n_dev, u64 cap, const u64 *npar_dev,
-                              u64 npar_cap, unsigned long long *rc, unsigned long long *counter, u32 *err)
-{
-    const bool big = cap >= (u64)PB_BALANCED_K * 1024u * 8u * (u64)sms;
-    const u64 per = (u64)PB_BALANCED_K * (big ? 1024u : 256u);
-    const unsigned grid = (unsigned)std::max<u64>((cap + per - 1) / per, 1);
-    if (big)
-        k_leaf2_rooted_balanced_dev<C, S, 1024><<<grid, 1024, 0, s>>>(b, st, r, pi, mv, n_dev, cap, npar_dev, npar_cap,
-                                                                      rc, counter, err);
-    else
-        k_leaf2_rooted_balanced_dev<C, S, 256><<<grid, 256, 0, s>>>(b, st, r, pi, mv, n_dev, cap, npar_dev, npar_cap,
-                                                                    rc, counter, err);
-}
 template <int C, bool S, int MODE>
 void launch_leaf_planned_t(bool queue, cudaStream_t s, int sms, const Board *b, const uint8_t *st, const u32 *r,
                            const u32 *pi, const uint16_t *mv, const u64 *n_dev, u64 cap, const u64 *npar_dev,
@@ -1140,9 +1172,7 @@ void launch_leaf_queue(int mode, bool queue, cudaStream_t s, int sms, const Boar
                        const u64 *npar_dev, u64 npar_cap, unsigned long long *cursor, unsigned long long *rc,
                        unsigned long long *counter, u32 *err)
 {
-    if (mode == 3 && !queue && cap >= (u64)PB_BALANCED_K * 256u * 8u * (u64)sms)
-        launch_leaf_balanced_dev<C, S>(s, sms, b, st, r, pi, mv, n_dev, cap, npar_dev, npar_cap, rc, counter, err);
-    else if (mode >= 2)
+    if (mode >= 2)
         launch_leaf_planned_t<C, S, 2>(queue, s, sms, b, st, r, pi, mv, n_dev, cap, npar_dev, npar_cap, cursor, rc,
                                        counter, err);
     else if (mode == 1)
@@ -1206,7 +1236,7 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
     PB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(g.rc, 0, sizeof(unsigned long long) * n, s);
     cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s);
-    cudaMemsetAsync(ctx->d_counter, 0, 2 * sizeof(unsigned long long), s);
+    reset_counters(ctx);
     cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), s);
     // level 0: root move counts -> E_1
     k_count_positions<WHITE, true><<<grid_for(n, 256), 256, 0, s>>>(g.b0, g.s0, n, cnt0);
@@ -1258,6 +1288,10 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
         else
             k_leaf1_rooted_dev<WHITE, false><<<gl, 256, 0, s>>>(pb_, ps, pr, L[1].pi, L[1].mv, d_n0 + 1, lcap, npar,
                                                                 npar_cap, g.rc, ctx->d_err);
+    } else if (g.mode == 3 && !g.queue && fold_fits(fold_queue(ctx, ar))) {
+        // a queue too short counts as an outgrown plan
+        const LeafEdges e{pb_, ps, pr, L[nlev].pi, L[nlev].mv, lcap, npar_cap, d_n0 + nlev, npar};
+        launch_fold<true>(ctx, c, g.strict, e, fold_queue(ctx, ar), false, g.rc, DEVERR_OVERFLOW);
     } else if (c == WHITE) {
         if (g.strict)
             launch_leaf_queue<WHITE, true>(g.mode, g.queue, s, ctx->num_sms, pb_, ps, pr, L[nlev].pi, L[nlev].mv, d_n0 + nlev, lcap, npar,
@@ -1790,6 +1824,55 @@ u64 check_listed_t(const Board &y, u32 ys, u64 *checked)
     return bad;
 }
 
+// Folded counting against making and counting every move, on position `y`
+// (side Z to move), both counting conventions; returns the disagreements.
+struct CountSink {
+    const Board &b;
+    u32 st;
+    bool strict;
+    u64 total;
+    u32 n;
+    template <int Z> void count(uint16_t m)
+    {
+        Board g = b;
+        u32 gs = st;
+        make_move<Z>(g, gs, m);
+        total += host_count(g, gs, 1 - Z, strict);
+        n++;
+    }
+};
+template <int Z>
+struct FoldSink : CountSink {
+    void set(int from, u64 t)
+    {
+        for (; t; t &= t - 1) count<Z>(make_move_code(from, lsb(t), MF_QUIET));
+    }
+    void one(uint16_t m, bool promotes)
+    {
+        if (!promotes) count<Z>(m);
+        for (int k = 0; promotes && k < 4; k++) count<Z>((uint16_t)(m | (MF_PROMO + k) << 12));
+    }
+};
+template <int Z>
+u64 check_fold_t(const Board &y, u32 ys, u64 *checked, u64 *made)
+{
+    u64 bad = 0;
+    for (int strict = 0; strict < 2; strict++) {
+        uint16_t mv[MAX_MOVES];
+        ArraySink all{mv, 0};
+        gen_moves<Z>(y, ys, all);
+        CountSink want{y, ys, strict != 0, 0, 0};
+        for (int k = 0; k < all.n; k++) want.count<Z>(mv[k]);
+        FoldSink<Z> sink{{y, ys, strict != 0, 0, 0}};
+        u32 simple = 0;
+        const u32 sum = strict ? fold_child<Z, true>(y, ys, sink, &simple) : fold_child<Z, false>(y, ys, sink, &simple);
+        bad += sum + sink.total != want.total || simple + sink.n != want.n;
+        *checked += want.n;
+        *made += sink.n;
+    }
+    return bad;
+}
+
 // Launch depth: the deepest GPU call whose BFS levels fit half the arena,
 // from the root's branching factor (estimateLaunchDepth, launcher.cu:533-562).
 int estimate_launch_depth(pb_ctx *ctx, const Board &b, u32 st, int c)
@@ -2010,6 +2093,22 @@ int pb_selftest_listed_counts(const pb_pos *pos, int n, uint64_t *checked, uint6
                                              : check_listed_t<BLACK>(y, pos[i].state, &c);
         *checked += c;
     }
+    return PB_OK;
+}
+
+int pb_selftest_fold(const pb_pos *pos, int n, uint64_t *checked, uint64_t *made, uint64_t *mismatches)
+{
+    if (!pos || n < 0 || !checked || !made || !mismatches) return PB_ERR_ARG;
+    build_host_tables();
+    u64 c = 0, m = 0, bad = 0;
+    for (int i = 0; i < n; i++) {
+        const Board y = to_board(pos[i]);
+        bad += pos[i].color == WHITE ? check_fold_t<WHITE>(y, pos[i].state, &c, &m)
+                                     : check_fold_t<BLACK>(y, pos[i].state, &c, &m);
+    }
+    *checked = c;
+    *made = m;
+    *mismatches = bad;
     return PB_OK;
 }
 

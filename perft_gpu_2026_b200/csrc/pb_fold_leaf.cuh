@@ -1,0 +1,198 @@
+// pb_fold_leaf.cuh - the fused two-ply leaf on folded counting (pb_fold.cuh),
+// leaf kernel 6 and the default leaf of every path without tables.
+//
+// Two kernels per chunk of edges: k_fold makes each edge's child, sums its
+// simple moves (fold_child) and appends its other moves to a queue in device
+// memory; k_fold_count makes the queued moves and counts each of them in full,
+// one per thread.  Both are bound by integer issue.  The queue between them
+// costs 16 B of traffic per queued move (two per child on the benchmark's
+// leaves, seven on middle-game playouts) and buys full warps in both halves,
+// no barriers, and 55 + 20 KB of code instead of one kernel whose warps fetch
+// from both at once (one kernel with a shared-memory queue and a barrier
+// between the halves: 10.9 ms against 8.15 ms on the benchmark's leaves).
+//
+// Measured on B200 against the leaf that makes and counts every move
+// (balanced, listed pieces; the benchmark's 27.2 M edges, 774 M moves):
+// 20.09 -> 8.15 ms (k_fold 5.99, k_fold_count 2.16); 5.2 M edges of 6-40 ply
+// playouts 5.33 -> 2.95 ms; 4.2 M edges of 60-140 ply playouts 4.26 -> 3.63 ms.
+#pragma once
+#include "pb_fold.cuh"
+#include "pb_kernels.cuh"
+
+namespace pb {
+
+// k_fold's CTA: 80 registers a thread, 24 warps per SM.  On the benchmark's
+// leaves 24 warps ran 5.99 ms, 32 (64 registers, spills) 6.54, 16 (128
+// registers) 6.74; at the same 24 warps, CTAs of 128 / 384 / 768 threads 6.48 /
+// 6.10 / 6.38.  Small launches use 64 threads so that they reach every SM.
+constexpr int FOLD_THREADS = 256;
+constexpr int FOLD_SMALL_THREADS = 64;
+constexpr int FOLD_THREADS_PER_SM = 768;
+constexpr int FOLD_STAGE = 12;  // staged moves per thread of a warp
+
+enum : u32 { DEVERR_QUEUE = 8u };  // a queue was too short for its chunk: the leaf runs again in smaller chunks
+
+// The edges of a leaf.  With n_dev the sizes are in device memory (captured
+// graphs): n and nparents are then the planned capacities.
+struct LeafEdges {
+    const Board *boards;  // positions the edges leave from
+    const uint8_t *states;
+    const u32 *root;  // root index of each position (rooted leaves)
+    const u32 *pidx;
+    const uint16_t *moves;
+    u64 n, nparents;
+    const u64 *n_dev, *nparents_dev;
+};
+
+// Queued moves of one chunk: edge << 16 | move.
+struct FoldQueue {
+    u64 *items;
+    unsigned long long *cursor;
+    u64 cap;
+};
+
+// A warp's sink: moves are staged in shared memory (lane << 16 | move) and
+// flushed to the queue when the warp is done, so its queue entries are
+// contiguous and take one atomic.  A set that does not fit the stage takes
+// queue slots at once; every later set then does not fit either (the stage's
+// cursor only grows), so the stage holds the entries below the smallest cursor
+// of a set that did not fit, without holes.
+struct StagedSink {
+    u32 *stage;
+    u32 *used;  // [0] slots taken, [1] the stage's length
+    u32 lane_tag;
+    u64 edge;
+    FoldQueue q;
+    static constexpr u32 CAP = FOLD_STAGE * 32;
+    __device__ __forceinline__ void set(int from, u64 t)
+    {
+        if (!t) return;
+        const u32 n = (u32)popc(t);
+        u32 slot = atomicAdd(used, n);
+        if (slot + n <= CAP) {
+            const u32 w = lane_tag | (u32)from;
+            for (; t; t &= t - 1) stage[slot++] = w | ((u32)lsb(t) << 6);
+        } else {
+            if (slot < CAP) atomicMin(used + 1, slot);
+            u64 g = atomicAdd(q.cursor, (unsigned long long)n);
+            for (; t; t &= t - 1, g++)
+                if (g < q.cap) q.items[g] = (edge << 16) | (u32)from | ((u32)lsb(t) << 6);
+        }
+    }
+    __device__ __forceinline__ void one(uint16_t m, bool promotes)
+    {
+        const u32 n = promotes ? 4 : 1;
+        u32 w = m | (promotes ? (u32)MF_PROMO << 12 : 0u);
+        const u32 slot = atomicAdd(used, n);
+        if (slot + n <= CAP) {
+            w |= lane_tag;
+            stage[slot] = w;
+            if (promotes)
+                for (u32 k = 1; k < 4; k++) stage[slot + k] = w + (k << 12);
+        } else {
+            if (slot < CAP) atomicMin(used + 1, slot);
+            const u64 g = atomicAdd(q.cursor, (unsigned long long)n);
+            for (u32 k = 0; k < n; k++)
+                if (g + k < q.cap) q.items[g + k] = (edge << 16) | (w + (k << 12));
+        }
+    }
+};
+
+// Edges [first, first + count) of the leaf, cut to its size.  counter[0] +=
+// counts of the simple moves (or, ROOTED, each root's counter), counter[1] +=
+// their number.
+template <int C, bool STRICT, int T, bool ROOTED>
+__global__ void __launch_bounds__(T, FOLD_THREADS_PER_SM / T)
+    k_fold(const __grid_constant__ LeafEdges e, u64 first, u64 count, const __grid_constant__ FoldQueue queue,
+           unsigned long long *__restrict__ root_counts, unsigned long long *__restrict__ counter,
+           u32 *__restrict__ err)
+{
+    constexpr int W = T / 32;
+    __shared__ u32 s_stage[W][FOLD_STAGE * 32];
+    __shared__ u32 s_used[W][2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u64 n = e.n, nparents = e.nparents;
+    if (e.n_dev) {
+        if (plan_overflowed(err)) return;
+        n = dev_size(e.n_dev, n, err);
+        nparents = min(*e.nparents_dev, nparents);
+    }
+    n = min(n, first + count);
+    const u64 i = first + (u64)blockIdx.x * T + threadIdx.x;
+    if (i - lane >= n) return;
+    if (lane == 0) s_used[warp][0] = 0, s_used[warp][1] = FOLD_STAGE * 32;
+    __syncwarp();
+    u32 total = 0, simple = 0, root = 0;
+    const u32 p = i < n ? e.pidx[i] : 0xFFFFFFFFu;
+    const bool valid = i < n && p < nparents;
+    if (valid) {
+        if (ROOTED) root = e.root[p];
+        Board b = load_board(e.boards + p);
+        u32 st = e.states[p];
+        make_move<C>(b, st, e.moves[i]);
+        StagedSink sink{s_stage[warp], s_used[warp], (u32)lane << 16, i, queue};
+        total = fold_child<1 - C, STRICT>(b, st, sink, &simple);
+    }
+    __syncwarp();
+    const u32 used = min(s_used[warp][0], s_used[warp][1]);
+    u64 base = 0;
+    if (lane == 0 && used) base = atomicAdd(queue.cursor, (unsigned long long)used);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (u32 k = lane; k < used; k += 32) {
+        const u32 w = s_stage[warp][k];
+        if (base + k < queue.cap) queue.items[base + k] = ((i - lane + (w >> 16)) << 16) | (w & 0xFFFFu);
+    }
+    if (ROOTED)
+        add_by_key(root_counts, root, total, valid);
+    else
+        total = __reduce_add_sync(0xffffffffu, total);
+    simple = __reduce_add_sync(0xffffffffu, simple);
+    if (lane == 0 && simple) {
+        if (!ROOTED) atomicAdd(counter, (unsigned long long)total);
+        atomicAdd(counter + 1, (unsigned long long)simple);
+    }
+}
+
+// Counts the queued moves (a fixed grid strides over them; their number is on
+// the device).  A queue that was too short sets `overflow` in the error word.
+template <int C, bool STRICT, bool ROOTED>
+__global__ void __launch_bounds__(256, 4)
+    k_fold_count(const __grid_constant__ LeafEdges e, const __grid_constant__ FoldQueue queue,
+                 unsigned long long *__restrict__ root_counts, unsigned long long *__restrict__ counter,
+                 u32 overflow, u32 *__restrict__ err)
+{
+    const u64 len = *queue.cursor;
+    if (len > queue.cap) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, overflow);
+        return;
+    }
+    u64 total = 0;
+    const u64 stride = (u64)gridDim.x * 256;
+    for (u64 k0 = (u64)blockIdx.x * 256 + (threadIdx.x & ~31u); k0 < len; k0 += stride) {
+        const u64 k = k0 + (threadIdx.x & 31);
+        u32 c = 0, root = 0;
+        const bool valid = k < len;
+        if (valid) {
+            const u64 w = queue.items[k], i = w >> 16;
+            const u32 p = e.pidx[i];
+            if (ROOTED) root = e.root[p];
+            Board b = load_board(e.boards + p);
+            u32 st = e.states[p];
+            make_move<C>(b, st, e.moves[i]);
+            make_move<1 - C>(b, st, (uint16_t)w);
+            c = count_moves<C, STRICT>(b, st);
+        }
+        if (ROOTED)
+            add_by_key(root_counts, root, c, valid);
+        else
+            total += c;
+    }
+    if (!ROOTED) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        if ((threadIdx.x & 31) == 0 && total) atomicAdd(counter, (unsigned long long)total);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && len) atomicAdd(counter + 1, (unsigned long long)len);
+}
+
+}  // namespace pb

@@ -140,6 +140,10 @@ inline bool build_host_tables()
             }
         }
     }
+    // past t on the ray s -> t: the squares whose path from s holds t
+    for (int a = 0; a < 64; a++)
+        for (int b = 0; b < 64; b++)
+            for (u64 path = h_tab.between[a][b]; path; path &= path - 1) h_tab.beyond[a][lsb(path)] |= 1ULL << b;
     // zone reach: every square whose empty-board slider rays touch the zone
     for (int k = 0; k < 64; k++) {
         u64 zone = h_tab.king[k] | (1ULL << k);

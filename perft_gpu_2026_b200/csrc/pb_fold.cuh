@@ -7,23 +7,27 @@
 // move, to be made and counted in full (count_moves).
 //
 // X moves, Y = 1 - X is counted.  The base is Y's move count in the position
-// as it stands (no en passant).  A move f -> t of a piece p is SIMPLE when it
-// leaves Y's king moves, castling, pins and checks alone:
-//   - p attacks no square of Y's zone from f or from t.  The zone is the king,
-//     the squares next to it without a Y piece, and the safe squares of a
-//     castling whose path has no Y piece; X-rays through Y's first blocker
-//     towards the king count as attacks (a slider there would pin);
-//   - f is not an X piece that shields a zone square from an X slider, nor
-//     one of two blockers with a Y piece between an X slider and the king;
-//   - t is not on a line from an X slider to a zone square it attacks, nor
-//     between a pinned Y piece's pinner and the king;
+// as it stands (no en passant).  Two sets of squares matter: the core, which is
+// Y's king and the safe squares of a castling whose path has no Y piece, and
+// the ring, the squares next to the king without a Y piece.  A move f -> t of
+// a piece p is SIMPLE when it leaves Y's castling, pins and checks alone and
+// what it does to the king's moves is plain:
+//   - p attacks no core square from f or from t; X-rays through Y's first
+//     blocker towards the king count as attacks (a slider there would pin).
+//     Pawns attack no ring square either;
+//   - f is not an X piece that shields a core or ring square from an X slider,
+//     nor one of two blockers with a Y piece between an X slider and the king;
+//   - t is not on a line from an X slider to a core or ring square it attacks,
+//     nor between a pinned Y piece's pinner and the king;
 //   - neither f nor t is on such a castling path;
 //   - a piece captured on t is not next to the king, pinned, on a castling
 //     corner or a pawn about to promote, is not a slider that sees f along
 //     the line of the capture, and is not a pawn that bears on f (unless a
 //     pawn takes it, where the overlap is one known move).
 // After a simple move
-//   - Y's king, pinned-piece and castling moves are as before;
+//   - Y's pinned-piece and castling moves are as before; its king moves too,
+//     unless p attacks ring squares from f or t: those moves are counted again
+//     from the ring squares that X then attacks (one lookup per move);
 //   - a captured piece's moves are gone; Y's pieces that guarded t take there;
 //   - Y's unpinned pawns change by a weight of f plus a weight of t (pushes
 //     unblocked and captures lost on f, pushes blocked and captures gained on
@@ -37,8 +41,9 @@
 // reach one square: eight lines and eight knight jumps).
 //
 // Promotions, en passant, castling and double pushes that allow an en-passant
-// capture go to the sink.  On the benchmark's leaves 7.5 % of the moves do, on
-// middle-game playouts 21 %, in endgames of pieces alone two thirds.
+// capture go to the sink.  On the benchmark's leaves 4.2 % of the moves do, on
+// middle-game playouts 14 %, late in a game 21 %; without the recounted king
+// moves it was 7.5 %, 21 % and 37 %.
 #pragma once
 #include "pb_core.cuh"
 
@@ -79,6 +84,44 @@ struct TargetPlanes {
 
 PB_HD u64 beyond(int s, int t) { return ldg64(&PB_TAB.beyond[s][t]); }
 
+// x as a value the compiler does not recognise, so that what is computed from
+// it is computed again instead of kept in registers across the piece loops.
+PB_HD u64 fresh(u64 x)
+{
+#ifdef __CUDA_ARCH__
+    asm volatile("" : "+l"(x));
+#endif
+    return x;
+}
+
+// What Y's unpinned pawns `fp` add to its count, by square: pushes (p1 single,
+// dbl double), captures (cw, cc: squares attacked; on the promotion rank a
+// square counts once unless STRICT).  And what an X piece that leaves f gives
+// back: m1 a push, m2 the double push behind it too, m3 a double push.
+template <int Y, bool STRICT>
+struct PawnTerms {
+    static constexpr u64 DP = Y == WHITE ? RANK3 : RANK6;
+    u64 p1, dbl, cw, cc, m1, m2, m3;
+    PB_HD PawnTerms(u64 fp, u64 us, u64 empty)
+    {
+        const u64 pu = push1<Y>(fp);
+        p1 = pu & empty;
+        const u64 dreach = push1<Y>(p1 & DP), ce = cap_east<Y>(fp);
+        dbl = dreach & empty;
+        cw = cap_west<Y>(fp);
+        cc = STRICT ? ce : ce & ~(cw & PROMO_RANKS);
+        m1 = pu & us;
+        m2 = m1 & DP & push1<1 - Y>(empty);
+        m3 = dreach & us;
+    }
+    // weight of leaving the square `fb`
+    PB_HD int leave(u64 fb) const
+    {
+        const int g = (fb & m1 ? 1 : 0) + (fb & m2 ? 1 : 0) + (fb & m3 ? 1 : 0) - (fb & cw ? 1 : 0) - (fb & cc ? 1 : 0);
+        return fb & PROMO_RANKS ? 4 * g : g;
+    }
+};
+
 // Sink: set(from, targets) takes the moves from -> t of one piece (flags 0),
 // one(move, promotes) one move, or with `promotes` the four promotions.
 // Returns the simple moves' sum of counts; *simple = how many they are.
@@ -104,21 +147,22 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
 
     // ---- Y's zone and what in X's position bears on it
     const u64 ring = king_att(yk) & ~them;
-    u64 zone = ring | ykb, path = 0;
+    u64 core = ykb, path = 0;  // the king and the safe squares of an open castling
     const u32 castle_y = Y == WHITE ? (st & 3) : ((st >> 2) & 3);
     if (castle_y) {
-        if ((castle_y & 1) && !(KS_Y & them)) path |= KS_Y, zone |= KS_Y;
-        if ((castle_y & 2) && !(QE_Y & them)) path |= QE_Y, zone |= QS_Y;
+        if ((castle_y & 1) && !(KS_Y & them)) path |= KS_Y, core |= KS_Y;
+        if ((castle_y & 2) && !(QE_Y & them)) path |= QE_Y, core |= QS_Y;
     }
-    u64 reach_b, reach_r;           // squares from which a diagonal / orthogonal slider bears on the zone
+    u64 core_b, core_r;             // squares from which a diagonal / orthogonal slider bears on the core
+    u64 ring_b = 0, ring_r = 0;     // ... on the ring
     u64 keep = path, lines = path;  // squares no simple move leaves / enters
     u64 pinned_y = 0;
-    u64 threat = knights_bulk(s.knights & us) | cap_west<X>(s.pawns & us) | cap_east<X>(s.pawns & us) | king_att(xk);
+    u64 threat = 0, multi = 0;      // zone squares X attacks / attacks more than once
     {
         u64 a = bishop_att(yk, occ);
-        reach_b = a | bishop_att(yk, occ & ~(a & them));
+        core_b = a | bishop_att(yk, occ & ~(a & them));
         a = rook_att(yk, occ);
-        reach_r = a | rook_att(yk, occ & ~(a & them));
+        core_r = a | rook_att(yk, occ & ~(a & them));
     }
     for (u64 sn = (bishop_empty(yk) & bqX) | (rook_empty(yk) & rqX); sn; sn &= sn - 1) {
         const u64 bw = between(lsb(sn), yk), bt = bw & occ, rest = bt & (bt - 1);
@@ -132,12 +176,18 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
         }
     }
     const u64 occ_k = occ ^ ykb;
-    for (u64 z = zone & ~ykb; z; z &= z - 1) {
+    for (u64 z = (ring | core) & ~ykb; z; z &= z - 1) {
         const int q = lsb(z);
+        const u64 zb = z & (0 - z);
         const u64 a = bishop_att(q, occ_k), c = rook_att(q, occ_k);
-        reach_b |= a;
-        reach_r |= c;
-        if ((a & bqX) | (c & rqX)) threat |= 1ULL << q;
+        if (zb & core)
+            core_b |= a, core_r |= c;
+        else
+            ring_b |= a, ring_r |= c;
+        const u64 attackers = (a & bqX) | (c & rqX) | (knight_att(q) & s.knights & us) |
+                              ((cap_west<Y>(zb) | cap_east<Y>(zb)) & s.pawns & us) | (king_att(q) & xkb);
+        if (attackers) threat |= zb;
+        if (more_than_one(attackers)) multi |= zb;
         for (u64 t = (bishop_empty(q) & bqX) | (rook_empty(q) & rqX); t; t &= t - 1) {
             const u64 bw = between(lsb(t), q), bt = bw & occ_k;
             if (!bt)
@@ -162,24 +212,19 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
     }
 
     // ---- Y's base count without its sliders (added with their terms below)
-    u32 base = popc(ring & ~threat);
+    const int kings = popc(ring & ~threat);
+    u32 base = kings;
     if (castle_y) {
         if ((castle_y & 1) && !(KS_Y & (occ | threat))) base++;
         if ((castle_y & 2) && !(QE_Y & occ) && !(QS_Y & threat)) base++;
     }
     const u64 fp = s.pawns & them & ~pinned_y;
-    const u64 pu = push1<Y>(fp), p1 = pu & empty;
-    const u64 dreach = push1<Y>(p1 & DP_Y), dbl = dreach & empty;
-    const u64 cw = cap_west<Y>(fp), ce = cap_east<Y>(fp);
-    // on the promotion rank a square counts 4, and captures onto it once
-    // unless STRICT
-    const u64 cc = STRICT ? ce : ce & ~(cw & PROMO_RANKS);
-    base += popc(p1) + popc(dbl) + popc(cw & us) + popc(cc & us);
     const bool promo = (fp & RANK7_Y) != 0;
-    if (promo) base += 3 * (popc(p1 & PROMO_RANKS) + popc(cw & us & PROMO_RANKS) + popc(cc & us & PROMO_RANKS));
-    // weights of a square left: f unblocks a push (m1), the double push
-    // behind it too (m2), a double push (m3); captures lost are cw, cc
-    const u64 m1 = pu & us, m2 = pu & DP_Y & us & push1<X>(empty), m3 = dreach & us;
+    u64 weighted;  // X pieces whose leaving changes a pawn term
+    {
+        const PawnTerms<Y, STRICT> w(fp, us, empty);
+        weighted = w.m1 | w.m3 | ((w.cw | w.cc) & us);
+    }
     // captured pieces whose loss is no simple term: next to the king, pinned,
     // a castling rook, a pawn about to promote
     const u64 no_cap = king_att(yk) | pinned_y | (castle_y ? CORNERS_Y : 0ULL) | (promo ? fp & RANK7_Y : 0ULL);
@@ -211,7 +256,7 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
     u64 moved0 = 0, moved1 = 0, moved2 = 0;
     const u64 pawns = s.pawns & mine;
     const u64 flagged = east1(s.pawns & them) | west1(s.pawns & them);  // a double push here allows en passant
-    const u64 reach_p = cap_west<Y>(zone) | cap_east<Y>(zone);
+    const u64 reach_p = cap_west<Y>(ring | core) | cap_east<Y>(ring | core);
     const u64 ok_to = ~(reach_p | stay | PROMO_RANKS);
     {
         // pinned pawns push along their king's file and capture along its
@@ -239,13 +284,16 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
         moved0 = x ^ fe;
         moved1 = c ^ c2;
         moved2 = c & c2;
-        if ((moved0 | moved1 | moved2) & (m1 | m3 | cw | cc)) {
-            corr += popc(moved0 & m1) + 2 * popc(moved1 & m1) + 4 * popc(moved2 & m1);
-            corr += popc(moved0 & m2) + 2 * popc(moved1 & m2) + 4 * popc(moved2 & m2);
-            corr += popc(moved0 & m3) + 2 * popc(moved1 & m3) + 4 * popc(moved2 & m3);
-            corr -= popc(moved0 & cw) + 2 * popc(moved1 & cw) + 4 * popc(moved2 & cw);
-            corr -= popc(moved0 & cc) + 2 * popc(moved1 & cc) + 4 * popc(moved2 & cc);
-            corr -= popc(f1 & m3);  // from the double-push square of a Y pawn onto its single-push square
+        if ((moved0 | moved1 | moved2) & weighted) {
+            const PawnTerms<Y, STRICT> w(fresh(fp), us, empty);
+            const u64 plus[3] = {w.m1, w.m2, w.m3}, minus[2] = {w.cw, w.cc};
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                corr += popc(moved0 & plus[k]) + 2 * popc(moved1 & plus[k]) + 4 * popc(moved2 & plus[k]);
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+                corr -= popc(moved0 & minus[k]) + 2 * popc(moved1 & minus[k]) + 4 * popc(moved2 & minus[k]);
+            corr -= popc(f1 & w.m3);  // from the double-push square of a Y pawn onto its single-push square
         }
         // the rest, move by move: en passant (by source), pushes, captures
         u64 ep_from = 0;
@@ -297,70 +345,100 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
     // moves of each, five bits at five times its rank among them; pieces past
     // the twelfth have none (their moves go to the sink).
     const u64 pieces = us & ~s.pawns;
-    u64 moved = 0;
+    u64 moved = 0, movers = moved0 | moved1 | moved2;  // movers: every X piece with a simple move
+    // the moves of one piece: `sm` simple ones, the others to the sink
+    auto split = [&](int f, u64 fb, u64 t, u64 sm) {
+        sink.set(f, t ^ sm);
+        if (!sm) return;
+        const int n = popc(sm);
+        ns += n;
+        to.add(sm);
+        moved |= (u64)n << (5 * popc(pieces & (fb - 1)));
+        movers |= fb;
+        if (fb & weighted) {
+            const PawnTerms<Y, STRICT> w(fresh(fp), us, empty);
+            corr += w.leave(fb) * n;
+            // sliding between the two squares in front of an unmoved pawn
+            if (fb & w.m2) corr -= popc(sm & push1<Y>(fb));
+            if (fb & w.m3) corr -= popc(sm & push1<X>(fb));
+        }
+    };
     {
-        const u64 reach_n = knights_bulk(zone);
-        u64 reach_k = zone | east1(zone) | west1(zone);
-        reach_k |= north(reach_k) | south(reach_k);
-        u64 kn = s.knights & mine & ~pinned_x, sl = (bqX | rqX) & mine, cur = xkb;
+        const u64 core_n = knights_bulk(core), ring_n = knights_bulk(ring);
+        u64 kn = s.knights & mine & ~pinned_x, cur = xkb;
         for (;;) {
             const int f = lsb(cur);
             const u64 fb = cur & (0 - cur);
-            u64 t, no = stay;
-            if (cur == xkb) {
-                t = king_att(f) & ~threat_y;
-                no |= reach_k | bY | rY | (fp & (king_att(f) | push1<X>(push1<X>(fb))));
-                if (fb & reach_k) no = ~0ULL;
-            } else if (fb & s.knights) {
-                t = knight_att(f) & safe;
-                no |= reach_n;
-                if (fb & reach_n) no = ~0ULL;
-            } else {
-                t = 0;
-                if (fb & bqX) {
-                    t = bishop_att(f, occ);
-                    no |= reach_b | (t & bY);
-                    if (fb & reach_b) no = ~0ULL;
+            const bool king = cur == xkb;
+            const u64 a = king ? king_att(f) : knight_att(f);
+            const u64 t = a & ~us & (king ? ~threat_y : safe);
+            if (t) {
+                u64 core_f = core_n, ring_f = ring_n, no = stay;
+                if (king) {
+                    core_f = core | east1(core) | west1(core);
+                    core_f |= north(core_f) | south(core_f);
+                    ring_f = ring | east1(ring) | west1(ring);
+                    ring_f |= north(ring_f) | south(ring_f);
+                    no |= bY | rY | (fp & (a | push1<X>(push1<X>(fb))));
                 }
-                if (fb & rqX) {
-                    const u64 a = rook_att(f, occ);
-                    no |= reach_r | (a & rY);
-                    if (fb & reach_r) no = ~0ULL;
-                    t |= a;
+                const u64 sm = ((fb & (keep | core_f)) || popc(pieces & (fb - 1)) >= 12) ? 0 : t & ~(no | core_f);
+                const u64 left = fb & ring_f ? a & ring & threat & ~multi : 0, near = sm & ring_f;
+                if (near | left) {
+                    // the ring squares attacked change: Y's king moves do
+                    const u64 other = threat & ~left;
+                    if (left) corr += (popc(ring & ~other) - kings) * popc(sm & ~near);
+                    for (u64 q = near; q; q &= q - 1) {
+                        const u64 att = king ? king_att(lsb(q)) : knight_att(lsb(q));
+                        corr += popc(ring & ~(other | att)) - kings;
+                    }
                 }
-                no |= fp & (king_att(f) | push1<X>(push1<X>(fb)));
-                t &= safe;
-                if (fb & pinned_x) t &= line_through(f, xk);
+                split(f, fb, t, sm);
             }
-            t &= ~us;
-            const int rank = popc(pieces & (fb - 1));
-            u64 sm = ((fb & keep) || rank >= 12) ? 0 : t & ~no;
-            sink.set(f, t ^ sm);
-            if (sm) {
-                const int n = popc(sm);
-                ns += n;
-                to.add(sm);
-                moved |= (u64)n << (5 * rank);
-                if (fb & (m1 | m3 | cw | cc)) {
-                    int g = (fb & m1 ? 1 : 0) + (fb & m2 ? 1 : 0) + (fb & m3 ? 1 : 0) - (fb & cw ? 1 : 0) -
-                            (fb & cc ? 1 : 0);
-                    if (fb & PROMO_RANKS) g *= 4;
-                    corr += g * n;
-                    // sliding between the two squares in front of an unmoved pawn
-                    if (fb & m2) corr -= popc(sm & push1<Y>(fb));
-                    if (fb & m3) corr -= popc(sm & push1<X>(fb));
-                }
-            }
-            if (kn) {
-                cur = kn;
-                kn &= kn - 1;
-            } else if (sl) {
-                cur = sl;
-                sl &= sl - 1;
-            } else {
-                break;
+            if (!kn) break;
+            cur = kn;
+            kn &= kn - 1;
+        }
+    }
+    for (u64 sl = (bqX | rqX) & mine; sl; sl &= sl - 1) {
+        const int f = lsb(sl);
+        const u64 fb = sl & (0 - sl);
+        u64 a = 0, core_f = 0, ring_f = 0, seen = 0;
+        if (fb & bqX) {
+            a = bishop_att(f, occ);
+            seen = a & bY;
+            core_f = core_b;
+            ring_f = ring_b;
+        }
+        if (fb & rqX) {
+            const u64 c = rook_att(f, occ);
+            seen |= c & rY;
+            core_f |= core_r;
+            ring_f |= ring_r;
+            a |= c;
+        }
+        u64 t = a & safe & ~us;
+        if (fb & pinned_x) t &= line_through(f, xk);
+        if (!t) continue;
+        const u64 no = stay | core_f | seen | (fp & (king_att(f) | push1<X>(push1<X>(fb))));
+        const u64 sm = ((fb & (keep | core_f)) || popc(pieces & (fb - 1)) >= 12) ? 0 : t & ~no;
+        u64 near = sm & ring_f, left = 0;
+        if (fb & ring_f) {
+            left = a & ring & threat & ~multi;
+            // a slider that moves away along its line keeps its attack
+            for (u64 z = a & ring; z; z &= z - 1) near |= sm & line_through(f, lsb(z));
+        }
+        if (near | left) {
+            const u64 other = threat & ~left;
+            if (left) corr += (popc(ring & ~other) - kings) * popc(sm & ~near);
+            for (u64 q = near; q; q &= q - 1) {
+                const int to_sq = lsb(q);
+                const u64 occ2 = (occ ^ fb) | (q & (0 - q));
+                u64 att = fb & bqX ? bishop_att(to_sq, occ2) : 0;
+                if (fb & rqX) att |= rook_att(to_sq, occ2);
+                corr += popc(ring & ~(other | att)) - kings;
             }
         }
+        split(f, fb, t, sm);
     }
     if (!checkers) {
         const u32 castle_x = X == WHITE ? (st & 3) : ((st >> 2) & 3);
@@ -373,19 +451,25 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
     // ---- weights of the squares entered: Y's pawns, then its pieces
     const u64 any = to.any();
     {
+        const u64 mine_y = fresh(fp);
+        const PawnTerms<Y, STRICT> w(mine_y, us, empty);
+        base += popc(w.p1) + popc(w.dbl) + popc(w.cw & us) + popc(w.cc & us);
         // weight of t: captures gained (cw, cc) less pushes lost (p1, the
         // double push behind it, dbl), plus 2 so that it is never negative,
         // in three bit planes
-        const u64 p1d = p1 & DP_Y & push1<X>(dbl), n0 = (p1 ^ p1d) | dbl;
-        const u64 q0 = cw ^ cc, q1 = cw & cc, r1 = ~(n0 | p1d), k0 = q0 & n0;
+        const u64 p1d = w.p1 & DP_Y & push1<X>(w.dbl), n0 = (w.p1 ^ p1d) | w.dbl;
+        const u64 q0 = w.cw ^ w.cc, q1 = w.cw & w.cc, r1 = ~(n0 | p1d), k0 = q0 & n0;
         const u64 b0 = q0 ^ n0, b1 = q1 ^ r1 ^ k0, b2 = (q1 & r1) | (k0 & (q1 ^ r1));
         corr += to.sum(b0) + 2 * to.sum(b1) - 2 * (int)ns;
         if (any & b2) corr += 4 * to.sum(b2);
-        if (promo) corr += 3 * (to.sum(cw & PROMO_RANKS) + to.sum(cc & PROMO_RANKS) - to.sum(p1 & PROMO_RANKS));
+        if (promo) {  // on the promotion rank a move counts 4
+            base += 3 * (popc(w.p1 & PROMO_RANKS) + popc(w.cw & us & PROMO_RANKS) + popc(w.cc & us & PROMO_RANKS));
+            corr += 3 * (to.sum(w.cw & PROMO_RANKS) + to.sum(w.cc & PROMO_RANKS) - to.sum(w.p1 & PROMO_RANKS));
+        }
+        if (any & mine_y)  // captured pawns take their moves along
+            corr -= to.sum(push1<X>(w.p1)) + to.sum(push1<X>(push1<X>(w.dbl))) + to.sum(mine_y & cap_east<X>(us)) +
+                    to.sum(mine_y & cap_west<X>(us));
     }
-    if (any & fp)  // captured pawns take their moves along
-        corr -= to.sum(push1<X>(p1)) + to.sum(push1<X>(push1<X>(dbl))) + to.sum(fp & cap_east<X>(us)) +
-                to.sum(fp & cap_west<X>(us));
     for (u64 kn = s.knights & them & ~pinned_y; kn; kn &= kn - 1) {
         const u64 a = knight_att(lsb(kn)), bit = kn & (0 - kn);
         const int mob = popc(a & ~them);
@@ -408,6 +492,7 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
         const u64 a = magic_lookup(e, occ);
         const int mob = popc(a & ~them);
         base += mob;
+        if (!((a | bit) & any) && !(a & movers)) continue;
         if (any & bit) corr -= to.at(bit) * mob;
         if (any & a & them) corr += to.sum(a & them);
         // the nearest such square of each ray at once: a lookup with them
@@ -437,21 +522,21 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
                     h &= ~cut;
                 }
         }
-        for (u64 g = a & us; g; g &= g - 1) {
+        for (u64 g = a & movers; g; g &= g - 1) {
             const u64 fb = g & (0 - g);
             int n;
             if (fb & s.pawns) {
                 n = (fb & moved0 ? 1 : 0) + (fb & moved1 ? 2 : 0) + (fb & moved2 ? 4 : 0);
             } else {
-                const int rank = popc(pieces & (fb - 1));
-                n = rank < 12 ? (int)(moved >> (5 * rank)) & 31 : 0;
+                n = (int)(moved >> (5 * popc(pieces & (fb - 1)))) & 31;
             }
-            if (!n) continue;
             const int f = lsb(g);
-            const u64 past = magic_lookup(e, occ ^ fb) & beyond(sq, f);
-            const int ext = popc(past & ~them);
+            const u64 open = magic_lookup(e, occ ^ fb);
+            const int ext = popc(open & ~them) - mob;
             corr += ext * n;
             // moves of f along the same line
+            if (!(fb & (s.pawns | (diag ? bqX : rqX)))) continue;
+            const u64 past = open & beyond(sq, f);
             u64 line = 0;
             if (fb & s.pawns) {
                 if (diag) {
@@ -460,10 +545,10 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
                     const u64 d = push1<X>(fb) & empty;
                     line = (d | (push1<X>(d & DP_X) & empty & ~flagged)) & safe & ok_to;
                 }
-            } else if (fb & (diag ? bqX : rqX)) {
+            } else {
                 u64 no = stay | us | (past & (diag ? bY : rY)) | (fp & (king_att(f) | push1<X>(push1<X>(fb))));
-                if (fb & bqX) no |= reach_b;
-                if (fb & rqX) no |= reach_r;
+                if (fb & bqX) no |= core_b;
+                if (fb & rqX) no |= core_r;
                 line = (between(sq, f) | past) & safe & ~no;
                 if (fb & pinned_x) line &= line_through(f, xk);
             }

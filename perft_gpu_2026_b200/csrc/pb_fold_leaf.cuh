@@ -25,9 +25,9 @@ namespace pb {
 // leaves 24 warps ran 5.99 ms, 32 (64 registers, spills) 6.54, 16 (128
 // registers) 6.74; at the same 24 warps, CTAs of 128 / 384 / 768 threads 6.48 /
 // 6.10 / 6.38.  Small launches use 64 threads so that they reach every SM.
-constexpr int FOLD_THREADS = 256;
+constexpr int FOLD_THREADS = 320;
 constexpr int FOLD_SMALL_THREADS = 64;
-constexpr int FOLD_THREADS_PER_SM = 768;
+constexpr int FOLD_THREADS_PER_SM = 640;
 constexpr int FOLD_STAGE = 12;  // staged moves per thread of a warp
 
 enum : u32 { DEVERR_QUEUE = 8u };  // a queue was too short for its chunk: the leaf runs again in smaller chunks

@@ -190,8 +190,7 @@ typedef struct {
  * listed once for all of its grandchild counts, 6 = folded counting: most
  * grandchildren are summed by set arithmetic, the rest made and counted one
  * per thread from a queue in the BFS arena (default; an arena without room for
- * the queue runs 5 instead); batched and planned leaves follow 4 to 6, table
- * leaves rank their children for 4 to 6 and list pieces for 5 and 6;
+ * the queue runs 5 instead); batched, planned and table leaves follow 4 to 6;
  * leaf_blocks_per_sm: persistent grid of the cooperative leaf. */
 typedef struct {
     int leaf_kernel;
@@ -211,9 +210,10 @@ typedef struct {
                            call per subtree (perft_cpu_recurse, launcher.cu:572-715; default);
                            2 = breadth first, transpositions merged by key with tables, the
                            launch-depth positions in batched GPU calls */
-    int tt_leaf;        /* table leaf with leaf kernels 4 and 5: 1 = one edge per thread;
-                           2 = persistent CTAs that queue their table misses in shared memory and
-                           count only full CTAs of misses (default) */
+    int tt_leaf;        /* table leaf with leaf kernels 4 to 6: 1 = one edge per thread; 2 = only the
+                           table misses are counted, by folding with leaf kernel 6, else (and in
+                           arenas too small for its queue) in persistent CTAs that queue their
+                           misses in shared memory and count full CTAs of them (default) */
 } pb_tuning;
 
 int pb_set_tuning(pb_ctx *ctx, const pb_tuning *t);

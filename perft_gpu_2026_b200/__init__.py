@@ -502,8 +502,8 @@ class Engine:
         planned_leaf 1 = grid over the planned capacity (default),
         2 = persistent work-queue leaf; host_driver 1 = depth-first tree
         above the launch depth (default), 2 = breadth first with batched
-        GPU calls; tt_leaf 1 = one edge per thread, 2 = persistent table leaf
-        that counts only full CTAs of table misses."""
+        GPU calls; tt_leaf 1 = one edge per thread, 2 = only the table misses are
+        counted (folded with leaf kernel 6, else in persistent CTAs)."""
         t = Tuning()
         t.tt_replace = tt_replace
         t.planned_leaf = planned_leaf

@@ -222,7 +222,7 @@ inline cudaError_t reset_counters(pb_ctx *ctx) { return cudaMemsetAsync(ctx->d_c
 
 // The folded leaf over e.n edges; `overflow` is the error bit of a queue that
 // was too short.  The caller has reset the counters.
-template <int C, bool S, bool ROOTED>
+template <int C, bool S, FoldOut OUT>
 cudaError_t launch_fold_t(pb_ctx *ctx, const LeafEdges &e, const FoldQueue &q, bool careful, unsigned long long *rc,
                           u32 overflow)
 {
@@ -235,25 +235,25 @@ cudaError_t launch_fold_t(pb_ctx *ctx, const LeafEdges &e, const FoldQueue &q, b
         }
         const u64 m = std::min(chunk, e.n - first);
         if (m < (u64)ctx->num_sms * FOLD_THREADS_PER_SM)
-            k_fold<C, S, FOLD_SMALL_THREADS, ROOTED><<<grid_for(m, FOLD_SMALL_THREADS), FOLD_SMALL_THREADS, 0, s>>>(
+            k_fold<C, S, FOLD_SMALL_THREADS, OUT><<<grid_for(m, FOLD_SMALL_THREADS), FOLD_SMALL_THREADS, 0, s>>>(
                 e, first, m, q, rc, ctx->d_counter, ctx->d_err);
         else
-            k_fold<C, S, FOLD_THREADS, ROOTED><<<grid_for(m, FOLD_THREADS), FOLD_THREADS, 0, s>>>(
+            k_fold<C, S, FOLD_THREADS, OUT><<<grid_for(m, FOLD_THREADS), FOLD_THREADS, 0, s>>>(
                 e, first, m, q, rc, ctx->d_counter, ctx->d_err);
         // at most a few queued moves per thread of a small launch
         const unsigned g = (unsigned)std::min<u64>((u64)ctx->num_sms * 4, grid_for(m * 16, 256));
-        k_fold_count<C, S, ROOTED><<<g, 256, 0, s>>>(e, q, rc, ctx->d_counter, overflow, ctx->d_err);
+        k_fold_count<C, S, OUT><<<g, 256, 0, s>>>(e, q, rc, ctx->d_counter, overflow, ctx->d_err);
     }
     return cudaGetLastError();
 }
-template <bool ROOTED>
+template <FoldOut OUT>
 cudaError_t launch_fold(pb_ctx *ctx, int c, bool strict, const LeafEdges &e, const FoldQueue &q, bool careful,
                         unsigned long long *rc, u32 overflow)
 {
-    if (c == WHITE) return strict ? launch_fold_t<WHITE, true, ROOTED>(ctx, e, q, careful, rc, overflow)
-                                  : launch_fold_t<WHITE, false, ROOTED>(ctx, e, q, careful, rc, overflow);
-    return strict ? launch_fold_t<BLACK, true, ROOTED>(ctx, e, q, careful, rc, overflow)
-                  : launch_fold_t<BLACK, false, ROOTED>(ctx, e, q, careful, rc, overflow);
+    if (c == WHITE) return strict ? launch_fold_t<WHITE, true, OUT>(ctx, e, q, careful, rc, overflow)
+                                  : launch_fold_t<WHITE, false, OUT>(ctx, e, q, careful, rc, overflow);
+    return strict ? launch_fold_t<BLACK, true, OUT>(ctx, e, q, careful, rc, overflow)
+                  : launch_fold_t<BLACK, false, OUT>(ctx, e, q, careful, rc, overflow);
 }
 
 // NVTX range for profilers (header-only NVTX v3: free unless a tool attaches):
@@ -453,8 +453,8 @@ int bfs_perft(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth,
         {
             NvtxRange nvtx_leaf("leaf");
             if (fold) {
-                const LeafEdges e{cur_b, cur_s, nullptr, epi, emv, n, n_par, nullptr, nullptr};
-                PB_CUDA(launch_fold<false>(ctx, c, strict, e, queue, attempt > 0, nullptr, DEVERR_QUEUE));
+                const LeafEdges e{cur_b, cur_s, nullptr, epi, emv, n, n_par, nullptr, nullptr, nullptr, nullptr, nullptr};
+                PB_CUDA(launch_fold<FOLD_SUM>(ctx, c, strict, e, queue, attempt > 0, nullptr, DEVERR_QUEUE));
             } else {
                 int rc = launch_leaf(ctx, c, strict, cur_b, cur_s, epi, emv, n, n_par);
                 if (rc != PB_OK) return rc;
@@ -499,6 +499,79 @@ int ensure_dtt(pb_ctx *ctx, int max_r)
     ctx->dtt.init(ctx->opts.device_tt_mb, ctx->dtt_free_bytes, max_r, ctx->opts.verbose, &ctx->err);
     ctx->dtt_max_depth = max_r;
     return PB_OK;
+}
+
+// The folded table leaf over n edges, in chunks whose lists and queue fit the
+// arena's rest at 256 queued moves per edge (so no queue is ever too short):
+// false when not even TT_FOLD_MIN edges fit.  The caller has reset the counters
+// (the first chunk's cursors among them).
+// Five launches per chunk: start position-like perft 9 with 8 GB of tables ran
+// 235 ms at 2 M edges per chunk, 241 at 1 M, 233 at 4 M (twice the queue).
+constexpr u64 TT_FOLD_MIN = 1u << 16;   // edges of a chunk at least
+constexpr u64 TT_FOLD_CHUNK = 1u << 21;  // and at most
+static_assert(TT_FOLD_CHUNK <= TT_AT_MASK, "edges of a chunk fit the election's words");
+struct TTFold {
+    u64 chunk = 0;
+    TTChunk ch{};
+    FoldQueue q{};
+};
+bool plan_tt_fold(const pb_ctx *ctx, Arena ar, u64 n, TTFold *f)
+{
+    u64 bytes = 0;
+    ar.rest<char>(&bytes);
+    // queue, key, owner, miss, up to four election slots, padding
+    const u64 per_edge = MAX_MOVES * sizeof(u64) + sizeof(Hash128) + 2 * sizeof(u32) + 4 * sizeof(u32) + 8;
+    f->chunk = std::min(std::min(n, TT_FOLD_CHUNK), bytes / per_edge);
+    if (f->chunk < std::min(n, TT_FOLD_MIN)) return false;
+    u64 slots = 1024;
+    while (slots < 2 * f->chunk) slots *= 2;
+    f->ch.keys = ar.take<Hash128>(f->chunk);
+    f->ch.owner = ar.take<u32>(f->chunk);
+    f->ch.misses = ar.take<u32>(f->chunk);
+    f->ch.slots = ar.take<u32>(slots);
+    f->ch.mask = (u32)(slots - 1);
+    if (!f->ch.keys || !f->ch.owner || !f->ch.misses || !f->ch.slots) return false;
+    f->q = fold_queue(ctx, ar);
+    f->ch.misses_len = f->q.cursor + 1;
+    return f->q.cap / MAX_MOVES >= f->chunk;
+}
+template <int C, bool S>
+cudaError_t launch_tt_fold_t(pb_ctx *ctx, const TTFold &f, const Board *b, const uint8_t *st, const Hash128 *h,
+                             const u32 *pi, const uint16_t *mv, u64 n, u64 npar, TTView tv, u32 *out)
+{
+    cudaStream_t s = ctx->stream;
+    const LeafEdges e{b, st, nullptr, pi, mv, n, npar, nullptr, nullptr, f.ch.misses, f.ch.misses_len, out};
+    u32 gen = 0;
+    for (u64 first = 0; first < n; first += f.chunk) {
+        const u64 m = std::min(f.chunk, n - first);
+        cudaError_t me = cudaSuccess;
+        if (first) me = cudaMemsetAsync(f.q.cursor, 0, 2 * sizeof(unsigned long long), s);
+        // generations 1.. per chunk; the slots are cleared when they run out
+        if (me == cudaSuccess && gen == 0) me = cudaMemsetAsync(f.ch.slots, 0, sizeof(u32) * ((u64)f.ch.mask + 1), s);
+        if (me != cudaSuccess) return me;
+        gen++;
+        k_tt_keys<C><<<grid_for(m, 256), 256, 0, s>>>(b, st, h, pi, mv, first, (u32)m, npar, f.ch, gen);
+        k_tt_probe<<<grid_for(m, 256), 256, 0, s>>>(f.ch, first, (u32)m, tv, out);
+        if (m < (u64)ctx->num_sms * FOLD_THREADS_PER_SM)
+            k_fold<C, S, FOLD_SMALL_THREADS, FOLD_EACH><<<grid_for(m, FOLD_SMALL_THREADS), FOLD_SMALL_THREADS, 0, s>>>(
+                e, 0, m, f.q, nullptr, ctx->d_counter, ctx->d_err);
+        else
+            k_fold<C, S, FOLD_THREADS, FOLD_EACH><<<grid_for(m, FOLD_THREADS), FOLD_THREADS, 0, s>>>(
+                e, 0, m, f.q, nullptr, ctx->d_counter, ctx->d_err);
+        const unsigned g = (unsigned)std::min<u64>((u64)ctx->num_sms * 4, grid_for(m * 16, 256));
+        k_fold_count<C, S, FOLD_EACH><<<g, 256, 0, s>>>(e, f.q, nullptr, ctx->d_counter, DEVERR_QUEUE, ctx->d_err);
+        k_tt_keep<<<grid_for(m, 256), 256, 0, s>>>(f.ch, first, (u32)m, out, tv);
+        if (gen == (1u << (32 - TT_AT_BITS)) - 1) gen = 0;
+    }
+    return cudaGetLastError();
+}
+cudaError_t launch_tt_fold(pb_ctx *ctx, int c, bool strict, const TTFold &f, const Board *b, const uint8_t *st,
+                           const Hash128 *h, const u32 *pi, const uint16_t *mv, u64 n, u64 npar, TTView tv, u32 *out)
+{
+    if (c == WHITE) return strict ? launch_tt_fold_t<WHITE, true>(ctx, f, b, st, h, pi, mv, n, npar, tv, out)
+                                  : launch_tt_fold_t<WHITE, false>(ctx, f, b, st, h, pi, mv, n, npar, tv, out);
+    return strict ? launch_tt_fold_t<BLACK, true>(ctx, f, b, st, h, pi, mv, n, npar, tv, out)
+                  : launch_tt_fold_t<BLACK, false>(ctx, f, b, st, h, pi, mv, n, npar, tv, out);
 }
 
 struct TTLevel {
@@ -745,9 +818,13 @@ int bfs_tt_roots(pb_ctx *ctx, const Board *rb, const uint8_t *rs, const Hash128 
         *bfs_status = BFS_TOO_BIG;
         return PB_OK;
     }
-    PB_CUDA(cudaMemsetAsync(ctx->d_counter, 0, 2 * sizeof(unsigned long long), s));
+    PB_CUDA(reset_counters(ctx));
     if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[1], s));
-    if (n > 0 && leaf_mode(ctx) >= 1 && ctx->tuning.tt_leaf == 2) {
+    TTFold fold;
+    if (n > 0 && leaf_mode(ctx) == 3 && ctx->tuning.tt_leaf == 2 && plan_tt_fold(ctx, ar, n, &fold)) {
+        PB_CUDA(launch_tt_fold(ctx, c, strict, fold, cur_b, cur_s, cur_h, epi, emv, n, n_par, ctx->dtt.at(2), leafcnt));
+        stats.kernels += 1;
+    } else if (n > 0 && leaf_mode(ctx) >= 1 && ctx->tuning.tt_leaf == 2) {
         PB_CUDA(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), s));
         int rc2 = launch_tt_fill(ctx, c, strict, std::min(leaf_mode(ctx), 2), cur_b, cur_s, cur_h, epi, emv, n,
                                  n_par, ctx->dtt.at(2), leafcnt, cursor);
@@ -1036,8 +1113,8 @@ int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth,
                     else k_leaf1_rooted<BLACK, false><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
                 }
             } else if (fold) {
-                const LeafEdges e{cur_b, cur_s, cur_r, epi, emv, ne, n_par, nullptr, nullptr};
-                PB_CUDA(launch_fold<true>(ctx, c, strict, e, queue, attempt > 0, rc, DEVERR_QUEUE));
+                const LeafEdges e{cur_b, cur_s, cur_r, epi, emv, ne, n_par, nullptr, nullptr, nullptr, nullptr, nullptr};
+                PB_CUDA(launch_fold<FOLD_ROOTED>(ctx, c, strict, e, queue, attempt > 0, rc, DEVERR_QUEUE));
             } else {
                 unsigned g = grid_for(ne, PB_LEAF_THREADS);
                 const int mode = std::min(leaf_mode(ctx), 2);
@@ -1290,8 +1367,8 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
                                                                 npar_cap, g.rc, ctx->d_err);
     } else if (g.mode == 3 && !g.queue && fold_fits(fold_queue(ctx, ar))) {
         // a queue too short counts as an outgrown plan
-        const LeafEdges e{pb_, ps, pr, L[nlev].pi, L[nlev].mv, lcap, npar_cap, d_n0 + nlev, npar};
-        launch_fold<true>(ctx, c, g.strict, e, fold_queue(ctx, ar), false, g.rc, DEVERR_OVERFLOW);
+        const LeafEdges e{pb_, ps, pr, L[nlev].pi, L[nlev].mv, lcap, npar_cap, d_n0 + nlev, npar, nullptr, nullptr, nullptr};
+        launch_fold<FOLD_ROOTED>(ctx, c, g.strict, e, fold_queue(ctx, ar), false, g.rc, DEVERR_OVERFLOW);
     } else if (c == WHITE) {
         if (g.strict)
             launch_leaf_queue<WHITE, true>(g.mode, g.queue, s, ctx->num_sms, pb_, ps, pr, L[nlev].pi, L[nlev].mv, d_n0 + nlev, lcap, npar,

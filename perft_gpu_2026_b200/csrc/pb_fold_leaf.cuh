@@ -42,7 +42,15 @@ struct LeafEdges {
     const uint16_t *moves;
     u64 n, nparents;
     const u64 *n_dev, *nparents_dev;
+    // FOLD_EACH: the edges to count (the table leaf's misses) and how many, the
+    // count of each edge
+    const u32 *list;
+    const unsigned long long *list_len;
+    u32 *each;
 };
+
+// Where the counts go: one sum, each root's counter, each listed edge's word.
+enum FoldOut { FOLD_SUM, FOLD_ROOTED, FOLD_EACH };
 
 // Queued moves of one chunk: edge << 16 | move.
 struct FoldQueue {
@@ -99,9 +107,8 @@ struct StagedSink {
 };
 
 // Edges [first, first + count) of the leaf, cut to its size.  counter[0] +=
-// counts of the simple moves (or, ROOTED, each root's counter), counter[1] +=
-// their number.
-template <int C, bool STRICT, int T, bool ROOTED>
+// counts of the simple moves (or as OUT says), counter[1] += their number.
+template <int C, bool STRICT, int T, FoldOut OUT>
 __global__ void __launch_bounds__(T, FOLD_THREADS_PER_SM / T)
     k_fold(const __grid_constant__ LeafEdges e, u64 first, u64 count, const __grid_constant__ FoldQueue queue,
            unsigned long long *__restrict__ root_counts, unsigned long long *__restrict__ counter,
@@ -117,16 +124,17 @@ __global__ void __launch_bounds__(T, FOLD_THREADS_PER_SM / T)
         n = dev_size(e.n_dev, n, err);
         nparents = min(*e.nparents_dev, nparents);
     }
-    n = min(n, first + count);
-    const u64 i = first + (u64)blockIdx.x * T + threadIdx.x;
-    if (i - lane >= n) return;
+    n = OUT == FOLD_EACH ? (u64)*e.list_len : min(n, first + count);
+    const u64 at = first + (u64)blockIdx.x * T + threadIdx.x;
+    if (at - lane >= n) return;
     if (lane == 0) s_used[warp][0] = 0, s_used[warp][1] = FOLD_STAGE * 32;
     __syncwarp();
     u32 total = 0, simple = 0, root = 0;
-    const u32 p = i < n ? e.pidx[i] : 0xFFFFFFFFu;
-    const bool valid = i < n && p < nparents;
+    const u64 i = OUT == FOLD_EACH && at < n ? e.list[at] : at;
+    const u32 p = at < n ? e.pidx[i] : 0xFFFFFFFFu;
+    const bool valid = at < n && p < nparents;
     if (valid) {
-        if (ROOTED) root = e.root[p];
+        if (OUT == FOLD_ROOTED) root = e.root[p];
         Board b = load_board(e.boards + p);
         u32 st = e.states[p];
         make_move<C>(b, st, e.moves[i]);
@@ -140,22 +148,23 @@ __global__ void __launch_bounds__(T, FOLD_THREADS_PER_SM / T)
     base = __shfl_sync(0xffffffffu, base, 0);
     for (u32 k = lane; k < used; k += 32) {
         const u32 w = s_stage[warp][k];
-        if (base + k < queue.cap) queue.items[base + k] = ((i - lane + (w >> 16)) << 16) | (w & 0xFFFFu);
+        const u64 from = at - lane + (w >> 16);
+        if (base + k < queue.cap)
+            queue.items[base + k] = ((OUT == FOLD_EACH ? (u64)e.list[from] : from) << 16) | (w & 0xFFFFu);
     }
-    if (ROOTED)
-        add_by_key(root_counts, root, total, valid);
-    else
-        total = __reduce_add_sync(0xffffffffu, total);
+    if (OUT == FOLD_ROOTED) add_by_key(root_counts, root, total, valid);
+    if (OUT == FOLD_EACH && at < n) e.each[i] = total;
+    if (OUT == FOLD_SUM) total = __reduce_add_sync(0xffffffffu, total);
     simple = __reduce_add_sync(0xffffffffu, simple);
     if (lane == 0 && simple) {
-        if (!ROOTED) atomicAdd(counter, (unsigned long long)total);
+        if (OUT == FOLD_SUM) atomicAdd(counter, (unsigned long long)total);
         atomicAdd(counter + 1, (unsigned long long)simple);
     }
 }
 
 // Counts the queued moves (a fixed grid strides over them; their number is on
 // the device).  A queue that was too short sets `overflow` in the error word.
-template <int C, bool STRICT, bool ROOTED>
+template <int C, bool STRICT, FoldOut OUT>
 __global__ void __launch_bounds__(256, 4)
     k_fold_count(const __grid_constant__ LeafEdges e, const __grid_constant__ FoldQueue queue,
                  unsigned long long *__restrict__ root_counts, unsigned long long *__restrict__ counter,
@@ -175,19 +184,18 @@ __global__ void __launch_bounds__(256, 4)
         if (valid) {
             const u64 w = queue.items[k], i = w >> 16;
             const u32 p = e.pidx[i];
-            if (ROOTED) root = e.root[p];
+            if (OUT == FOLD_ROOTED) root = e.root[p];
             Board b = load_board(e.boards + p);
             u32 st = e.states[p];
             make_move<C>(b, st, e.moves[i]);
             make_move<1 - C>(b, st, (uint16_t)w);
             c = count_moves<C, STRICT>(b, st);
+            if (OUT == FOLD_EACH) atomicAdd(e.each + i, c);
         }
-        if (ROOTED)
-            add_by_key(root_counts, root, c, valid);
-        else
-            total += c;
+        if (OUT == FOLD_ROOTED) add_by_key(root_counts, root, c, valid);
+        if (OUT == FOLD_SUM) total += c;
     }
-    if (!ROOTED) {
+    if (OUT == FOLD_SUM) {
 #pragma unroll
         for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
         if ((threadIdx.x & 31) == 0 && total) atomicAdd(counter, (unsigned long long)total);

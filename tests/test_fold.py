@@ -91,3 +91,22 @@ def test_folded_leaf_in_tight_arenas(arena_mb):
     with pg.Engine(device=0, use_tt=False, arena_bytes=arena_mb << 20) as eng:
         assert eng.perft_position(p, 6) == want
         assert eng.perft_batch(roots, 5) == want_b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("arena_mb", [48, 192, 2048])
+@pytest.mark.parametrize("replace", [1, 2])
+def test_folded_table_leaf_is_exact(arena_mb, replace):
+    """Table leaf by folding: one chunk, several chunks (192 MB) and an arena
+    too small for a chunk (the persistent leaf runs instead); both replacement
+    policies; tables full of transpositions, each depth after the others."""
+    known = {pg.START_FEN: 119060324, FENS[0]: 8031647685, FENS[1]: 11030083}
+    with pg.Engine(device=0, use_tt=True, arena_bytes=arena_mb << 20, device_tt_mb=2048, host_tt_mb=64) as eng:
+        eng.set_tuning(tt_replace=replace)
+        for fen, want in known.items():
+            p = pg.parse_fen(fen)
+            for _ in range(2):  # cold and warm tables
+                assert eng.perft_position(p, 6) == want
+        # a perft-3 call per child: leaves of one partial warp
+        kids = [pg.make_move(pg.parse_fen(FENS[0]), m) for m in pg.generate_moves(pg.parse_fen(FENS[0]))]
+        assert sum(eng.perft_position(k, 3) for k in kids) == 4085603

@@ -2712,9 +2712,11 @@ int pb_mlp_gradients(pb_ctx *ctx, const pb_pos *pos, const float *targets, int n
     Mlp &m = ctx->mlp;
     cudaStream_t s = ctx->stream;
     PB_CUDA(m.alloc_batch(n));
-    PB_CUDA(m.load_positions(pos, n, s));
+    PB_CUDA(m.features_to(pos, m.pos, n, n, m.idx, s));
     PB_CUDA(cudaMemcpyAsync(m.t, targets, sizeof(float) * MLP_OUT * n, cudaMemcpyHostToDevice, s));
-    PB_CUDA(m.forward_backward(n, true, s));
+    PB_CUDA(cudaMemsetAsync(m.loss, 0, sizeof(float), s));
+    PB_CUDA(m.clear_gradients(s));
+    PB_CUDA(m.forward_backward(n, {m.idx, m.t, nullptr, m.loss}, s));
     if (grads) PB_CUDA(cudaMemcpyAsync(grads, m.g, MLP_PARAMS * sizeof(float), cudaMemcpyDeviceToHost, s));
     float l = 0;
     PB_CUDA(cudaMemcpyAsync(&l, m.loss, sizeof(float), cudaMemcpyDeviceToHost, s));
@@ -2737,50 +2739,41 @@ int pb_mlp_train(pb_ctx *ctx, const pb_pos *pos, const float *targets, int n, in
     cudaStream_t s = ctx->stream;
     PB_CUDA(m.alloc_batch(batch));
     // The training set goes to the device once (feature indices and
-    // targets); every step gathers its batch there, so a step is kernel
-    // launches only and the host reads the loss once per epoch.
-    DeviceBuffer<int16_t> all_idx;
-    DeviceBuffer<float> all_t;
-    DeviceBuffer<int> order_d;
-    DeviceBuffer<double> acc;
-    PB_CUDA(all_idx.alloc((size_t)n * MLP_MAX_ACTIVE));
-    PB_CUDA(all_t.alloc((size_t)n * MLP_OUT));
-    PB_CUDA(order_d.alloc((size_t)n));
-    PB_CUDA(acc.alloc(1));
-    for (int c0 = 0; c0 < n; c0 += batch) {
-        const int k = std::min(batch, n - c0);
-        PB_CUDA(m.features_to(pos + c0, k, all_idx.p + (size_t)c0 * MLP_MAX_ACTIVE, s));
-    }
-    PB_CUDA(cudaMemcpyAsync(all_t.p, targets, sizeof(float) * MLP_OUT * (size_t)n, cudaMemcpyHostToDevice, s));
+    // targets); a step's kernels read its samples there through the epoch's
+    // order, so a step is kernel launches only and the host reads the steps'
+    // losses once per epoch.
+    const int steps = n / batch;
+    Mlp::TrainSet set;
+    PB_CUDA(m.alloc_train((size_t)n, (size_t)std::max(steps, 1), &set));
+    std::vector<float> step_loss(std::max(steps, 1), 0.f);
+    PB_CUDA(m.clear_gradients(s));
+    PB_CUDA(m.features_to(pos, set.pos, n, n, set.idx, s));
+    PB_CUDA(cudaMemcpyAsync(set.t, targets, sizeof(float) * MLP_OUT * (size_t)n, cudaMemcpyHostToDevice, s));
     std::vector<int> order(n);
     for (int i = 0; i < n; i++) order[i] = i;
     u64 rng = seed;
     double epoch_loss = 0;
-    const int V = MLP_MAX_ACTIVE * (int)sizeof(int16_t) / 16 + 1;  // gather threads per row
     for (int ep = 0; ep < epochs; ep++) {
         for (int i = n - 1; i > 0; i--) {
             u64 r = splitmix64(&rng);
             int j = (int)(((unsigned __int128)r * (u64)(i + 1)) >> 64);
             std::swap(order[i], order[j]);
         }
-        PB_CUDA(cudaMemcpyAsync(order_d.p, order.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, s));
-        PB_CUDA(cudaMemsetAsync(acc.p, 0, sizeof(double), s));
-        int steps = 0;
-        for (int b0 = 0; b0 + batch <= n; b0 += batch) {
-            k_gather_batch<<<(batch * V + 255) / 256, 256, 0, s>>>(all_idx.p, all_t.p, order_d.p, b0, batch, m.idx,
-                                                                  m.t);
-            PB_CUDA(m.forward_backward(batch, true, s));
+        PB_CUDA(cudaMemcpyAsync(set.order, order.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, s));
+        PB_CUDA(cudaMemsetAsync(set.losses, 0, sizeof(float) * step_loss.size(), s));
+        for (int k = 0; k < steps; k++) {
+            PB_CUDA(m.forward_backward(batch, {set.idx, set.t, set.order + (size_t)k * batch, set.losses + k}, s));
             PB_CUDA(m.adam_step(lr, s));
-            k_accum_loss<<<1, 32, 0, s>>>(m.loss, acc.p, 1.0 / (double)(batch * MLP_OUT));
-            steps++;
         }
         PB_CUDA(cudaGetLastError());
-        double total = 0;
-        PB_CUDA(cudaMemcpyAsync(&total, acc.p, sizeof(double), cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaMemcpyAsync(step_loss.data(), set.losses, sizeof(float) * step_loss.size(), cudaMemcpyDeviceToHost, s));
         PB_CUDA(cudaStreamSynchronize(s));
+        double total = 0;
+        for (int k = 0; k < steps; k++) total += (double)step_loss[k] * (1.0 / (double)(batch * MLP_OUT));
         epoch_loss = steps ? total / steps : 0.0;
     }
     if (final_loss) *final_loss = (float)epoch_loss;
+    m.trim_train();
     return mlp_check(ctx);
 }
 
@@ -2797,10 +2790,8 @@ int pb_mlp_predict(pb_ctx *ctx, const pb_pos *pos, int n, float *out)
     for (int b0 = 0; b0 < n; b0 += chunk) {
         int k = std::min(chunk, n - b0);
         int padded = (k + 63) / 64 * 64;
-        std::vector<pb_pos> tmp(pos + b0, pos + b0 + k);
-        tmp.resize(padded, pos[b0]);
-        PB_CUDA(m.load_positions(tmp.data(), padded, s));
-        PB_CUDA(m.forward_backward(padded, false, s));
+        PB_CUDA(m.features_to(pos + b0, m.pos, k, padded, m.idx, s));
+        PB_CUDA(m.forward_backward(padded, {m.idx, nullptr, nullptr, nullptr}, s));
         PB_CUDA(cudaMemcpyAsync(out + (size_t)b0 * MLP_OUT, m.y, sizeof(float) * MLP_OUT * k, cudaMemcpyDeviceToHost, s));
         PB_CUDA(cudaMemcpyAsync(ctx->h_pinned + 3, m.err, sizeof(u32), cudaMemcpyDeviceToHost, s));
         PB_CUDA(cudaStreamSynchronize(s));

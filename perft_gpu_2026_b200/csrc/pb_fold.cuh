@@ -125,6 +125,9 @@ struct PawnTerms {
 // Sink: set(from, targets) takes the moves from -> t of one piece (flags 0),
 // one(move, promotes) one move, or with `promotes` the four promotions.
 // Returns the simple moves' sum of counts; *simple = how many they are.
+#ifdef __CUDACC__
+#pragma nv_exec_check_disable  // the self-test's sink runs on the host
+#endif
 template <int X, bool STRICT, class Sink>
 PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
 {

@@ -27,77 +27,81 @@ constexpr int MLP_OUT = 4;
 constexpr int MLP_MAX_ACTIVE = 40;
 
 // ---------------------------------------------------------------- features
-// Active feature indices of each position (padded with -1).
-__global__ void k_features(const Board *__restrict__ boards, const uint8_t *__restrict__ states,
-                           const uint8_t *__restrict__ colors, int n, int16_t *__restrict__ idx)
+// A position as callers pass it (pb_pos): quad bitboard, state, side to move.
+struct PosBytes {
+    u64 bb[4];
+    uint8_t state, color, pad[6];
+};
+static_assert(sizeof(PosBytes) == 40, "the layout of pb_pos");
+
+// Active feature indices of each position (padded with -1; rows past `n` have
+// none), one warp per position: a lane writes the features of its two squares
+// at their rank among the occupied ones.  One thread per position was a serial
+// chain of 32 pieces on 16 CTAs: 11.7 us for 4096 positions, read from arrays
+// that the host had split; now 4.5 us from the caller's array as it is.
+__global__ void __launch_bounds__(256) k_features(const PosBytes *__restrict__ pos, int n, int rows,
+                                                  int16_t *__restrict__ idx)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Board b = boards[i];
-    u32 st = states[i];
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (i >= rows) return;
     int16_t *o = idx + (size_t)i * MLP_MAX_ACTIVE;
     int k = 0;
-    u64 occ = b.bb[1] | b.bb[2] | b.bb[3];
-    while (occ && k < 32) {
-        int sq = lsb(occ);
-        int piece = (int)(((b.bb[1] >> sq) & 1) | (((b.bb[2] >> sq) & 1) << 1) | (((b.bb[3] >> sq) & 1) << 2));
-        int col = (int)((b.bb[0] >> sq) & 1);
-        o[k++] = (int16_t)((col * 6 + piece - 1) * 64 + sq);
-        occ &= occ - 1;
+    if (i < n) {
+        const PosBytes *p = pos + i;
+        const u64 b0 = p->bb[0], b1 = p->bb[1], b2 = p->bb[2], b3 = p->bb[3], occ = b1 | b2 | b3;
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            const int sq = lane + 32 * half, at = popc(occ & ((1ULL << sq) - 1));
+            if (((occ >> sq) & 1) && at < 32) {
+                const int piece = (int)(((b1 >> sq) & 1) | (((b2 >> sq) & 1) << 1) | (((b3 >> sq) & 1) << 2));
+                o[at] = (int16_t)(((int)((b0 >> sq) & 1) * 6 + piece - 1) * 64 + sq);
+            }
+        }
+        k = min(popc(occ), 32);
+        // then the side to move, castle rights and en-passant file
+        const u32 st = p->state, extra = (p->color == WHITE ? 1u : 0u) | ((st & 15u) << 1);
+        if (lane < 5 && ((extra >> lane) & 1)) o[k + __popc(extra & ((1u << lane) - 1))] = (int16_t)(768 + lane);
+        k += __popc(extra);
+        if (st >> 4) {
+            if (lane == 0) o[k] = (int16_t)(773 + (st >> 4) - 1);
+            k++;
+        }
     }
-    if (colors[i] == WHITE) o[k++] = 768;
-    for (int c = 0; c < 4; c++)
-        if (st & (1u << c)) o[k++] = (int16_t)(769 + c);
-    if (st >> 4) o[k++] = (int16_t)(773 + (st >> 4) - 1);
-    while (k < MLP_MAX_ACTIVE) o[k++] = -1;
-}
-
-// Training batch from the device-resident training set: row k of the batch
-// is example order[b0 + k] (feature indices, 80 B, and targets, 16 B, as
-// 16-byte vectors).
-__global__ void k_gather_batch(const int16_t *__restrict__ all_idx, const float *__restrict__ all_t,
-                               const int *__restrict__ order, int b0, int B, int16_t *__restrict__ idx,
-                               float *__restrict__ t)
-{
-    static_assert(MLP_MAX_ACTIVE * sizeof(int16_t) % 16 == 0 && MLP_OUT * sizeof(float) == 16, "16-byte rows");
-    constexpr int V = MLP_MAX_ACTIVE * (int)sizeof(int16_t) / 16;  // vectors per feature row
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * (V + 1)) return;
-    const int k = i / (V + 1), v = i % (V + 1);
-    const size_t src = (size_t)order[b0 + k];
-    if (v < V)
-        reinterpret_cast<uint4 *>(idx + (size_t)k * MLP_MAX_ACTIVE)[v] =
-            reinterpret_cast<const uint4 *>(all_idx + src * MLP_MAX_ACTIVE)[v];
-    else
-        reinterpret_cast<float4 *>(t)[k] = reinterpret_cast<const float4 *>(all_t)[src];
-}
-
-// acc += loss * scale, in FP64 and in step order (one thread).
-__global__ void k_accum_loss(const float *__restrict__ loss, double *__restrict__ acc, double scale)
-{
-    if (threadIdx.x == 0 && blockIdx.x == 0) *acc += (double)*loss * scale;
+    for (int j = k + lane; j < MLP_MAX_ACTIVE; j += 32) o[j] = -1;
 }
 
 // ---------------------------------------------------------------- layer 1
-// h1 = relu(b1 + sum of active rows of W1); stored FP32 (for backward) and
-// BF16 (GEMM operand).  One block of 256 threads per sample.
-__global__ void k_mlp_layer1(const int16_t *__restrict__ idx, const __nv_bfloat16 *__restrict__ w1,
-                             const float *__restrict__ b1, int n, float *__restrict__ h1f,
-                             __nv_bfloat16 *__restrict__ h1b)
+// h1 = relu(b1 + sum of active rows of W1), in the order of the row's indices;
+// BF16 (GEMM operand) and with h1f FP32 (for backward).  64 threads per sample,
+// four columns each, four samples per CTA; a training batch names its samples
+// by `order` (null: sample s is row s).  Bound by the W1 rows read from L1 and
+// L2 (16 KB per position): 2-byte loads of one column per thread ran 21.5 us for
+// 4096 positions, 8-byte loads 9.9 us.
+constexpr int L1_SAMPLES = 4;
+__global__ void __launch_bounds__(64 * L1_SAMPLES)
+    k_mlp_layer1(const int16_t *__restrict__ idx, const int *__restrict__ order, const __nv_bfloat16 *__restrict__ w1,
+                 const float *__restrict__ b1, int n, float *__restrict__ h1f, __nv_bfloat16 *__restrict__ h1b)
 {
-    int s = blockIdx.x, j = threadIdx.x;
+    const int s = blockIdx.x * L1_SAMPLES + threadIdx.x / 64, j = (threadIdx.x & 63) * 4;
     if (s >= n) return;
-    float acc = b1[j];
-    const int16_t *a = idx + (size_t)s * MLP_MAX_ACTIVE;
-#pragma unroll 4
+    const float4 b = *reinterpret_cast<const float4 *>(b1 + j);
+    float acc[4] = {b.x, b.y, b.z, b.w};
+    const int16_t *a = idx + (size_t)(order ? order[s] : s) * MLP_MAX_ACTIVE;
+#pragma unroll 8
     for (int k = 0; k < MLP_MAX_ACTIVE; k++) {
-        int f = a[k];
+        const int f = a[k];
         if (f < 0) break;
-        acc += __bfloat162float(w1[(size_t)f * MLP_H + j]);
+        const uint2 w = *reinterpret_cast<const uint2 *>(w1 + (size_t)f * MLP_H + j);
+        acc[0] += __uint_as_float(w.x << 16);
+        acc[1] += __uint_as_float(w.x & 0xFFFF0000u);
+        acc[2] += __uint_as_float(w.y << 16);
+        acc[3] += __uint_as_float(w.y & 0xFFFF0000u);
     }
-    acc = fmaxf(acc, 0.f);
-    h1f[(size_t)s * MLP_H + j] = acc;
-    h1b[(size_t)s * MLP_H + j] = __float2bfloat16(acc);
+    __nv_bfloat16 o[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) acc[q] = fmaxf(acc[q], 0.f), o[q] = __float2bfloat16(acc[q]);
+    if (h1f) *reinterpret_cast<float4 *>(h1f + (size_t)s * MLP_H + j) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<uint2 *>(h1b + (size_t)s * MLP_H + j) = *reinterpret_cast<const uint2 *>(o);
 }
 
 // ---------------------------------------------------------------- tensor-core GEMM
@@ -452,128 +456,185 @@ inline cudaError_t gemm_tc(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 
     return cudaGetLastError();
 }
 
-// h2 = relu(z2 + b2): FP32 and BF16 copies.
-__global__ void k_bias_relu(const float *__restrict__ z, const float *__restrict__ bias, int n, float *__restrict__ hf,
-                            __nv_bfloat16 *__restrict__ hb)
+// h2 = relu(z2 + b2) and y = b3 + h2 . W3, one warp per sample (two in turn, so
+// that the weights are read once); with targets t (rows by `order`) also h2 in
+// FP32, the loss gradient dy = 2 (y - t) / (n * 4) and the squared error sum,
+// one atomic per CTA.  Bound by reading z2.
+constexpr int OUT_SAMPLES = 2;  // per warp
+__global__ void __launch_bounds__(256)
+    k_mlp_out(const float *__restrict__ z2, const float *__restrict__ b2, const __nv_bfloat16 *__restrict__ w3,
+              const float *__restrict__ b3, int n, float *__restrict__ y, const float *__restrict__ t,
+              const int *__restrict__ order, float *__restrict__ h2, float *__restrict__ dy, float *__restrict__ loss)
 {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)n * MLP_H) return;
-    float v = fmaxf(z[i] + bias[i % MLP_H], 0.f);
-    hf[i] = v;
-    hb[i] = __float2bfloat16(v);
-}
-
-// y = b3 + h2 . W3 (one warp per sample), and with targets the loss gradient
-// dy = 2 (y - t) / (n * 4) and the squared error sum.
-__global__ void k_mlp_out(const float *__restrict__ h2, const __nv_bfloat16 *__restrict__ w3,
-                          const float *__restrict__ b3, int n, float *__restrict__ y, const float *__restrict__ t,
-                          float *__restrict__ dy, float *__restrict__ loss)
-{
-    int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (s >= n) return;
-    float acc[MLP_OUT] = {0.f, 0.f, 0.f, 0.f};
-    for (int j = lane; j < MLP_H; j += 32) {
-        float h = h2[(size_t)s * MLP_H + j];
+    constexpr int PER = MLP_H / 32;
+    __shared__ float s_se[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int s0 = (blockIdx.x * 8 + warp) * OUT_SAMPLES;
+    float w[PER][MLP_OUT], b[PER], se = 0.f;
 #pragma unroll
-        for (int o = 0; o < MLP_OUT; o++) acc[o] += h * __bfloat162float(w3[j * MLP_OUT + o]);
+    for (int i = 0; i < PER; i++) {
+        const int j = lane + 32 * i;
+        b[i] = b2[j];
+        const uint2 q = *reinterpret_cast<const uint2 *>(w3 + j * MLP_OUT);
+        w[i][0] = __uint_as_float(q.x << 16), w[i][1] = __uint_as_float(q.x & 0xFFFF0000u);
+        w[i][2] = __uint_as_float(q.y << 16), w[i][3] = __uint_as_float(q.y & 0xFFFF0000u);
     }
+#pragma unroll 1
+    for (int s = s0; s < min(s0 + OUT_SAMPLES, n); s++) {
+        float acc[MLP_OUT] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int o = 0; o < MLP_OUT; o++)
+        for (int i = 0; i < PER; i++) {
+            const size_t at = (size_t)s * MLP_H + lane + 32 * i;
+            const float h = fmaxf(z2[at] + b[i], 0.f);
+            if (t) h2[at] = h;
 #pragma unroll
-        for (int off = 16; off; off >>= 1) acc[o] += __shfl_xor_sync(0xffffffffu, acc[o], off);
-    if (lane == 0) {
-        float se = 0.f;
+            for (int o = 0; o < MLP_OUT; o++) acc[o] += h * w[i][o];
+        }
 #pragma unroll
-        for (int o = 0; o < MLP_OUT; o++) {
-            float v = acc[o] + b3[o];
-            y[s * MLP_OUT + o] = v;
-            if (t) {
-                float d = v - t[s * MLP_OUT + o];
-                dy[s * MLP_OUT + o] = 2.f * d / (float)(n * MLP_OUT);
-                se += d * d;
+        for (int o = 0; o < MLP_OUT; o++)
+#pragma unroll
+            for (int off = 16; off; off >>= 1) acc[o] += __shfl_xor_sync(0xffffffffu, acc[o], off);
+        if (lane == 0) {
+            const int row = t && order ? order[s] : s;
+#pragma unroll
+            for (int o = 0; o < MLP_OUT; o++) {
+                const float v = acc[o] + b3[o];
+                y[s * MLP_OUT + o] = v;
+                if (t) {
+                    const float d = v - t[(size_t)row * MLP_OUT + o];
+                    dy[s * MLP_OUT + o] = 2.f * d / (float)(n * MLP_OUT);
+                    se += d * d;
+                }
             }
         }
-        if (t) atomicAdd(loss, se);
     }
-}
-
-// dW3[j][o] = sum_s h2[s][j] dy[s][o]; db3[o] = sum_s dy[s][o].
-__global__ void k_grad_w3(const float *__restrict__ h2, const float *__restrict__ dy, int n, float *__restrict__ gw3,
-                          float *__restrict__ gb3)
-{
-    int j = blockIdx.x;  // 0..MLP_H (MLP_H = bias row)
-    int o = threadIdx.x & 3, part = threadIdx.x >> 2;  // 64 partial sums per output
-    float acc = 0.f;
-    for (int s = part; s < n; s += 64) acc += (j < MLP_H ? h2[(size_t)s * MLP_H + j] : 1.f) * dy[s * MLP_OUT + o];
-    __shared__ float red[256];
-    red[threadIdx.x] = acc;
+    if (!t) return;
+    if (lane == 0) s_se[warp] = se;
     __syncthreads();
-    for (int w = 128; w >= 4; w >>= 1) {
-        if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x < 4) {
-        if (j < MLP_H)
-            gw3[j * MLP_OUT + threadIdx.x] = red[threadIdx.x];
-        else
-            gb3[threadIdx.x] = red[threadIdx.x];
+    if (threadIdx.x == 0) {
+        float sum = 0.f;
+        for (int k = 0; k < 8; k++) sum += s_se[k];
+        atomicAdd(loss, sum);
     }
 }
 
-// dh2 = (dy . W3^T) * relu'(h2) in FP32 and BF16.
-__global__ void k_back_h2(const float *__restrict__ dy, const __nv_bfloat16 *__restrict__ w3,
-                          const float *__restrict__ h2, int n, float *__restrict__ dh2f,
-                          __nv_bfloat16 *__restrict__ dh2b)
+// Backward through layers 3 and 2's activation for BACK_SAMPLES samples per CTA,
+// one column j per thread: dh2 = (dy . W3^T) * relu'(h2) in BF16 (GEMM operand),
+// and this CTA's part of dW3, db2 and db3 in parts[cta][BACK_PARTS] (dW3[j][o]
+// at j * 4 + o, db2[j] at 1024 + j, db3[o] at 1280 + o), added in a fixed order
+// by k_sum_parts.  One pass over h2 replaces three kernels, of which the column
+// sum ran on one CTA (162 us of a 340 us step at 4096 samples).
+constexpr int BACK_SAMPLES = 32;
+constexpr int BACK_PARTS = MLP_H * MLP_OUT + MLP_H + MLP_OUT;
+__global__ void __launch_bounds__(MLP_H)
+    k_back_h2(const float *__restrict__ dy, const __nv_bfloat16 *__restrict__ w3, const float *__restrict__ h2, int n,
+              __nv_bfloat16 *__restrict__ dh2b, float *__restrict__ parts)
 {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)n * MLP_H) return;
-    size_t s = i / MLP_H;
-    int j = (int)(i % MLP_H);
-    float g = 0.f;
+    __shared__ float s_dy[BACK_SAMPLES * MLP_OUT];
+    const int j = threadIdx.x, s0 = blockIdx.x * BACK_SAMPLES, m = min(BACK_SAMPLES, n - s0);
+    if (j < m * MLP_OUT) s_dy[j] = dy[s0 * MLP_OUT + j];
+    float w[MLP_OUT], gw[MLP_OUT] = {0.f, 0.f, 0.f, 0.f}, gb = 0.f;
 #pragma unroll
-    for (int o = 0; o < MLP_OUT; o++) g += dy[s * MLP_OUT + o] * __bfloat162float(w3[j * MLP_OUT + o]);
-    g = h2[i] > 0.f ? g : 0.f;
-    dh2f[i] = g;
-    dh2b[i] = __float2bfloat16(g);
+    for (int o = 0; o < MLP_OUT; o++) w[o] = __bfloat162float(w3[j * MLP_OUT + o]);
+    __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < m; k++) {
+        const size_t at = (size_t)(s0 + k) * MLP_H + j;
+        const float h = h2[at];
+        float g = 0.f;
+#pragma unroll
+        for (int o = 0; o < MLP_OUT; o++) {
+            const float d = s_dy[k * MLP_OUT + o];
+            g += d * w[o];
+            gw[o] += h * d;
+        }
+        g = h > 0.f ? g : 0.f;
+        gb += g;
+        dh2b[at] = __float2bfloat16(g);
+    }
+    float *out = parts + (size_t)blockIdx.x * BACK_PARTS;
+    *reinterpret_cast<float4 *>(out + j * MLP_OUT) = make_float4(gw[0], gw[1], gw[2], gw[3]);
+    out[MLP_H * MLP_OUT + j] = gb;
+    if (j < MLP_OUT) {
+        float db = 0.f;
+        for (int k = 0; k < m; k++) db += s_dy[k * MLP_OUT + j];
+        out[MLP_H * MLP_OUT + MLP_H + j] = db;
+    }
 }
-
-// Column sums of a [n x MLP_H] FP32 matrix (bias gradients).
-__global__ void k_colsum(const float *__restrict__ m, int n, float *__restrict__ out)
+// 32 sums per CTA, eight threads each over a contiguous eighth of the parts.
+__global__ void __launch_bounds__(256) k_sum_parts(const float *__restrict__ parts, int nparts, float *__restrict__ gw3,
+                                                   float *__restrict__ gb2, float *__restrict__ gb3)
 {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= MLP_H) return;
+    __shared__ float s_acc[8][32];
+    const int lane = threadIdx.x & 31, eighth = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    const int p0 = nparts * eighth / 8, p1 = nparts * (eighth + 1) / 8;
     float acc = 0.f;
-    for (int s = 0; s < n; s++) acc += m[(size_t)s * MLP_H + j];
-    out[j] = acc;
+    if (i < BACK_PARTS) {
+#pragma unroll 8
+        for (int p = p0; p < p1; p++) acc += parts[(size_t)p * BACK_PARTS + i];
+    }
+    s_acc[eighth][lane] = acc;
+    __syncthreads();
+    if (eighth || i >= BACK_PARTS) return;
+    for (int q = 1; q < 8; q++) acc += s_acc[q][lane];
+    if (i < MLP_H * MLP_OUT)
+        gw3[i] = acc;
+    else if (i < MLP_H * MLP_OUT + MLP_H)
+        gb2[i - MLP_H * MLP_OUT] = acc;
+    else
+        gb3[i - MLP_H * MLP_OUT - MLP_H] = acc;
 }
 
 // dh1 (FP32, from the GEMM) masked by relu'(h1), then scattered into the
-// active rows of dW1 (FP32 atomics) and summed into db1.
-__global__ void k_back_l1(const int16_t *__restrict__ idx, const float *__restrict__ dh1raw,
-                          const float *__restrict__ h1, int n, float *__restrict__ gw1, float *__restrict__ gb1)
+// active rows of dW1 with four-wide FP32 reductions and summed into db1.  64
+// threads per sample, four columns each; a thread keeps its part of db1 over
+// BACK1_SAMPLES samples.  Bound by the reductions in L2 (128 K rows of 1 KB per
+// 4096 samples): one-wide atomics and one db1 atomic per sample and column ran
+// 64 us, this 56 (2.4 TB/s of additions into L2).
+constexpr int BACK1_SAMPLES = 8;
+__device__ __forceinline__ void red_add4(float *p, const float4 &v)
 {
-    int s = blockIdx.x, j = threadIdx.x;
-    if (s >= n) return;
-    float g = dh1raw[(size_t)s * MLP_H + j];
-    g = h1[(size_t)s * MLP_H + j] > 0.f ? g : 0.f;
-    if (g == 0.f) return;
-    atomicAdd(gb1 + j, g);
-    const int16_t *a = idx + (size_t)s * MLP_MAX_ACTIVE;
-    for (int k = 0; k < MLP_MAX_ACTIVE; k++) {
-        int f = a[k];
-        if (f < 0) break;
-        atomicAdd(gw1 + (size_t)f * MLP_H + j, g);
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+__global__ void __launch_bounds__(256)
+    k_back_l1(const int16_t *__restrict__ idx, const int *__restrict__ order, const float *__restrict__ dh1raw,
+              const float *__restrict__ h1, int n, float *__restrict__ gw1, float *__restrict__ gb1)
+{
+    const int group = threadIdx.x / 64, j = (threadIdx.x & 63) * 4;
+    float4 db = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < BACK1_SAMPLES; q++) {
+        const int s = (blockIdx.x * BACK1_SAMPLES + q) * 4 + group;
+        if (s >= n) break;
+        float4 g = *reinterpret_cast<const float4 *>(dh1raw + (size_t)s * MLP_H + j);
+        const float4 h = *reinterpret_cast<const float4 *>(h1 + (size_t)s * MLP_H + j);
+        g.x = h.x > 0.f ? g.x : 0.f;
+        g.y = h.y > 0.f ? g.y : 0.f;
+        g.z = h.z > 0.f ? g.z : 0.f;
+        g.w = h.w > 0.f ? g.w : 0.f;
+        if (g.x == 0.f && g.y == 0.f && g.z == 0.f && g.w == 0.f) continue;
+        db.x += g.x, db.y += g.y, db.z += g.z, db.w += g.w;
+        const int16_t *a = idx + (size_t)(order ? order[s] : s) * MLP_MAX_ACTIVE;
+#pragma unroll 4
+        for (int k = 0; k < MLP_MAX_ACTIVE; k++) {
+            const int f = a[k];
+            if (f < 0) break;
+            red_add4(gw1 + (size_t)f * MLP_H + j, g);
+        }
     }
+    red_add4(gb1 + j, db);
 }
 
-// Adam (Kingma and Ba 2015) on FP32 master weights; writes the BF16 copy.
-__global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
+// Adam (Kingma and Ba 2015) on FP32 master weights; writes the BF16 copy.  The
+// first `clear` gradients, which the next step adds to, are zeroed here.
+__global__ void k_adam(float *__restrict__ p, float *__restrict__ g, size_t clear, float *__restrict__ m,
                        float *__restrict__ v, __nv_bfloat16 *__restrict__ pb, size_t n, float lr, float b1,
                        float b2, float eps, float c1, float c2)
 {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float gi = g[i];
+    const float gi = g[i];
+    if (i < clear) g[i] = 0.f;
     float mi = b1 * m[i] + (1.f - b1) * gi;
     float vi = b2 * v[i] + (1.f - b2) * gi * gi;
     m[i] = mi;

@@ -25,20 +25,6 @@ constexpr size_t MLP_OFF_W3 = MLP_OFF_B2 + MLP_H;
 constexpr size_t MLP_OFF_B3 = MLP_OFF_W3 + (size_t)MLP_H * MLP_OUT;
 constexpr size_t MLP_PARAMS = MLP_OFF_B3 + MLP_OUT;
 
-// An owning device array, freed when it leaves scope.
-template <class T>
-struct DeviceBuffer {
-    T *p = nullptr;
-    DeviceBuffer() = default;
-    DeviceBuffer(const DeviceBuffer &) = delete;
-    DeviceBuffer &operator=(const DeviceBuffer &) = delete;
-    ~DeviceBuffer()
-    {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t n) { return cudaMalloc(reinterpret_cast<void **>(&p), n * sizeof(T)); }
-};
-
 struct Mlp {
     bool ready = false;
     int max_batch = 0;
@@ -48,28 +34,70 @@ struct Mlp {
     __nv_bfloat16 *pb = nullptr;
     // activations for one batch
     int16_t *idx = nullptr;
-    float *h1f = nullptr, *z2 = nullptr, *h2f = nullptr, *y = nullptr, *dy = nullptr, *dh2f = nullptr,
+    float *h1f = nullptr, *z2 = nullptr, *h2f = nullptr, *y = nullptr, *dy = nullptr, *parts = nullptr,
           *dh1 = nullptr, *t = nullptr, *loss = nullptr;
     u32 *err = nullptr;     // GEMM error word (a tensor-core wait that gave up)
     float *work = nullptr;  // GEMM K-split partial tiles
     static constexpr size_t WORK_ELEMS = (size_t)tc::MAX_SPLITS * MLP_H * MLP_H;
-    __nv_bfloat16 *h1b = nullptr, *h2b = nullptr, *dh2b = nullptr;
-    Board *pos_b = nullptr;
-    uint8_t *pos_s = nullptr, *pos_c = nullptr;
+    __nv_bfloat16 *h1b = nullptr, *dh2b = nullptr;
+    PosBytes *pos = nullptr;
+    // The training set of the last mlp_train (positions, feature indices,
+    // targets, order, losses of an epoch's steps), kept for the next one unless
+    // larger than TRAIN_KEEP: allocating and freeing it took 0.4 ms per call.
+    char *train = nullptr;
+    size_t train_bytes = 0;
+    static constexpr size_t TRAIN_KEEP = (size_t)64 << 20;
 
     void release()
     {
-        void *ptrs[] = {p,   g,   m,   v,   pb,  idx,  h1f,  z2,    h2f,   y,     dy,
-                        dh2f, dh1, t, loss, err, work, h1b, h2b, dh2b, pos_b, pos_s, pos_c};
+        void *ptrs[] = {p,  g,     m,   v, pb,   idx, h1f,  z2,  h2f, y,
+                        dy, parts, dh1, t, loss, err, work, h1b, dh2b, pos, train};
         for (void *q : ptrs)
             if (q) cudaFree(q);
         *this = Mlp();
     }
 
+    // Device arrays of a training run over n examples and `steps` steps.
+    struct TrainSet {
+        PosBytes *pos;
+        int16_t *idx;
+        float *t;
+        int *order;
+        float *losses;
+    };
+    cudaError_t alloc_train(size_t n, size_t steps, TrainSet *set)
+    {
+        size_t off[6] = {0};
+        const size_t bytes[5] = {n * sizeof(PosBytes), n * MLP_MAX_ACTIVE * sizeof(int16_t),
+                                 n * MLP_OUT * sizeof(float), n * sizeof(int), steps * sizeof(float)};
+        for (int k = 0; k < 5; k++) off[k + 1] = off[k] + ((bytes[k] + 255) & ~(size_t)255);
+        if (off[5] > train_bytes) {
+            if (train) cudaFree(train);
+            train = nullptr;
+            train_bytes = 0;
+            cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&train), off[5]);
+            if (e != cudaSuccess) return e;
+            train_bytes = off[5];
+        }
+        set->pos = reinterpret_cast<PosBytes *>(train + off[0]);
+        set->idx = reinterpret_cast<int16_t *>(train + off[1]);
+        set->t = reinterpret_cast<float *>(train + off[2]);
+        set->order = reinterpret_cast<int *>(train + off[3]);
+        set->losses = reinterpret_cast<float *>(train + off[4]);
+        return cudaSuccess;
+    }
+    void trim_train()
+    {
+        if (train_bytes <= TRAIN_KEEP) return;
+        cudaFree(train);
+        train = nullptr;
+        train_bytes = 0;
+    }
+
     cudaError_t alloc_batch(int B)
     {
         if (B <= max_batch) return cudaSuccess;
-        void *old[] = {idx, h1f, z2, h2f, y, dy, dh2f, dh1, t, h1b, h2b, dh2b, pos_b, pos_s, pos_c};
+        void *old[] = {idx, h1f, z2, h2f, y, dy, parts, dh1, t, h1b, dh2b, pos};
         for (void *q : old)
             if (q) cudaFree(q);
         cudaError_t e;
@@ -80,17 +108,14 @@ struct Mlp {
         PB_MLP_ALLOC(h1f, H * 4);
         PB_MLP_ALLOC(z2, H * 4);
         PB_MLP_ALLOC(h2f, H * 4);
-        PB_MLP_ALLOC(dh2f, H * 4);
+        PB_MLP_ALLOC(parts, (size_t)(B + BACK_SAMPLES - 1) / BACK_SAMPLES * BACK_PARTS * 4);
         PB_MLP_ALLOC(dh1, H * 4);
         PB_MLP_ALLOC(h1b, H * 2);
-        PB_MLP_ALLOC(h2b, H * 2);
         PB_MLP_ALLOC(dh2b, H * 2);
         PB_MLP_ALLOC(y, (size_t)B * MLP_OUT * 4);
         PB_MLP_ALLOC(dy, (size_t)B * MLP_OUT * 4);
         PB_MLP_ALLOC(t, (size_t)B * MLP_OUT * 4);
-        PB_MLP_ALLOC(pos_b, (size_t)B * sizeof(Board));
-        PB_MLP_ALLOC(pos_s, (size_t)B);
-        PB_MLP_ALLOC(pos_c, (size_t)B);
+        PB_MLP_ALLOC(pos, (size_t)B * sizeof(PosBytes));
 #undef PB_MLP_ALLOC
         max_batch = B;
         return cudaSuccess;
@@ -142,45 +167,44 @@ struct Mlp {
         return cudaGetLastError();
     }
 
-    // Positions -> feature indices (device), for rows [0, n) of the batch buffers.
-    cudaError_t load_positions(const pb_pos *pos, int n, cudaStream_t s) { return features_to(pos, n, idx, s); }
-
-    // Feature indices of n positions (n <= max_batch) into rows [0, n) of `out`.
-    cudaError_t features_to(const pb_pos *pos, int n, int16_t *out, cudaStream_t s)
+    // Feature indices of n positions into rows [0, n) of `out`, by way of `dev`;
+    // rows up to `rows` get none.
+    cudaError_t features_to(const pb_pos *from, PosBytes *dev, int n, int rows, int16_t *out, cudaStream_t s)
     {
-        std::vector<Board> b(n);
-        std::vector<uint8_t> st(n), col(n);
-        for (int i = 0; i < n; i++) {
-            for (int k = 0; k < 4; k++) b[i].bb[k] = pos[i].bb[k];
-            st[i] = pos[i].state;
-            col[i] = pos[i].color;
-        }
-        cudaError_t e;
-        if ((e = cudaMemcpyAsync(pos_b, b.data(), sizeof(Board) * n, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
-        if ((e = cudaMemcpyAsync(pos_s, st.data(), n, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
-        if ((e = cudaMemcpyAsync(pos_c, col.data(), n, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
-        k_features<<<(n + 255) / 256, 256, 0, s>>>(pos_b, pos_s, pos_c, n, out);
+        static_assert(sizeof(pb_pos) == sizeof(PosBytes), "positions are copied as they are");
+        cudaError_t e = cudaMemcpyAsync(dev, from, sizeof(PosBytes) * n, cudaMemcpyHostToDevice, s);
+        if (e != cudaSuccess) return e;
+        k_features<<<(unsigned)(((size_t)rows * 32 + 255) / 256), 256, 0, s>>>(dev, n, rows, out);
         return cudaGetLastError();
     }
 
-    // Forward over rows [0, B) (B a multiple of 64); with targets also the
-    // loss, its gradient and all parameter gradients.
-    cudaError_t forward_backward(int B, bool with_grad, cudaStream_t s)
+    // A batch: feature indices and targets by row, the batch's samples by `order`
+    // (null: rows 0, 1, ...).
+    struct Batch {
+        const int16_t *idx;
+        const float *t;    // null: forward only
+        const int *order;
+        float *loss;       // squared error sum, added to
+    };
+
+    // Forward over B samples (a multiple of 64); with targets also the loss, its
+    // gradient and all parameter gradients.  dW1 and db1 are added to `g` (zeroed
+    // by the caller, then by every adam_step).
+    cudaError_t forward_backward(int B, const Batch &in, cudaStream_t s)
     {
         const __nv_bfloat16 *w1 = pb + MLP_OFF_W1, *w2 = pb + MLP_OFF_W2, *w3 = pb + MLP_OFF_W3;
-        k_mlp_layer1<<<B, MLP_H, 0, s>>>(idx, w1, p + MLP_OFF_B1, B, h1f, h1b);
+        k_mlp_layer1<<<(B + L1_SAMPLES - 1) / L1_SAMPLES, 64 * L1_SAMPLES, 0, s>>>(
+            in.idx, in.order, w1, p + MLP_OFF_B1, B, in.t ? h1f : nullptr, h1b);
         cudaError_t e =
             gemm_tc<false, false>(h1b, MLP_H, w2, MLP_H, z2, MLP_H, B, MLP_H, MLP_H, err, work, WORK_ELEMS, s);
         if (e != cudaSuccess) return e;
-        size_t H = (size_t)B * MLP_H;
-        k_bias_relu<<<(unsigned)((H + 255) / 256), 256, 0, s>>>(z2, p + MLP_OFF_B2, B, h2f, h2b);
-        if (with_grad) cudaMemsetAsync(loss, 0, sizeof(float), s);
-        k_mlp_out<<<(B * 32 + 255) / 256, 256, 0, s>>>(h2f, w3, p + MLP_OFF_B3, B, y, with_grad ? t : nullptr, dy,
-                                                       loss);
-        if (!with_grad) return cudaGetLastError();
-        k_grad_w3<<<MLP_H + 1, 256, 0, s>>>(h2f, dy, B, g + MLP_OFF_W3, g + MLP_OFF_B3);
-        k_back_h2<<<(unsigned)((H + 255) / 256), 256, 0, s>>>(dy, w3, h2f, B, dh2f, dh2b);
-        k_colsum<<<1, MLP_H, 0, s>>>(dh2f, B, g + MLP_OFF_B2);
+        k_mlp_out<<<(B + 8 * OUT_SAMPLES - 1) / (8 * OUT_SAMPLES), 256, 0, s>>>(
+            z2, p + MLP_OFF_B2, w3, p + MLP_OFF_B3, B, y, in.t, in.order, h2f, dy, in.loss);
+        if (!in.t) return cudaGetLastError();
+        const int np = (B + BACK_SAMPLES - 1) / BACK_SAMPLES;
+        k_back_h2<<<np, MLP_H, 0, s>>>(dy, w3, h2f, B, dh2b, parts);
+        k_sum_parts<<<(BACK_PARTS + 31) / 32, 256, 0, s>>>(parts, np, g + MLP_OFF_W3, g + MLP_OFF_B2,
+                                                            g + MLP_OFF_B3);
         // dW2 = h1^T dh2 ; dh1 = dh2 W2^T
         if ((e = gemm_tc<true, false>(h1b, MLP_H, dh2b, MLP_H, g + MLP_OFF_W2, MLP_H, MLP_H, MLP_H, B, err, work,
                                       WORK_ELEMS, s)) != cudaSuccess)
@@ -188,9 +212,13 @@ struct Mlp {
         if ((e = gemm_tc<false, true>(dh2b, MLP_H, w2, MLP_H, dh1, MLP_H, B, MLP_H, MLP_H, err, work, WORK_ELEMS,
                                       s)) != cudaSuccess)
             return e;
-        cudaMemsetAsync(g + MLP_OFF_W1, 0, sizeof(float) * ((size_t)MLP_IN * MLP_H + MLP_H), s);
-        k_back_l1<<<B, MLP_H, 0, s>>>(idx, dh1, h1f, B, g + MLP_OFF_W1, g + MLP_OFF_B1);
+        k_back_l1<<<(B + 4 * BACK1_SAMPLES - 1) / (4 * BACK1_SAMPLES), 256, 0, s>>>(
+            in.idx, in.order, dh1, h1f, B, g + MLP_OFF_W1, g + MLP_OFF_B1);
         return cudaGetLastError();
+    }
+    cudaError_t clear_gradients(cudaStream_t s)
+    {
+        return cudaMemsetAsync(g + MLP_OFF_W1, 0, sizeof(float) * (MLP_OFF_W2 - MLP_OFF_W1), s);
     }
 
     cudaError_t adam_step(float lr, cudaStream_t s)
@@ -198,8 +226,8 @@ struct Mlp {
         const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
         step++;
         float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-        k_adam<<<(unsigned)((MLP_PARAMS + 255) / 256), 256, 0, s>>>(p, g, m, v, pb, MLP_PARAMS, lr, b1, b2, eps, c1,
-                                                                    c2);
+        k_adam<<<(unsigned)((MLP_PARAMS + 255) / 256), 256, 0, s>>>(p, g, MLP_OFF_W2, m, v, pb, MLP_PARAMS, lr, b1, b2, eps,
+                                                                    c1, c2);
         return cudaGetLastError();
     }
 };

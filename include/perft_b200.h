@@ -174,7 +174,8 @@ typedef struct {
     uint64_t leaf_edges;       /* edges the leaf kernel took (one perft(2) each) */
     uint64_t leaf_positions;   /* positions the leaf kernel counted (move-count calls) */
     uint64_t nodes;            /* the perft result of the call */
-    uint32_t kernels;          /* kernel launches of the call (a leaf counts once) */
+    uint32_t kernels;          /* kernel launches of the call: three per BFS level and one per leaf,
+                                  however few or many kernels a level or leaf took */
     uint32_t levels;           /* BFS expand levels */
     uint64_t level_sizes[16];  /* edges per level, level 0 = root moves */
     uint64_t h2d_bytes;        /* host-to-device bytes copied */

@@ -28,6 +28,7 @@
 #include "pb_util.cuh"
 #include "pb_kernels.cuh"
 #include "pb_fold_leaf.cuh"
+#include "pb_wide.cuh"
 #include "pb_tt.cuh"
 #include "pb_devtt.cuh"
 #include "pb_mlp_host.cuh"
@@ -59,6 +60,14 @@ struct GraphPlan {
 
 }  // namespace pb
 
+// The device scratch block: counters at word 0, the error word at 8, the scan's
+// ticket at 16, level totals from 24 (the scan's, then one per whole-level
+// kernel).  Cleared and read back as a whole.
+constexpr size_t SCRATCH_BYTES = 256;
+constexpr int SCRATCH_ERR = 8;
+constexpr int WIDE_LEVELS = 7;
+constexpr size_t STAGE_BYTES = 512 * 1024;  // uploads and readbacks of calls with few roots
+
 struct pb_ctx {
     int device = -1;
     bool gpu = false;
@@ -72,6 +81,7 @@ struct pb_ctx {
     u32 *d_ticket = nullptr;
     u64 *d_total = nullptr;
     u64 *h_pinned = nullptr;  // pinned host words for readbacks
+    char *h_stage = nullptr;  // pinned host bytes for uploads (STAGE_BYTES, in the same block)
     int launch_depth = 0;
     bool timing = false;
     pb_tuning tuning{6, 0, 1024, 128, 2, 1, 1, 1, 2};
@@ -217,6 +227,10 @@ inline u64 fold_chunk(const FoldQueue &q, u64 n, bool careful)
     return std::min(n, std::max(q.cap / 64, std::min<u64>(q.cap / 16, 1u << 20)));
 }
 
+// Below one wave of edges k_fold runs small CTAs, which reach every SM (up to two
+// waves either size takes the same time; at 1.5 M edges small ones take 11 % more).
+inline bool fold_small(const pb_ctx *ctx, u64 m) { return m < (u64)ctx->num_sms * FOLD_THREADS_PER_SM; }
+
 // Zeroes the counters and the first chunk's queue cursor (one 64-byte block).
 inline cudaError_t reset_counters(pb_ctx *ctx) { return cudaMemsetAsync(ctx->d_counter, 0, 64, ctx->stream); }
 
@@ -234,7 +248,7 @@ cudaError_t launch_fold_t(pb_ctx *ctx, const LeafEdges &e, const FoldQueue &q, b
             if (me != cudaSuccess) return me;
         }
         const u64 m = std::min(chunk, e.n - first);
-        if (m < (u64)ctx->num_sms * FOLD_THREADS_PER_SM)
+        if (fold_small(ctx, m))
             k_fold<C, S, FOLD_SMALL_THREADS, OUT><<<grid_for(m, FOLD_SMALL_THREADS), FOLD_SMALL_THREADS, 0, s>>>(
                 e, first, m, q, rc, ctx->d_counter, ctx->d_err);
         else
@@ -334,6 +348,16 @@ int launch_leaf(pb_ctx *ctx, int c, bool strict, const Board *b, const uint8_t *
                   : launch_leaf_t<BLACK, false>(ctx, b, st, pi, mv, n, npar);
 }
 
+// Levels and leaves of at most this many positions run one warp per position.
+// Where the line lies: 200 roots at perft 4 (5,981 positions in the level) ran
+// the level in 26 us wide and 42 us by three kernels; at 28 K edges a wide leaf
+// would issue 1,600 warp instructions per edge, 62 us, and the folded one takes 44.
+constexpr u64 WIDE_MAX = 8192;
+// From at most this many positions the leaf follows without the host reading
+// the number of its edges (a chess position has about 30 moves).
+constexpr u64 WIDE_UNREAD = 64;
+inline unsigned wide_grid(u64 n) { return grid_for(n, WIDE_WARPS); }
+
 // Staged generation with the tuned CTA size.
 void launch_generate(pb_ctx *ctx, int c, const Board *b, const uint8_t *st, const u64 *offs, u64 n, uint16_t *mv,
                      u32 *pi)
@@ -345,6 +369,77 @@ void launch_generate(pb_ctx *ctx, int c, const Board *b, const uint8_t *st, cons
     } else {
         if (c == WHITE) k_generate<WHITE, 128><<<grid_for(n, 128), 128, 0, s>>>(b, st, offs, ctx->d_total, n, mv, pi, ctx->d_err);
         else k_generate<BLACK, 128><<<grid_for(n, 128), 128, 0, s>>>(b, st, offs, ctx->d_total, n, mv, pi, ctx->d_err);
+    }
+}
+
+// A small level in one kernel (k_level_wide): children of n edges (pi null: the
+// n positions themselves) and their moves; cr null: without roots.
+void launch_level_wide(pb_ctx *ctx, int c, const Board *pb_, const uint8_t *ps, const u32 *pr, const u32 *pi,
+                       const uint16_t *mv, u64 n, u64 npar, Board *cb, uint8_t *cs, u32 *cr, uint16_t *nmv, u32 *npi,
+                       unsigned long long *total)
+{
+    cudaStream_t s = ctx->stream;
+    const u64 cap = n * MAX_MOVES;
+#define PB_LEVEL_W(CC, EE, RR, WW)                                                                                    \
+    k_level_wide<CC, EE, RR, WW><<<grid_for(n, WW), 32 * WW, 0, s>>>(pb_, ps, pr, pi, mv, (u32)n, npar, cb, cs, cr, nmv, \
+                                                                     npi, cap, total, ctx->d_err)
+#define PB_LEVEL(CC, EE, RR)                            \
+    do {                                                \
+        if (n <= WIDE_SMALL)                            \
+            PB_LEVEL_W(CC, EE, RR, WIDE_WARPS);         \
+        else                                            \
+            PB_LEVEL_W(CC, EE, RR, WIDE_LEVEL_WARPS);   \
+    } while (0)
+    if (!pi) PB_LEVEL(WHITE, false, true);  // batched roots have white to move
+    else if (cr && c == WHITE) PB_LEVEL(WHITE, true, true);
+    else if (cr) PB_LEVEL(BLACK, true, true);
+    else if (c == WHITE) PB_LEVEL(WHITE, true, false);
+    else PB_LEVEL(BLACK, true, false);
+#undef PB_LEVEL
+#undef PB_LEVEL_W
+}
+// Whether a level of n positions runs as one kernel: small, and the bound on
+// its moves takes no notable part of the arena.
+inline bool wide_level(const pb_ctx *ctx, u64 n)
+{
+    return n <= WIDE_MAX && n * MAX_MOVES * (sizeof(uint16_t) + sizeof(u32)) <= ctx->arena_bytes / 16;
+}
+
+// Scan of n counts into offsets, the total to ctx->d_total; false if the arena
+// has no room.
+bool launch_scan(pb_ctx *ctx, Arena &ar, const u32 *cnt, u64 n, u64 *offs)
+{
+    const u64 tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+    u64 *status = ar.take<u64>(tiles + 1);  // and the tile ticket
+    if (!status) return false;
+    cudaMemsetAsync(status, 0, sizeof(u64) * (tiles + 1), ctx->stream);
+    k_scan<<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(cnt, n, offs, status, reinterpret_cast<u32 *>(status + tiles),
+                                                             ctx->d_total, ctx->d_err);
+    return true;
+}
+
+// The fused two-ply leaf of a small level; counts to one sum or (rc) per root.
+// With n_dev the number of edges is on the device and the grid (for n edges at
+// most WIDE_MAX) strides over them.
+template <int C, bool S>
+void launch_leaf_wide_t(pb_ctx *ctx, const Board *b, const uint8_t *st, const u32 *r, const u32 *pi,
+                        const uint16_t *mv, u64 n, const unsigned long long *n_dev, u64 npar, unsigned long long *rc)
+{
+    const unsigned w = wide_grid(std::min(n, WIDE_MAX)), wt = 32 * WIDE_WARPS;
+    if (rc)
+        k_leaf2_wide<C, S, true><<<w, wt, 0, ctx->stream>>>(b, st, r, pi, mv, (u32)n, n_dev, npar, rc, ctx->d_counter);
+    else
+        k_leaf2_wide<C, S, false><<<w, wt, 0, ctx->stream>>>(b, st, r, pi, mv, (u32)n, n_dev, npar, rc, ctx->d_counter);
+}
+void launch_leaf_wide(pb_ctx *ctx, int c, bool strict, const Board *b, const uint8_t *st, const u32 *r, const u32 *pi,
+                      const uint16_t *mv, u64 n, const unsigned long long *n_dev, u64 npar, unsigned long long *rc)
+{
+    if (c == WHITE) {
+        if (strict) launch_leaf_wide_t<WHITE, true>(ctx, b, st, r, pi, mv, n, n_dev, npar, rc);
+        else launch_leaf_wide_t<WHITE, false>(ctx, b, st, r, pi, mv, n, n_dev, npar, rc);
+    } else {
+        if (strict) launch_leaf_wide_t<BLACK, true>(ctx, b, st, r, pi, mv, n, n_dev, npar, rc);
+        else launch_leaf_wide_t<BLACK, false>(ctx, b, st, r, pi, mv, n, n_dev, npar, rc);
     }
 }
 
@@ -375,12 +470,19 @@ int bfs_perft(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth,
         *bfs_status = BFS_TOO_BIG;
         return PB_OK;
     }
-    uint8_t st8 = (uint8_t)root_st;
-    PB_CUDA(cudaMemcpyAsync(pb_, &root, sizeof(Board), cudaMemcpyHostToDevice, s));
-    PB_CUDA(cudaMemcpyAsync(ps, &st8, 1, cudaMemcpyHostToDevice, s));
-    PB_CUDA(cudaMemcpyAsync(emv, root_moves, sizeof(uint16_t) * n0, cudaMemcpyHostToDevice, s));
-    PB_CUDA(cudaMemsetAsync(epi, 0, sizeof(u32) * n0, s));
-    PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));
+    // root, state, moves and parent indices (zero) in one copy, laid out as in
+    // the arena; error word, counters and totals cleared in one memset
+    {
+        const size_t bytes = (size_t)(reinterpret_cast<char *>(epi) - ctx->arena) + sizeof(u32) * n0;
+        char *stage = ctx->h_stage;
+        const uint8_t st8 = (uint8_t)root_st;
+        memset(stage, 0, bytes);
+        memcpy(stage, &root, sizeof(Board));
+        memcpy(stage + (reinterpret_cast<char *>(ps) - ctx->arena), &st8, 1);
+        memcpy(stage + (reinterpret_cast<char *>(emv) - ctx->arena), root_moves, sizeof(uint16_t) * n0);
+        PB_CUDA(cudaMemcpyAsync(ctx->arena, stage, bytes, cudaMemcpyHostToDevice, s));
+    }
+    PB_CUDA(cudaMemsetAsync(ctx->d_counter, 0, SCRATCH_BYTES, s));
     stats.h2d_bytes += sizeof(Board) + 1 + sizeof(uint16_t) * n0;
     if (stats.levels < 16) stats.level_sizes[stats.levels] = (u64)n0;
     if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[0], s));
@@ -391,51 +493,77 @@ int bfs_perft(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth,
     u64 n_par = 1;  // positions the current edges point into
     int c = color;
     const int fuse = ctx->tuning.leaf_fuse == 1 ? 1 : 2;
+    const unsigned long long *n_dev = nullptr;  // the leaf's edges, where the host does not wait for their number
+    int wide_levels = 0;
     for (int rem = depth - 1; rem > fuse; rem--) {
         Board *cb = ar.take<Board>(n);
         uint8_t *cs = ar.take<uint8_t>(n);
-        u32 *cnt = ar.take<u32>(n);
-        u64 *offs = ar.take<u64>(n);
-        u64 tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-        u64 *status = ar.take<u64>(tiles);
-        if (!cb || !cs || !cnt || !offs || !status) {
+        if (!cb || !cs) {
             *bfs_status = BFS_TOO_BIG;
             return PB_OK;
         }
-        if (c == WHITE)
-            k_expand_count<WHITE><<<grid_for(n, 256), 256, 0, s>>>(cur_b, cur_s, epi, emv, n, n_par, cb, cs, cnt, ctx->d_err);
-        else
-            k_expand_count<BLACK><<<grid_for(n, 256), 256, 0, s>>>(cur_b, cur_s, epi, emv, n, n_par, cb, cs, cnt, ctx->d_err);
-        PB_CUDA(cudaGetLastError());
-        PB_CUDA(cudaMemsetAsync(status, 0, sizeof(u64) * tiles, s));
-        PB_CUDA(cudaMemsetAsync(ctx->d_ticket, 0, sizeof(u32), s));
-        k_scan<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(cnt, n, offs, status, ctx->d_ticket, ctx->d_total, ctx->d_err);
-        PB_CUDA(cudaGetLastError());
-        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_total, sizeof(u64), cudaMemcpyDeviceToHost, s));
-        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned + 1, ctx->d_err, sizeof(u32), cudaMemcpyDeviceToHost, s));
-        PB_CUDA(cudaStreamSynchronize(s));
+        uint16_t *nmv = nullptr;
+        u32 *npi = nullptr;
+        u64 *offs = nullptr;
+        const bool whole = wide_level(ctx, n) && wide_levels < WIDE_LEVELS;
+        unsigned long long *total = reinterpret_cast<unsigned long long *>(ctx->d_total);
+        if (whole) {
+            total += 1 + wide_levels++;
+            nmv = ar.take<uint16_t>(n * MAX_MOVES);
+            npi = ar.take<u32>(n * MAX_MOVES);
+            if (!nmv || !npi) {
+                *bfs_status = BFS_TOO_BIG;
+                return PB_OK;
+            }
+            launch_level_wide(ctx, c, cur_b, cur_s, nullptr, epi, emv, n, n_par, cb, cs, nullptr, nmv, npi, total);
+            PB_CUDA(cudaGetLastError());
+            if (rem - 1 == fuse && fuse == 2 && n <= WIDE_UNREAD && ctx->tuning.leaf_kernel == 6) n_dev = total;
+        } else {
+            u32 *cnt = ar.take<u32>(n);
+            offs = ar.take<u64>(n);
+            if (!cnt || !offs) {
+                *bfs_status = BFS_TOO_BIG;
+                return PB_OK;
+            }
+            if (c == WHITE)
+                k_expand_count<WHITE><<<grid_for(n, 256), 256, 0, s>>>(cur_b, cur_s, epi, emv, n, n_par, cb, cs, cnt, ctx->d_err);
+            else
+                k_expand_count<BLACK><<<grid_for(n, 256), 256, 0, s>>>(cur_b, cur_s, epi, emv, n, n_par, cb, cs, cnt, ctx->d_err);
+            if (!launch_scan(ctx, ar, cnt, n, offs)) {
+                *bfs_status = BFS_TOO_BIG;
+                return PB_OK;
+            }
+            PB_CUDA(cudaGetLastError());
+        }
         stats.kernels += 2;
-        stats.d2h_bytes += 12;
-        if ((u32)ctx->h_pinned[1]) return fail(ctx, PB_ERR_DEVICE, "scan reported a device error");
-        u64 next = ctx->h_pinned[0];
         stats.levels++;
-        if (stats.levels < 16) stats.level_sizes[stats.levels] = next;
-        if (next == 0) {
-            *out = 0;
-            return PB_OK;
+        u64 next = n * MAX_MOVES;
+        if (!n_dev) {
+            PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, SCRATCH_BYTES, cudaMemcpyDeviceToHost, s));
+            PB_CUDA(cudaStreamSynchronize(s));
+            stats.d2h_bytes += SCRATCH_BYTES;
+            if ((u32)ctx->h_pinned[SCRATCH_ERR]) return fail(ctx, PB_ERR_DEVICE, "a BFS level reported a device error");
+            next = ctx->h_pinned[total - ctx->d_counter];
+            if (stats.levels < 16) stats.level_sizes[stats.levels] = next;
+            if (next == 0) {
+                *out = 0;
+                return PB_OK;
+            }
+            if (next > 0xFFFFFFFFULL) {  // parent indices are u32
+                *bfs_status = BFS_TOO_BIG;
+                return PB_OK;
+            }
         }
-        if (next > 0xFFFFFFFFULL) {  // parent indices are u32
-            *bfs_status = BFS_TOO_BIG;
-            return PB_OK;
+        if (!whole) {
+            nmv = ar.take<uint16_t>(next);
+            npi = ar.take<u32>(next);
+            if (!nmv || !npi) {
+                *bfs_status = BFS_TOO_BIG;
+                return PB_OK;
+            }
+            launch_generate(ctx, 1 - c, cb, cs, offs, n, nmv, npi);
+            PB_CUDA(cudaGetLastError());
         }
-        uint16_t *nmv = ar.take<uint16_t>(next);
-        u32 *npi = ar.take<u32>(next);
-        if (!nmv || !npi) {
-            *bfs_status = BFS_TOO_BIG;
-            return PB_OK;
-        }
-        launch_generate(ctx, 1 - c, cb, cs, offs, n, nmv, npi);
-        PB_CUDA(cudaGetLastError());
         stats.kernels += 1;
         cur_b = cb;
         cur_s = cs;
@@ -446,13 +574,16 @@ int bfs_perft(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth,
         c = 1 - c;
     }
     const FoldQueue queue = fold_queue(ctx, ar);
+    const bool wide = n_dev || (ctx->tuning.leaf_kernel == 6 && fuse == 2 && n <= WIDE_MAX);
     const bool fold = ctx->tuning.leaf_kernel == 6 && fuse == 2 && fold_fits(queue);
     for (int attempt = 0;; attempt++) {
-        PB_CUDA(reset_counters(ctx));
+        if (attempt) PB_CUDA(reset_counters(ctx));
         if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[1], s));
         {
             NvtxRange nvtx_leaf("leaf");
-            if (fold) {
+            if (wide) {
+                launch_leaf_wide(ctx, c, strict, cur_b, cur_s, nullptr, epi, emv, n, n_dev, n_par, nullptr);
+            } else if (fold) {
                 const LeafEdges e{cur_b, cur_s, nullptr, epi, emv, n, n_par, nullptr, nullptr, nullptr, nullptr, nullptr};
                 PB_CUDA(launch_fold<FOLD_SUM>(ctx, c, strict, e, queue, attempt > 0, nullptr, DEVERR_QUEUE));
             } else {
@@ -465,18 +596,21 @@ int bfs_perft(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth,
             PB_CUDA(cudaEventRecord(ctx->ev[2], s));
             PB_CUDA(cudaEventRecord(ctx->ev[3], s));
         }
-        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, 2 * sizeof(u64), cudaMemcpyDeviceToHost, s));
-        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned + 2, ctx->d_err, sizeof(u32), cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, SCRATCH_BYTES, cudaMemcpyDeviceToHost, s));
         PB_CUDA(cudaStreamSynchronize(s));
-        if ((u32)ctx->h_pinned[2] != DEVERR_QUEUE || attempt > 0) break;
+        if ((u32)ctx->h_pinned[SCRATCH_ERR] != DEVERR_QUEUE || attempt > 0) break;
         PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));  // a queue was too short
     }
-    if ((u32)ctx->h_pinned[2]) return fail(ctx, PB_ERR_DEVICE, "kernel reported a device error");
+    if ((u32)ctx->h_pinned[SCRATCH_ERR]) return fail(ctx, PB_ERR_DEVICE, "kernel reported a device error");
+    if (n_dev) {
+        n = ctx->h_pinned[n_dev - ctx->d_counter];
+        if (stats.levels < 16) stats.level_sizes[stats.levels] = n;
+    }
     *out = ctx->h_pinned[0];
     stats.kernels += 1;
     stats.leaf_edges += n;
     stats.leaf_positions += ctx->h_pinned[1];
-    stats.d2h_bytes += 20;
+    stats.d2h_bytes += SCRATCH_BYTES;
     if (ctx->timing) {
         float a = 0, b2 = 0;
         PB_CUDA(cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[3]));
@@ -552,7 +686,7 @@ cudaError_t launch_tt_fold_t(pb_ctx *ctx, const TTFold &f, const Board *b, const
         gen++;
         k_tt_keys<C><<<grid_for(m, 256), 256, 0, s>>>(b, st, h, pi, mv, first, (u32)m, npar, f.ch, gen);
         k_tt_probe<<<grid_for(m, 256), 256, 0, s>>>(f.ch, first, (u32)m, tv, out);
-        if (m < (u64)ctx->num_sms * FOLD_THREADS_PER_SM)
+        if (fold_small(ctx, m))
             k_fold<C, S, FOLD_SMALL_THREADS, FOLD_EACH><<<grid_for(m, FOLD_SMALL_THREADS), FOLD_SMALL_THREADS, 0, s>>>(
                 e, 0, m, f.q, nullptr, ctx->d_counter, ctx->d_err);
         else
@@ -978,19 +1112,22 @@ int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth,
     u32 *cnt0 = ar.take<u32>(n);
     u64 *off0 = ar.take<u64>(n);
     unsigned long long *rc = ar.take<unsigned long long>(n);
-    u64 tiles0 = (n + SCAN_TILE - 1) / SCAN_TILE;
-    u64 *status0 = ar.take<u64>(tiles0);
-    if (!b0 || !s0 || !r0 || !cnt0 || !off0 || !rc || !status0) {
+    if (!b0 || !s0 || !r0 || !cnt0 || !off0 || !rc) {
         *bfs_status = BFS_TOO_BIG;
         return PB_OK;
     }
-    std::vector<u32> iota(n);
-    for (u64 i = 0; i < n; i++) iota[i] = (u32)i;
-    PB_CUDA(cudaMemcpyAsync(b0, rb, sizeof(Board) * n, cudaMemcpyHostToDevice, s));
-    PB_CUDA(cudaMemcpyAsync(s0, rs, n, cudaMemcpyHostToDevice, s));
-    PB_CUDA(cudaMemcpyAsync(r0, iota.data(), sizeof(u32) * n, cudaMemcpyHostToDevice, s));
+    const bool few = n <= WIDE_MAX;  // boards, states and counts fit the pinned staging area
+    if (few) {
+        const size_t at = (size_t)(reinterpret_cast<char *>(s0) - ctx->arena);
+        memcpy(ctx->h_stage, rb, sizeof(Board) * n);
+        memcpy(ctx->h_stage + at, rs, n);
+        PB_CUDA(cudaMemcpyAsync(ctx->arena, ctx->h_stage, at + n, cudaMemcpyHostToDevice, s));
+    } else {
+        PB_CUDA(cudaMemcpyAsync(b0, rb, sizeof(Board) * n, cudaMemcpyHostToDevice, s));
+        PB_CUDA(cudaMemcpyAsync(s0, rs, n, cudaMemcpyHostToDevice, s));
+    }
     PB_CUDA(cudaMemsetAsync(rc, 0, sizeof(unsigned long long) * n, s));
-    PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));
+    PB_CUDA(cudaMemsetAsync(ctx->d_counter, 0, SCRATCH_BYTES, s));
     stats.h2d_bytes += (sizeof(Board) + 1 + 4) * n;
     if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[0], s));
     if (depth == 1) {
@@ -1007,100 +1144,105 @@ int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth,
         stats.d2h_bytes += 4 * n;
         return PB_OK;
     }
-    // root moves as the first edges
-    k_count_positions<WHITE, true><<<grid_for(n, 256), 256, 0, s>>>(b0, s0, n, cnt0);
-    PB_CUDA(cudaMemsetAsync(status0, 0, sizeof(u64) * tiles0, s));
-    PB_CUDA(cudaMemsetAsync(ctx->d_ticket, 0, sizeof(u32), s));
-    k_scan<<<(unsigned)tiles0, SCAN_THREADS, 0, s>>>(cnt0, n, off0, status0, ctx->d_ticket, ctx->d_total, ctx->d_err);
-    PB_CUDA(cudaGetLastError());
-    PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_total, sizeof(u64), cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaStreamSynchronize(s));
-    stats.kernels += 2;
-    u64 ne = ctx->h_pinned[0];
-    if (ne > 0xFFFFFFFFULL) {
-        *bfs_status = BFS_TOO_BIG;
-        return PB_OK;
-    }
-    uint16_t *emv = ar.take<uint16_t>(ne ? ne : 1);
-    u32 *epi = ar.take<u32>(ne ? ne : 1);
-    if (!emv || !epi) {
-        *bfs_status = BFS_TOO_BIG;
-        return PB_OK;
-    }
-    if (ne) {
-        k_generate<WHITE><<<grid_for(n, GEN_THREADS), GEN_THREADS, 0, s>>>(b0, s0, off0, ctx->d_total, n, emv, epi,
-                                                                         ctx->d_err);
-        PB_CUDA(cudaGetLastError());
-        stats.kernels += 1;
-    }
-    if (stats.levels < 16) stats.level_sizes[stats.levels] = ne;
     Board *cur_b = b0;
     uint8_t *cur_s = s0;
     u32 *cur_r = r0;
-    u64 n_par = n;
-    int c = WHITE;
-    for (int rem = depth - 1; rem > 2 && ne; rem--) {
-        Board *cb = ar.take<Board>(ne);
-        uint8_t *cs = ar.take<uint8_t>(ne);
-        u32 *cr = ar.take<u32>(ne);
-        u32 *cnt = ar.take<u32>(ne);
-        u64 *offs = ar.take<u64>(ne);
-        u64 tiles = (ne + SCAN_TILE - 1) / SCAN_TILE;
-        u64 *status = ar.take<u64>(tiles);
-        if (!cb || !cs || !cr || !cnt || !offs || !status) {
+    uint16_t *emv = nullptr;
+    u32 *epi = nullptr;
+    u64 ne = n, n_par = n;
+    int c = WHITE, wide_levels = 0;
+    std::vector<u32> iota;
+    // One level: the children of the current edges (at first the roots as they
+    // are) and their moves as the next edges.
+    for (int rem = depth; (rem == depth || rem > 2) && ne; rem--) {
+        const bool roots = rem == depth;
+        const u64 m = ne;
+        Board *cb = roots ? b0 : ar.take<Board>(m);
+        uint8_t *cs = roots ? s0 : ar.take<uint8_t>(m);
+        u32 *cr = roots ? r0 : ar.take<u32>(m);
+        u64 *offs = off0;
+        uint16_t *nmv = nullptr;
+        u32 *npi = nullptr;
+        const bool whole = wide_level(ctx, m) && wide_levels < WIDE_LEVELS;
+        unsigned long long *total = reinterpret_cast<unsigned long long *>(ctx->d_total);
+        if (!cb || !cs || !cr) {
             *bfs_status = BFS_TOO_BIG;
             return PB_OK;
         }
-        unsigned g = grid_for(ne, 256);
-        if (c == WHITE)
-            k_expand_count_rooted<WHITE><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, cb, cs, cr, cnt, ctx->d_err);
-        else
-            k_expand_count_rooted<BLACK><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, cb, cs, cr, cnt, ctx->d_err);
-        PB_CUDA(cudaMemsetAsync(status, 0, sizeof(u64) * tiles, s));
-        PB_CUDA(cudaMemsetAsync(ctx->d_ticket, 0, sizeof(u32), s));
-        k_scan<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(cnt, ne, offs, status, ctx->d_ticket, ctx->d_total, ctx->d_err);
+        if (whole) {
+            total += 1 + wide_levels++;
+            nmv = ar.take<uint16_t>(m * MAX_MOVES);
+            npi = ar.take<u32>(m * MAX_MOVES);
+            if (!nmv || !npi) {
+                *bfs_status = BFS_TOO_BIG;
+                return PB_OK;
+            }
+            launch_level_wide(ctx, c, cur_b, cur_s, cur_r, roots ? nullptr : epi, emv, m, n_par, cb, cs, cr, nmv, npi,
+                              total);
+        } else {
+            u32 *cnt = cnt0;
+            if (roots) {
+                iota.resize(n);
+                for (u64 i = 0; i < n; i++) iota[i] = (u32)i;
+                PB_CUDA(cudaMemcpyAsync(r0, iota.data(), sizeof(u32) * n, cudaMemcpyHostToDevice, s));
+                k_count_positions<WHITE, true><<<grid_for(n, 256), 256, 0, s>>>(b0, s0, n, cnt0);
+            } else {
+                cnt = ar.take<u32>(m);
+                offs = ar.take<u64>(m);
+                if (!cnt || !offs) {
+                    *bfs_status = BFS_TOO_BIG;
+                    return PB_OK;
+                }
+                const unsigned g = grid_for(m, 256);
+                if (c == WHITE)
+                    k_expand_count_rooted<WHITE><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, m, n_par, cb, cs, cr, cnt, ctx->d_err);
+                else
+                    k_expand_count_rooted<BLACK><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, m, n_par, cb, cs, cr, cnt, ctx->d_err);
+            }
+            if (!launch_scan(ctx, ar, cnt, m, offs)) {
+                *bfs_status = BFS_TOO_BIG;
+                return PB_OK;
+            }
+        }
         PB_CUDA(cudaGetLastError());
-        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_total, sizeof(u64), cudaMemcpyDeviceToHost, s));
-        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned + 1, ctx->d_err, sizeof(u32), cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, SCRATCH_BYTES, cudaMemcpyDeviceToHost, s));
         PB_CUDA(cudaStreamSynchronize(s));
         stats.kernels += 2;
-        stats.d2h_bytes += 12;
-        if ((u32)ctx->h_pinned[1]) return fail(ctx, PB_ERR_DEVICE, "batched level reported a device error");
-        u64 next = ctx->h_pinned[0];
-        stats.levels++;
+        stats.d2h_bytes += SCRATCH_BYTES;
+        if ((u32)ctx->h_pinned[SCRATCH_ERR]) return fail(ctx, PB_ERR_DEVICE, "batched level reported a device error");
+        const u64 next = ctx->h_pinned[total - ctx->d_counter];
+        if (!roots) stats.levels++;
         if (stats.levels < 16) stats.level_sizes[stats.levels] = next;
         cur_b = cb;
         cur_s = cs;
         cur_r = cr;
-        n_par = ne;
-        c = 1 - c;
+        n_par = m;
+        if (!roots) c = 1 - c;
         if (next > 0xFFFFFFFFULL) {
             *bfs_status = BFS_TOO_BIG;
             return PB_OK;
         }
-        uint16_t *nmv = ar.take<uint16_t>(next ? next : 1);
-        u32 *npi = ar.take<u32>(next ? next : 1);
-        if (!nmv || !npi) {
-            *bfs_status = BFS_TOO_BIG;
-            return PB_OK;
-        }
-        if (next) {
-            if (c == WHITE)
-                k_generate<WHITE><<<grid_for(n_par, GEN_THREADS), GEN_THREADS, 0, s>>>(cb, cs, offs, ctx->d_total, n_par, nmv, npi, ctx->d_err);
-            else
-                k_generate<BLACK><<<grid_for(n_par, GEN_THREADS), GEN_THREADS, 0, s>>>(cb, cs, offs, ctx->d_total, n_par, nmv, npi, ctx->d_err);
+        if (!whole) {
+            nmv = ar.take<uint16_t>(next ? next : 1);
+            npi = ar.take<u32>(next ? next : 1);
+            if (!nmv || !npi) {
+                *bfs_status = BFS_TOO_BIG;
+                return PB_OK;
+            }
+            if (next) launch_generate(ctx, c, cb, cs, offs, m, nmv, npi);
             PB_CUDA(cudaGetLastError());
-            stats.kernels += 1;
         }
+        if (next) stats.kernels += 1;
         emv = nmv;
         epi = npi;
         ne = next;
     }
     const FoldQueue queue = fold_queue(ctx, ar);
     const bool fold = leaf_mode(ctx) == 3 && depth > 2 && fold_fits(queue);
-    std::vector<unsigned long long> tmp(n);
+    std::vector<unsigned long long> many(few ? 0 : n);
+    unsigned long long *tmp = few ? reinterpret_cast<unsigned long long *>(ctx->h_stage) : many.data();
     for (int attempt = 0;; attempt++) {
-        PB_CUDA(reset_counters(ctx));
+        if (attempt) PB_CUDA(reset_counters(ctx));
         if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[1], s));
         if (ne) {
             if (depth == 2) {
@@ -1112,6 +1254,8 @@ int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth,
                     if (strict) k_leaf1_rooted<BLACK, true><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
                     else k_leaf1_rooted<BLACK, false><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
                 }
+            } else if (leaf_mode(ctx) == 3 && ne <= WIDE_MAX) {
+                launch_leaf_wide(ctx, c, strict, cur_b, cur_s, cur_r, epi, emv, ne, nullptr, n_par, rc);
             } else if (fold) {
                 const LeafEdges e{cur_b, cur_s, cur_r, epi, emv, ne, n_par, nullptr, nullptr, nullptr, nullptr, nullptr};
                 PB_CUDA(launch_fold<FOLD_ROOTED>(ctx, c, strict, e, queue, attempt > 0, rc, DEVERR_QUEUE));
@@ -1149,16 +1293,15 @@ int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth,
             PB_CUDA(cudaEventRecord(ctx->ev[2], s));
             PB_CUDA(cudaEventRecord(ctx->ev[3], s));
         }
-        PB_CUDA(cudaMemcpyAsync(tmp.data(), rc, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, s));
-        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, 2 * sizeof(u64), cudaMemcpyDeviceToHost, s));
-        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned + 2, ctx->d_err, sizeof(u32), cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaMemcpyAsync(tmp, rc, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, s));
+        PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, SCRATCH_BYTES, cudaMemcpyDeviceToHost, s));
         PB_CUDA(cudaStreamSynchronize(s));
-        if ((u32)ctx->h_pinned[2] != DEVERR_QUEUE || attempt > 0) break;
+        if ((u32)ctx->h_pinned[SCRATCH_ERR] != DEVERR_QUEUE || attempt > 0) break;
         // a queue was too short: the leaf again, in chunks that always fit
         PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));
         PB_CUDA(cudaMemsetAsync(rc, 0, sizeof(unsigned long long) * n, s));
     }
-    if ((u32)ctx->h_pinned[2]) return fail(ctx, PB_ERR_DEVICE, "batched leaf reported a device error");
+    if ((u32)ctx->h_pinned[SCRATCH_ERR]) return fail(ctx, PB_ERR_DEVICE, "batched leaf reported a device error");
     if (ne) stats.kernels += 1;
     for (u64 i = 0; i < n; i++) out[i] = tmp[i];
     stats.leaf_edges += ne;
@@ -2027,12 +2170,13 @@ int pb_create(int device, const pb_opts *opts, pb_ctx **out)
             }
             if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess) { rc = cuda_fail(ctx, e, "stream"); break; }
             char *small = nullptr;
-            if ((e = cudaMalloc(&small, 256)) != cudaSuccess) { rc = cuda_fail(ctx, e, "scratch"); break; }
+            if ((e = cudaMalloc(&small, SCRATCH_BYTES)) != cudaSuccess) { rc = cuda_fail(ctx, e, "scratch"); break; }
             ctx->d_counter = reinterpret_cast<unsigned long long *>(small);  // two words
             ctx->d_err = reinterpret_cast<u32 *>(small + 64);
             ctx->d_ticket = reinterpret_cast<u32 *>(small + 128);
             ctx->d_total = reinterpret_cast<u64 *>(small + 192);
-            if ((e = cudaMallocHost(&ctx->h_pinned, 4096)) != cudaSuccess) { rc = cuda_fail(ctx, e, "pinned"); break; }
+            if ((e = cudaMallocHost(&ctx->h_pinned, 4096 + STAGE_BYTES)) != cudaSuccess) { rc = cuda_fail(ctx, e, "pinned"); break; }
+            ctx->h_stage = reinterpret_cast<char *>(ctx->h_pinned) + 4096;
             if ((e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) { rc = cuda_fail(ctx, e, "sm count"); break; }
             ctx->spill_blocks = (size_t)ctx->num_sms * 8;
             if ((e = cudaMalloc(&ctx->spill, ctx->spill_blocks * LEAF_T * LEAF_OVF * sizeof(uint16_t))) != cudaSuccess) { rc = cuda_fail(ctx, e, "spill"); break; }

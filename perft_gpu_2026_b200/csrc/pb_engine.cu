@@ -231,6 +231,12 @@ inline u64 fold_chunk(const FoldQueue &q, u64 n, bool careful)
 // waves either size takes the same time; at 1.5 M edges small ones take 11 % more).
 inline bool fold_small(const pb_ctx *ctx, u64 m) { return m < (u64)ctx->num_sms * FOLD_THREADS_PER_SM; }
 
+// Grid of k_fold_count for a chunk of m edges (one to a dozen queued moves each).
+inline unsigned fold_count_grid(const pb_ctx *ctx, u64 m)
+{
+    return (unsigned)std::min<u64>((u64)ctx->num_sms * 64, grid_for(m * 4, 256));
+}
+
 // Zeroes the counters and the first chunk's queue cursor (one 64-byte block).
 inline cudaError_t reset_counters(pb_ctx *ctx) { return cudaMemsetAsync(ctx->d_counter, 0, 64, ctx->stream); }
 
@@ -254,9 +260,7 @@ cudaError_t launch_fold_t(pb_ctx *ctx, const LeafEdges &e, const FoldQueue &q, b
         else
             k_fold<C, S, FOLD_THREADS, OUT><<<grid_for(m, FOLD_THREADS), FOLD_THREADS, 0, s>>>(
                 e, first, m, q, rc, ctx->d_counter, ctx->d_err);
-        // at most a few queued moves per thread of a small launch
-        const unsigned g = (unsigned)std::min<u64>((u64)ctx->num_sms * 4, grid_for(m * 16, 256));
-        k_fold_count<C, S, OUT><<<g, 256, 0, s>>>(e, q, rc, ctx->d_counter, overflow, ctx->d_err);
+        k_fold_count<C, S, OUT><<<fold_count_grid(ctx, m), 256, 0, s>>>(e, q, rc, ctx->d_counter, overflow, ctx->d_err);
     }
     return cudaGetLastError();
 }
@@ -692,8 +696,7 @@ cudaError_t launch_tt_fold_t(pb_ctx *ctx, const TTFold &f, const Board *b, const
         else
             k_fold<C, S, FOLD_THREADS, FOLD_EACH><<<grid_for(m, FOLD_THREADS), FOLD_THREADS, 0, s>>>(
                 e, 0, m, f.q, nullptr, ctx->d_counter, ctx->d_err);
-        const unsigned g = (unsigned)std::min<u64>((u64)ctx->num_sms * 4, grid_for(m * 16, 256));
-        k_fold_count<C, S, FOLD_EACH><<<g, 256, 0, s>>>(e, f.q, nullptr, ctx->d_counter, DEVERR_QUEUE, ctx->d_err);
+        k_fold_count<C, S, FOLD_EACH><<<fold_count_grid(ctx, m), 256, 0, s>>>(e, f.q, nullptr, ctx->d_counter, DEVERR_QUEUE, ctx->d_err);
         k_tt_keep<<<grid_for(m, 256), 256, 0, s>>>(f.ch, first, (u32)m, out, tv);
         if (gen == (1u << (32 - TT_AT_BITS)) - 1) gen = 0;
     }

@@ -160,7 +160,22 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
     u64 ring_b = 0, ring_r = 0;     // ... on the ring
     u64 keep = path, lines = path;  // squares no simple move leaves / enters
     u64 pinned_y = 0;
-    u64 threat = 0, multi = 0;      // zone squares X attacks / attacks more than once
+    u64 threat, multi;              // squares X attacks / attacks more than once, exact on the zone
+    {
+        u64 one = cap_west<X>(s.pawns & us), two, q = cap_east<X>(s.pawns & us);
+        two = one & q;
+        one |= q;
+        q = king_att(xk);
+        two |= one & q;
+        one |= q;
+        for (u64 kn = s.knights & us; kn; kn &= kn - 1) {
+            q = knight_att(lsb(kn));
+            two |= one & q;
+            one |= q;
+        }
+        threat = one;
+        multi = two;
+    }
     {
         u64 a = bishop_att(yk, occ);
         core_b = a | bishop_att(yk, occ & ~(a & them));
@@ -187,10 +202,11 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
             core_b |= a, core_r |= c;
         else
             ring_b |= a, ring_r |= c;
-        const u64 attackers = (a & bqX) | (c & rqX) | (knight_att(q) & s.knights & us) |
-                              ((cap_west<Y>(zb) | cap_east<Y>(zb)) & s.pawns & us) | (king_att(q) & xkb);
-        if (attackers) threat |= zb;
-        if (more_than_one(attackers)) multi |= zb;
+        const u64 attackers = (a & bqX) | (c & rqX);
+        if (attackers) {
+            multi |= zb & (more_than_one(attackers) ? ~0ULL : threat);
+            threat |= zb;
+        }
         for (u64 t = (bishop_empty(q) & bqX) | (rook_empty(q) & rqX); t; t &= t - 1) {
             const u64 bw = between(lsb(t), q), bt = bw & occ_k;
             if (!bt)
@@ -480,85 +496,89 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
         if (any & a & them) corr += to.sum(a & them);
         if (any & bit) corr -= to.at(bit) * mob;
     }
-    u64 bs = bY, rs = rY;
-    while (bs | rs) {
-        // one slider: its own moves, the squares of simple moves it sees, and
-        // the pieces with simple moves it sees
-        const bool diag = bs != 0;
-        const u64 bit = diag ? bs & (0 - bs) : rs & (0 - rs);
-        const int sq = diag ? lsb(bs) : lsb(rs);
-        const Magic *e = diag ? &PB_TAB.bishop[sq] : &PB_TAB.rook[sq];
-        if (diag)
-            bs ^= bit;
-        else
-            rs ^= bit;
-        const u64 a = magic_lookup(e, occ);
-        const int mob = popc(a & ~them);
-        base += mob;
-        if (!((a | bit) & any) && !(a & movers)) continue;
-        if (any & bit) corr -= to.at(bit) * mob;
-        if (any & a & them) corr += to.sum(a & them);
-        // the nearest such square of each ray at once: a lookup with them
-        // occupied loses what is beyond them
-        const u64 view = a & empty;
-        for (u64 h = to.c0 & view; h;) {
-            const u64 cut = magic_lookup(e, occ | h);
-            corr -= mob - popc(cut & ~them);
-            h &= ~cut;
-        }
-        for (u64 h = to.c1 & view; h;) {
-            const u64 cut = magic_lookup(e, occ | h);
-            corr -= 2 * (mob - popc(cut & ~them));
-            h &= ~cut;
-        }
-        for (u64 h = to.c2 & view; h;) {
-            const u64 cut = magic_lookup(e, occ | h);
-            corr -= 4 * (mob - popc(cut & ~them));
-            h &= ~cut;
-        }
-        if (to.rare()) {
+    // Y's sliders, diagonal movers first (a loop per kind: 1.3 % faster than one
+    // that selects)
 #pragma unroll 1
-            for (int k = 0; k < 2; k++)
-                for (u64 h = (k ? to.c4 : to.c3) & view; h;) {
+    for (int kind = 0; kind < 2; kind++) {
+        const bool diag = kind == 0;
+        const Magic *table = diag ? PB_TAB.bishop : PB_TAB.rook;
+        const u64 alike = diag ? bqX : rqX, y_alike = diag ? bY : rY;
+        for (u64 set = y_alike; set; set &= set - 1) {
+            // one slider: its own moves, the squares of simple moves it sees, and
+            // the pieces with simple moves it sees
+            const u64 bit = set & (0 - set);
+            const int sq = lsb(set);
+            const Magic *e = table + sq;
+            const u64 a = magic_lookup(e, occ);
+            const int mob = popc(a & ~them);
+            base += mob;
+            if (!((a | bit) & any) && !(a & movers)) continue;
+            if (any & bit) corr -= to.at(bit) * mob;
+            if (any & a & them) corr += to.sum(a & them);
+            // the nearest such square of each ray at once: a lookup with them
+            // occupied loses what is beyond them
+            const u64 view = a & empty;
+            if (any & view) {
+                for (u64 h = to.c0 & view; h;) {
                     const u64 cut = magic_lookup(e, occ | h);
-                    corr -= (8 << k) * (mob - popc(cut & ~them));
+                    corr -= mob - popc(cut & ~them);
                     h &= ~cut;
                 }
-        }
-        for (u64 g = a & movers; g; g &= g - 1) {
-            const u64 fb = g & (0 - g);
-            int n;
-            if (fb & s.pawns) {
-                n = (fb & moved0 ? 1 : 0) + (fb & moved1 ? 2 : 0) + (fb & moved2 ? 4 : 0);
-            } else {
-                n = (int)(moved >> (5 * popc(pieces & (fb - 1)))) & 31;
-            }
-            const int f = lsb(g);
-            const u64 open = magic_lookup(e, occ ^ fb);
-            const int ext = popc(open & ~them) - mob;
-            corr += ext * n;
-            // moves of f along the same line
-            if (!(fb & (s.pawns | (diag ? bqX : rqX)))) continue;
-            const u64 past = open & beyond(sq, f);
-            u64 line = 0;
-            if (fb & s.pawns) {
-                if (diag) {
-                    line = (cap_west<X>(fb) | cap_east<X>(fb)) & past & them & ~bY & safe & ok_to;
-                } else if (((sq ^ f) & 7) == 0) {
-                    const u64 d = push1<X>(fb) & empty;
-                    line = (d | (push1<X>(d & DP_X) & empty & ~flagged)) & safe & ok_to;
+                for (u64 h = to.c1 & view; h;) {
+                    const u64 cut = magic_lookup(e, occ | h);
+                    corr -= 2 * (mob - popc(cut & ~them));
+                    h &= ~cut;
                 }
-            } else {
-                u64 no = stay | us | (past & (diag ? bY : rY)) | (fp & (king_att(f) | push1<X>(push1<X>(fb))));
-                if (fb & bqX) no |= core_b;
-                if (fb & rqX) no |= core_r;
-                line = (between(sq, f) | past) & safe & ~no;
-                if (fb & pinned_x) line &= line_through(f, xk);
+                for (u64 h = to.c2 & view; h;) {
+                    const u64 cut = magic_lookup(e, occ | h);
+                    corr -= 4 * (mob - popc(cut & ~them));
+                    h &= ~cut;
+                }
+                if (to.rare()) {
+#pragma unroll 1
+                    for (int k = 0; k < 2; k++)
+                    for (u64 h = (k ? to.c4 : to.c3) & view; h;) {
+                        const u64 cut = magic_lookup(e, occ | h);
+                        corr -= (8 << k) * (mob - popc(cut & ~them));
+                        h &= ~cut;
+                    }
+                }
             }
-            if (line) {
-                corr -= ext * popc(line & ~past);
-                corr += popc(line & them);
-                for (u64 t = line & past & empty; t; t &= t - 1) corr -= popc(past & beyond(sq, lsb(t)) & ~them);
+            for (u64 g = a & movers; g; g &= g - 1) {
+                const u64 fb = g & (0 - g);
+                int n;
+                if (fb & s.pawns) {
+                    n = (fb & moved0 ? 1 : 0) + (fb & moved1 ? 2 : 0) + (fb & moved2 ? 4 : 0);
+                } else {
+                    n = (int)(moved >> (5 * popc(pieces & (fb - 1)))) & 31;
+                }
+                const int f = lsb(g);
+                const u64 open = magic_lookup(e, occ ^ fb);
+                const int ext = popc(open & ~them) - mob;
+                corr += ext * n;
+                // moves of f along the same line
+                if (!(fb & (s.pawns | alike))) continue;
+                const u64 past = open & beyond(sq, f);
+                u64 line = 0;
+                if (fb & s.pawns) {
+                    if (diag) {
+                        line = (cap_west<X>(fb) | cap_east<X>(fb)) & past & them & ~bY & safe & ok_to;
+                    } else if (((sq ^ f) & 7) == 0) {
+                        const u64 d = push1<X>(fb) & empty;
+                        line = (d | (push1<X>(d & DP_X) & empty & ~flagged)) & safe & ok_to;
+                    }
+                } else {
+                    u64 no = stay | us | (past & y_alike) | (fp & (king_att(f) | push1<X>(push1<X>(fb))));
+                    if (fb & bqX) no |= core_b;
+                    if (fb & rqX) no |= core_r;
+                    line = (between(sq, f) | past) & safe & ~no;
+                    if (fb & pinned_x) line &= line_through(f, xk);
+                }
+                if (line) {
+                    corr -= ext * popc(line & ~past);
+                    corr += popc(line & them);
+                    for (u64 t = line & past & empty; t; t &= t - 1) corr -= popc(past & beyond(sq, lsb(t)) & ~them);
+                }
             }
         }
     }

@@ -5,26 +5,29 @@
 // simple moves (fold_child) and appends its other moves to a queue in device
 // memory; k_fold_count makes the queued moves and counts each of them in full,
 // one per thread.  Both are bound by integer issue.  The queue between them
-// costs 16 B of traffic per queued move (two per child on the benchmark's
-// leaves, seven on middle-game playouts) and buys full warps in both halves,
-// no barriers, and 55 + 20 KB of code instead of one kernel whose warps fetch
-// from both at once (one kernel with a shared-memory queue and a barrier
-// between the halves: 10.9 ms against 8.15 ms on the benchmark's leaves).
+// costs 16 B of traffic per queued move (one per child on the benchmark's
+// leaves, five on middle-game playouts) and buys full warps in both halves, no
+// barriers, and 55 + 20 KB of code instead of one kernel whose warps fetch from
+// both at once (one kernel with a shared-memory queue and a barrier between the
+// halves: 10.9 ms against 8.15 ms for the first form of these two on the
+// benchmark's leaves).
 //
 // Measured on B200 against the leaf that makes and counts every move
 // (balanced, listed pieces; the benchmark's 27.2 M edges, 774 M moves):
-// 20.09 -> 8.15 ms (k_fold 5.99, k_fold_count 2.16); 5.2 M edges of 6-40 ply
-// playouts 5.33 -> 2.95 ms; 4.2 M edges of 60-140 ply playouts 4.26 -> 3.63 ms.
+// 20.09 -> 7.72 ms (k_fold 6.58, k_fold_count 1.14); 5.2 M edges of 6-40 ply
+// playouts 5.33 -> 2.41 ms; 4.2 M edges of 60-140 ply playouts 4.26 -> 2.18 ms.
 #pragma once
 #include "pb_fold.cuh"
 #include "pb_kernels.cuh"
 
 namespace pb {
 
-// k_fold's CTA: 80 registers a thread, 24 warps per SM.  On the benchmark's
-// leaves 24 warps ran 5.99 ms, 32 (64 registers, spills) 6.54, 16 (128
-// registers) 6.74; at the same 24 warps, CTAs of 128 / 384 / 768 threads 6.48 /
-// 6.10 / 6.38.  Small launches use 64 threads so that they reach every SM.
+// k_fold's CTA: 96 registers a thread, 20 warps per SM.  On the benchmark's
+// leaves 20 warps ran 6.69 ms, 24 (80 registers, spills) 7.13, 32 (64 registers)
+// 7.94.  The code is long and straight, so warps that start together share its
+// instruction fetches: at the same 20 warps CTAs of 128 threads ran 7.83 ms
+// (barriers between the stages gained nothing more).  Small launches use 64
+// threads so that they reach every SM.
 constexpr int FOLD_THREADS = 320;
 constexpr int FOLD_SMALL_THREADS = 64;
 constexpr int FOLD_THREADS_PER_SM = 640;
@@ -162,10 +165,13 @@ __global__ void __launch_bounds__(T, FOLD_THREADS_PER_SM / T)
     }
 }
 
-// Counts the queued moves (a fixed grid strides over them; their number is on
-// the device).  A queue that was too short sets `overflow` in the error word.
+// Counts the queued moves (the grid strides over them; their number is on the
+// device).  A queue that was too short sets `overflow` in the error word.  Bound
+// by integer issue behind the table loads: 40 warps per SM (48 registers, a few
+// spills) against 32, and 64 CTAs per SM that come and go against 4 that stay,
+// took 24.2 M moves of middle-game playouts from 0.99 to 0.85 ms.
 template <int C, bool STRICT, FoldOut OUT>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, 5)
     k_fold_count(const __grid_constant__ LeafEdges e, const __grid_constant__ FoldQueue queue,
                  unsigned long long *__restrict__ root_counts, unsigned long long *__restrict__ counter,
                  u32 overflow, u32 *__restrict__ err)

@@ -338,6 +338,8 @@ int launch_leaf_t(pb_ctx *ctx, const Board *b, const uint8_t *st, const u32 *pi,
     }
     u64 grid = std::min<u64>(nchunks, (u64)ctx->num_sms * per_sm);
     if (grid > ctx->spill_blocks) return fail(ctx, PB_ERR_NOMEM, "leaf spill area too small");
+    if (!ctx->spill)  // 130 MB that only this leaf uses
+        PB_CUDA(cudaMalloc(&ctx->spill, ctx->spill_blocks * LEAF_T * LEAF_OVF * sizeof(uint16_t)));
     k_leaf2_coop<C, S><<<(unsigned)grid, LEAF_T, 0, s>>>(b, st, pi, mv, n, npar, ctx->spill, ctx->d_counter);
     PB_CUDA(cudaGetLastError());
     return PB_OK;
@@ -2182,7 +2184,6 @@ int pb_create(int device, const pb_opts *opts, pb_ctx **out)
             ctx->h_stage = reinterpret_cast<char *>(ctx->h_pinned) + 4096;
             if ((e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) { rc = cuda_fail(ctx, e, "sm count"); break; }
             ctx->spill_blocks = (size_t)ctx->num_sms * 8;
-            if ((e = cudaMalloc(&ctx->spill, ctx->spill_blocks * LEAF_T * LEAF_OVF * sizeof(uint16_t))) != cudaSuccess) { rc = cuda_fail(ctx, e, "spill"); break; }
             size_t freeb = 0, totalb = 0;
             cudaMemGetInfo(&freeb, &totalb);
             size_t want = ctx->opts.arena_bytes;
@@ -2557,6 +2558,18 @@ int pb_perft_batch(pb_ctx *ctx, const pb_pos *roots, const int *depths, int n, u
     if (!ctx->gpu) return fail(ctx, PB_ERR_NODEVICE, "context has no GPU");
     PB_CUDA(cudaSetDevice(ctx->device));
     memset(&ctx->stats, 0, sizeof(ctx->stats));
+    // all at one depth: in the caller's order, counts straight to the caller
+    if (n > 0 && std::all_of(depths, depths + n, [&](int d) { return d == depths[0]; })) {
+        if (depths[0] < 0 || depths[0] > 20) return PB_ERR_ARG;
+        std::vector<Board> rb(n);
+        std::vector<uint8_t> rs(n);
+        for (int i = 0; i < n; i++) to_white_to_move(roots[i], rb[i], rs[i]);
+        static_assert(sizeof(uint64_t) == sizeof(u64), "counts are written in place");
+        int rc = gpu_batch(ctx, rb.data(), rs.data(), (u64)n, depths[0], reinterpret_cast<u64 *>(counts));
+        if (rc != PB_OK) return rc;
+        for (int i = 0; i < n; i++) ctx->stats.nodes += counts[i];
+        return PB_OK;
+    }
     // one batched pass per distinct depth
     std::vector<int> ds(depths, depths + n);
     std::sort(ds.begin(), ds.end());

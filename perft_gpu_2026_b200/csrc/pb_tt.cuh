@@ -130,8 +130,32 @@ struct HostEntry {
     u64 lo, hi, count;
 };
 
+// One depth's entries, zero pages until written: filling them up front took 17 ms
+// of a run's start per 64 MB, most of which a run never touches.
+struct HostSlots {
+    HostEntry *p = nullptr;
+    u64 n = 0;
+    HostSlots() = default;
+    HostSlots(HostSlots &&o) noexcept : p(o.p), n(o.n) { o.p = nullptr, o.n = 0; }
+    HostSlots(const HostSlots &) = delete;
+    HostSlots &operator=(const HostSlots &) = delete;
+    ~HostSlots() { free(p); }
+    // false (and no entries) if there is no memory
+    bool alloc(u64 slots)
+    {
+        free(p);
+        p = static_cast<HostEntry *>(calloc(slots, sizeof(HostEntry)));
+        n = p ? slots : 0;
+        return p != nullptr;
+    }
+    bool empty() const { return n == 0; }
+    u64 size() const { return n; }
+    HostEntry &operator[](u64 i) { return p[i]; }
+    const HostEntry &operator[](u64 i) const { return p[i]; }
+};
+
 struct HostTT {
-    std::vector<std::vector<HostEntry>> tab;  // per remaining depth
+    std::vector<HostSlots> tab;  // per remaining depth
     std::vector<u64> used;
     bool ok = false;
 
@@ -150,7 +174,8 @@ struct HostTT {
             u64 total = (pages > 0 && psz > 0) ? (u64)pages * (u64)psz : (8ULL << 30);
             budget = std::min<u64>(total / 4, 32ULL << 30);
         }
-        tab.assign(last + 1, {});
+        tab.clear();
+        tab.resize(last + 1);
         used.assign(last + 1, 0);
         double wsum = 0;
         for (int d = first; d <= last; d++) wsum += pow(30.0, last - d);
@@ -159,14 +184,14 @@ struct HostTT {
             u64 slots = (u64)(budget * w) / sizeof(HostEntry);
             u64 p2 = 1024;
             while (p2 * 2 <= slots) p2 *= 2;
-            tab[d].assign(p2, HostEntry{0, 0, 0});
+            tab[d].alloc(p2);
         }
         ok = true;
     }
     bool probe(int depth, const Hash128 &h, u64 *out) const
     {
         if (depth >= (int)tab.size() || tab[depth].empty()) return false;
-        const std::vector<HostEntry> &t = tab[depth];
+        const HostSlots &t = tab[depth];
         u64 mask = t.size() - 1;
         for (u64 i = h.lo & mask, k = 0; k < 64; k++, i = (i + 1) & mask) {
             const HostEntry &e = t[i];
@@ -181,7 +206,7 @@ struct HostTT {
     void store(int depth, const Hash128 &h, u64 count)
     {
         if (depth >= (int)tab.size() || tab[depth].empty()) return;
-        std::vector<HostEntry> &t = tab[depth];
+        HostSlots &t = tab[depth];
         if (used[depth] * 4 >= t.size() * 3) return;  // keep the load factor bounded
         u64 mask = t.size() - 1;
         for (u64 i = h.lo & mask, k = 0; k < 64; k++, i = (i + 1) & mask) {

@@ -240,6 +240,19 @@ inline unsigned fold_count_grid(const pb_ctx *ctx, u64 m)
 // Zeroes the counters and the first chunk's queue cursor (one 64-byte block).
 inline cudaError_t reset_counters(pb_ctx *ctx) { return cudaMemsetAsync(ctx->d_counter, 0, 64, ctx->stream); }
 
+// k_fold over edges [first, first + m) in CTAs of T threads.
+template <int C, bool S, int T, FoldOut OUT>
+cudaError_t launch_fold_kernel(pb_ctx *ctx, const LeafEdges &e, u64 first, u64 m, const FoldQueue &q,
+                               unsigned long long *rc)
+{
+    constexpr int SHELF = T * FOLD_SHELF_BYTES;
+    if (T == FOLD_THREADS) {  // with the stage more than 48 KB
+        cudaError_t r = cudaFuncSetAttribute(k_fold<C, S, T, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SHELF);
+        if (r != cudaSuccess) return r;
+    }
+    k_fold<C, S, T, OUT><<<grid_for(m, T), T, SHELF, ctx->stream>>>(e, first, m, q, rc, ctx->d_counter, ctx->d_err);
+    return cudaSuccess;
+}
 // The folded leaf over e.n edges; `overflow` is the error bit of a queue that
 // was too short.  The caller has reset the counters.
 template <int C, bool S, FoldOut OUT>
@@ -254,12 +267,9 @@ cudaError_t launch_fold_t(pb_ctx *ctx, const LeafEdges &e, const FoldQueue &q, b
             if (me != cudaSuccess) return me;
         }
         const u64 m = std::min(chunk, e.n - first);
-        if (fold_small(ctx, m))
-            k_fold<C, S, FOLD_SMALL_THREADS, OUT><<<grid_for(m, FOLD_SMALL_THREADS), FOLD_SMALL_THREADS, 0, s>>>(
-                e, first, m, q, rc, ctx->d_counter, ctx->d_err);
-        else
-            k_fold<C, S, FOLD_THREADS, OUT><<<grid_for(m, FOLD_THREADS), FOLD_THREADS, 0, s>>>(
-                e, first, m, q, rc, ctx->d_counter, ctx->d_err);
+        cudaError_t fe = fold_small(ctx, m) ? launch_fold_kernel<C, S, FOLD_SMALL_THREADS, OUT>(ctx, e, first, m, q, rc)
+                                            : launch_fold_kernel<C, S, FOLD_THREADS, OUT>(ctx, e, first, m, q, rc);
+        if (fe != cudaSuccess) return fe;
         k_fold_count<C, S, OUT><<<fold_count_grid(ctx, m), 256, 0, s>>>(e, q, rc, ctx->d_counter, overflow, ctx->d_err);
     }
     return cudaGetLastError();
@@ -692,12 +702,9 @@ cudaError_t launch_tt_fold_t(pb_ctx *ctx, const TTFold &f, const Board *b, const
         gen++;
         k_tt_keys<C><<<grid_for(m, 256), 256, 0, s>>>(b, st, h, pi, mv, first, (u32)m, npar, f.ch, gen);
         k_tt_probe<<<grid_for(m, 256), 256, 0, s>>>(f.ch, first, (u32)m, tv, out);
-        if (fold_small(ctx, m))
-            k_fold<C, S, FOLD_SMALL_THREADS, FOLD_EACH><<<grid_for(m, FOLD_SMALL_THREADS), FOLD_SMALL_THREADS, 0, s>>>(
-                e, 0, m, f.q, nullptr, ctx->d_counter, ctx->d_err);
-        else
-            k_fold<C, S, FOLD_THREADS, FOLD_EACH><<<grid_for(m, FOLD_THREADS), FOLD_THREADS, 0, s>>>(
-                e, 0, m, f.q, nullptr, ctx->d_counter, ctx->d_err);
+        me = fold_small(ctx, m) ? launch_fold_kernel<C, S, FOLD_SMALL_THREADS, FOLD_EACH>(ctx, e, 0, m, f.q, nullptr)
+                                : launch_fold_kernel<C, S, FOLD_THREADS, FOLD_EACH>(ctx, e, 0, m, f.q, nullptr);
+        if (me != cudaSuccess) return me;
         k_fold_count<C, S, FOLD_EACH><<<fold_count_grid(ctx, m), 256, 0, s>>>(e, f.q, nullptr, ctx->d_counter, DEVERR_QUEUE, ctx->d_err);
         k_tt_keep<<<grid_for(m, 256), 256, 0, s>>>(f.ch, first, (u32)m, out, tv);
         if (gen == (1u << (32 - TT_AT_BITS)) - 1) gen = 0;
@@ -2090,7 +2097,10 @@ u64 check_fold_t(const Board &y, u32 ys, u64 *checked, u64 *made)
         for (int k = 0; k < all.n; k++) want.count<Z>(mv[k]);
         FoldSink<Z> sink{{y, ys, strict != 0, 0, 0}};
         u32 simple = 0;
-        const u32 sum = strict ? fold_child<Z, true>(y, ys, sink, &simple) : fold_child<Z, false>(y, ys, sink, &simple);
+        u64 slots[SHELF_SLOTS];
+        const Shelf shelf{slots, 1};
+        const u32 sum = strict ? fold_child<Z, true>(y, ys, sink, &simple, shelf)
+                               : fold_child<Z, false>(y, ys, sink, &simple, shelf);
         bad += sum + sink.total != want.total || simple + sink.n != want.n;
         *checked += want.n;
         *made += sink.n;

@@ -49,10 +49,42 @@
 
 namespace pb {
 
+// Values that the loops over X's pieces read seldom: on the GPU one column of
+// shared memory per thread, slots `stride` apart.  Register pressure decides how
+// many warps an SM holds; left to itself the compiler kept these and spilled
+// what every iteration reads.
+enum ShelfSlot {
+    SHELF_C3,
+    SHELF_C4,
+    SHELF_THREAT,
+    SHELF_MULTI,
+    SHELF_THREAT_Y,
+    SHELF_MOVED0,
+    SHELF_MOVED1,
+    SHELF_MOVED2,
+    SHELF_FLAGGED,
+    SHELF_OK_TO,
+    SHELF_RING_B,
+    SHELF_RING_R,
+    SHELF_CORE_B,
+    SHELF_CORE_R,
+    SHELF_PINNED_Y,
+    SHELF_SLOTS
+};
+struct Shelf {
+    volatile u64 *column;
+    int stride;
+    PB_HD u64 get(int slot) const { return column[slot * stride]; }
+    PB_HD void set(int slot, u64 v) const { column[slot * stride] = v; }
+};
+
 // Number of simple moves onto each square, bit-sliced.  Eight or more onto one
 // square (c3, c4) are rare, so their terms hide behind one test.
 struct TargetPlanes {
-    u64 c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
+    Shelf shelf;
+    u64 c0 = 0, c1 = 0, c2 = 0;
+    bool rare = false;  // c3 and c4 are set
+    PB_HD explicit TargetPlanes(Shelf s) : shelf(s) {}
     PB_HD void add(u64 s)
     {
         u64 k = c0 & s;
@@ -62,22 +94,30 @@ struct TargetPlanes {
         k = c2 & s;
         c2 ^= s;
         if (k) {
-            c4 |= c3 & k;
-            c3 ^= k;
+            if (!rare) {
+                rare = true;
+                shelf.set(SHELF_C3, k);
+                shelf.set(SHELF_C4, 0);
+            } else {
+                const u64 c3 = shelf.get(SHELF_C3);
+                shelf.set(SHELF_C4, shelf.get(SHELF_C4) | (c3 & k));
+                shelf.set(SHELF_C3, c3 ^ k);
+            }
         }
     }
-    PB_HD bool rare() const { return c3 != 0 || c4 != 0; }
+    PB_HD u64 c3() const { return shelf.get(SHELF_C3); }
+    PB_HD u64 c4() const { return shelf.get(SHELF_C4); }
     PB_HD int sum(u64 m) const
     {
         int n = popc(c0 & m) + 2 * popc(c1 & m) + 4 * popc(c2 & m);
-        if (rare()) n += 8 * popc(c3 & m) + 16 * popc(c4 & m);
+        if (rare) n += 8 * popc(c3() & m) + 16 * popc(c4() & m);
         return n;
     }
-    PB_HD u64 any() const { return c0 | c1 | c2 | c3 | c4; }
+    PB_HD u64 any() const { return c0 | c1 | c2 | (rare ? c3() | c4() : 0); }
     PB_HD int at(u64 bit) const
     {
         int n = (c0 & bit ? 1 : 0) + (c1 & bit ? 2 : 0) + (c2 & bit ? 4 : 0);
-        if (rare()) n += (c3 & bit ? 8 : 0) + (c4 & bit ? 16 : 0);
+        if (rare) n += (c3() & bit ? 8 : 0) + (c4() & bit ? 16 : 0);
         return n;
     }
 };
@@ -129,7 +169,7 @@ struct PawnTerms {
 #pragma nv_exec_check_disable  // the self-test's sink runs on the host
 #endif
 template <int X, bool STRICT, class Sink>
-PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
+PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple, Shelf shelf)
 {
     constexpr int Y = 1 - X;
     constexpr u64 KS_X = X == WHITE ? 0x60ULL : 0x6000000000000000ULL;
@@ -266,7 +306,15 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
     }
 
     // ---- X's moves
-    TargetPlanes to;
+    TargetPlanes to(shelf);
+    shelf.set(SHELF_PINNED_Y, pinned_y);
+    shelf.set(SHELF_CORE_B, core_b);
+    shelf.set(SHELF_CORE_R, core_r);
+    shelf.set(SHELF_RING_B, ring_b);
+    shelf.set(SHELF_RING_R, ring_r);
+    shelf.set(SHELF_THREAT, threat);
+    shelf.set(SHELF_MULTI, multi);
+    shelf.set(SHELF_THREAT_Y, threat_y);
     int corr = 0;
     u32 ns = 0;
 
@@ -277,6 +325,8 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
     const u64 flagged = east1(s.pawns & them) | west1(s.pawns & them);  // a double push here allows en passant
     const u64 reach_p = cap_west<Y>(ring | core) | cap_east<Y>(ring | core);
     const u64 ok_to = ~(reach_p | stay | PROMO_RANKS);
+    shelf.set(SHELF_FLAGGED, flagged);
+    shelf.set(SHELF_OK_TO, ok_to);
     {
         // pinned pawns push along their king's file and capture along its
         // diagonals; all their moves go to the sink
@@ -303,6 +353,9 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
         moved0 = x ^ fe;
         moved1 = c ^ c2;
         moved2 = c & c2;
+        shelf.set(SHELF_MOVED0, moved0);
+        shelf.set(SHELF_MOVED1, moved1);
+        shelf.set(SHELF_MOVED2, moved2);
         if ((moved0 | moved1 | moved2) & weighted) {
             const PawnTerms<Y, STRICT> w(fresh(fp), us, empty);
             const u64 plus[3] = {w.m1, w.m2, w.m3}, minus[2] = {w.cw, w.cc};
@@ -360,6 +413,14 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
         }
     }
 
+    if (!checkers) {
+        const u32 castle_x = X == WHITE ? (st & 3) : ((st >> 2) & 3);
+        constexpr int K0 = X == WHITE ? 4 : 60;
+        if ((castle_x & 1) && !(KS_X & (occ | threat_y))) sink.one(make_move_code(K0, K0 + 2, MF_KING_CASTLE), false);
+        if ((castle_x & 2) && !(QE_X & occ) && !(QS_X & threat_y))
+            sink.one(make_move_code(K0, K0 - 2, MF_QUEEN_CASTLE), false);
+    }
+
     // knights, sliders and the king, one by one.  moved: the number of simple
     // moves of each, five bits at five times its rank among them; pieces past
     // the twelfth have none (their moves go to the sink).
@@ -390,7 +451,7 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
             const u64 fb = cur & (0 - cur);
             const bool king = cur == xkb;
             const u64 a = king ? king_att(f) : knight_att(f);
-            const u64 t = a & ~us & (king ? ~threat_y : safe);
+            const u64 t = a & ~us & (king ? ~shelf.get(SHELF_THREAT_Y) : safe);
             if (t) {
                 u64 core_f = core_n, ring_f = ring_n, no = stay;
                 if (king) {
@@ -401,10 +462,11 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
                     no |= bY | rY | (fp & (a | push1<X>(push1<X>(fb))));
                 }
                 const u64 sm = ((fb & (keep | core_f)) || popc(pieces & (fb - 1)) >= 12) ? 0 : t & ~(no | core_f);
-                const u64 left = fb & ring_f ? a & ring & threat & ~multi : 0, near = sm & ring_f;
+                const u64 near = sm & ring_f;
+                const u64 left = fb & ring_f ? a & ring & shelf.get(SHELF_THREAT) & ~shelf.get(SHELF_MULTI) : 0;
                 if (near | left) {
                     // the ring squares attacked change: Y's king moves do
-                    const u64 other = threat & ~left;
+                    const u64 other = shelf.get(SHELF_THREAT) & ~left;
                     if (left) corr += (popc(ring & ~other) - kings) * popc(sm & ~near);
                     for (u64 q = near; q; q &= q - 1) {
                         const u64 att = king ? king_att(lsb(q)) : knight_att(lsb(q));
@@ -421,19 +483,21 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
     for (u64 sl = (bqX | rqX) & mine; sl; sl &= sl - 1) {
         const int f = lsb(sl);
         const u64 fb = sl & (0 - sl);
-        u64 a = 0, core_f = 0, ring_f = 0, seen = 0;
-        if (fb & bqX) {
-            a = bishop_att(f, occ);
-            seen = a & bY;
-            core_f = core_b;
-            ring_f = ring_b;
+        const bool diag = (fb & bqX) != 0;
+        u64 a = magic_lookup((diag ? PB_TAB.bishop : PB_TAB.rook) + f, occ), core_f = 0, ring_f = 0;
+        u64 seen = a & (diag ? bY : rY);
+        if (diag) {
+            core_f = shelf.get(SHELF_CORE_B);
+            ring_f = shelf.get(SHELF_RING_B);
         }
         if (fb & rqX) {
-            const u64 c = rook_att(f, occ);
-            seen |= c & rY;
-            core_f |= core_r;
-            ring_f |= ring_r;
-            a |= c;
+            core_f |= shelf.get(SHELF_CORE_R);
+            ring_f |= shelf.get(SHELF_RING_R);
+            if (diag) {
+                const u64 c = rook_att(f, occ);
+                seen |= c & rY;
+                a |= c;
+            }
         }
         u64 t = a & safe & ~us;
         if (fb & pinned_x) t &= line_through(f, xk);
@@ -442,12 +506,12 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
         const u64 sm = ((fb & (keep | core_f)) || popc(pieces & (fb - 1)) >= 12) ? 0 : t & ~no;
         u64 near = sm & ring_f, left = 0;
         if (fb & ring_f) {
-            left = a & ring & threat & ~multi;
+            left = a & ring & shelf.get(SHELF_THREAT) & ~shelf.get(SHELF_MULTI);
             // a slider that moves away along its line keeps its attack
             for (u64 z = a & ring; z; z &= z - 1) near |= sm & line_through(f, lsb(z));
         }
         if (near | left) {
-            const u64 other = threat & ~left;
+            const u64 other = shelf.get(SHELF_THREAT) & ~left;
             if (left) corr += (popc(ring & ~other) - kings) * popc(sm & ~near);
             for (u64 q = near; q; q &= q - 1) {
                 const int to_sq = lsb(q);
@@ -458,13 +522,6 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
             }
         }
         split(f, fb, t, sm);
-    }
-    if (!checkers) {
-        const u32 castle_x = X == WHITE ? (st & 3) : ((st >> 2) & 3);
-        constexpr int K0 = X == WHITE ? 4 : 60;
-        if ((castle_x & 1) && !(KS_X & (occ | threat_y))) sink.one(make_move_code(K0, K0 + 2, MF_KING_CASTLE), false);
-        if ((castle_x & 2) && !(QE_X & occ) && !(QS_X & threat_y))
-            sink.one(make_move_code(K0, K0 - 2, MF_QUEEN_CASTLE), false);
     }
 
     // ---- weights of the squares entered: Y's pawns, then its pieces
@@ -489,7 +546,7 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
             corr -= to.sum(push1<X>(w.p1)) + to.sum(push1<X>(push1<X>(w.dbl))) + to.sum(mine_y & cap_east<X>(us)) +
                     to.sum(mine_y & cap_west<X>(us));
     }
-    for (u64 kn = s.knights & them & ~pinned_y; kn; kn &= kn - 1) {
+    for (u64 kn = s.knights & them & ~shelf.get(SHELF_PINNED_Y); kn; kn &= kn - 1) {
         const u64 a = knight_att(lsb(kn)), bit = kn & (0 - kn);
         const int mob = popc(a & ~them);
         base += mob;
@@ -512,65 +569,66 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple)
             const u64 a = magic_lookup(e, occ);
             const int mob = popc(a & ~them);
             base += mob;
-            if (!((a | bit) & any) && !(a & movers)) continue;
-            if (any & bit) corr -= to.at(bit) * mob;
-            if (any & a & them) corr += to.sum(a & them);
+            if (any & ((a & them) | bit)) corr += to.sum(a & them) - to.at(bit) * mob;
+            // the squares it gains when the pieces with simple moves leave; one
+            // lookup for all, as a ray holds at most one of them
+            u64 g = a & movers;
+            const u64 opened = magic_lookup(e, occ ^ g);
             // the nearest such square of each ray at once: a lookup with them
-            // occupied loses what is beyond them
+            // occupied loses what is beyond them (two planes in flight at a
+            // time: 1 % faster than one; three lose it again)
             const u64 view = a & empty;
             if (any & view) {
-                for (u64 h = to.c0 & view; h;) {
-                    const u64 cut = magic_lookup(e, occ | h);
-                    corr -= mob - popc(cut & ~them);
-                    h &= ~cut;
-                }
-                for (u64 h = to.c1 & view; h;) {
-                    const u64 cut = magic_lookup(e, occ | h);
-                    corr -= 2 * (mob - popc(cut & ~them));
-                    h &= ~cut;
+                for (u64 h0 = to.c0 & view, h1 = to.c1 & view; h0 | h1;) {
+                    const u64 cut0 = magic_lookup(e, occ | h0), cut1 = magic_lookup(e, occ | h1);
+                    corr -= 3 * mob - popc(cut0 & ~them) - 2 * popc(cut1 & ~them);
+                    h0 &= ~cut0;
+                    h1 &= ~cut1;
                 }
                 for (u64 h = to.c2 & view; h;) {
                     const u64 cut = magic_lookup(e, occ | h);
                     corr -= 4 * (mob - popc(cut & ~them));
                     h &= ~cut;
                 }
-                if (to.rare()) {
+                if (to.rare) {
 #pragma unroll 1
-                    for (int k = 0; k < 2; k++)
-                    for (u64 h = (k ? to.c4 : to.c3) & view; h;) {
-                        const u64 cut = magic_lookup(e, occ | h);
-                        corr -= (8 << k) * (mob - popc(cut & ~them));
-                        h &= ~cut;
+                    for (int k = 0; k < 2; k++) {
+                        for (u64 h = (k ? to.c4() : to.c3()) & view; h;) {
+                            const u64 cut = magic_lookup(e, occ | h);
+                            corr -= (8 << k) * (mob - popc(cut & ~them));
+                            h &= ~cut;
+                        }
                     }
                 }
             }
-            for (u64 g = a & movers; g; g &= g - 1) {
+            for (; g; g &= g - 1) {
                 const u64 fb = g & (0 - g);
                 int n;
                 if (fb & s.pawns) {
-                    n = (fb & moved0 ? 1 : 0) + (fb & moved1 ? 2 : 0) + (fb & moved2 ? 4 : 0);
+                    n = (fb & shelf.get(SHELF_MOVED0) ? 1 : 0) + (fb & shelf.get(SHELF_MOVED1) ? 2 : 0) +
+                        (fb & shelf.get(SHELF_MOVED2) ? 4 : 0);
                 } else {
                     n = (int)(moved >> (5 * popc(pieces & (fb - 1)))) & 31;
                 }
                 const int f = lsb(g);
-                const u64 open = magic_lookup(e, occ ^ fb);
-                const int ext = popc(open & ~them) - mob;
+                const u64 past = opened & beyond(sq, f);
+                const int ext = popc(past & ~them);
                 corr += ext * n;
                 // moves of f along the same line
                 if (!(fb & (s.pawns | alike))) continue;
-                const u64 past = open & beyond(sq, f);
                 u64 line = 0;
                 if (fb & s.pawns) {
                     if (diag) {
-                        line = (cap_west<X>(fb) | cap_east<X>(fb)) & past & them & ~bY & safe & ok_to;
+                        line = (cap_west<X>(fb) | cap_east<X>(fb)) & past & them & ~bY;
                     } else if (((sq ^ f) & 7) == 0) {
                         const u64 d = push1<X>(fb) & empty;
-                        line = (d | (push1<X>(d & DP_X) & empty & ~flagged)) & safe & ok_to;
+                        line = d | (push1<X>(d & DP_X) & empty & ~shelf.get(SHELF_FLAGGED));
                     }
+                    line &= safe & shelf.get(SHELF_OK_TO);
                 } else {
                     u64 no = stay | us | (past & y_alike) | (fp & (king_att(f) | push1<X>(push1<X>(fb))));
-                    if (fb & bqX) no |= core_b;
-                    if (fb & rqX) no |= core_r;
+                    if (fb & bqX) no |= shelf.get(SHELF_CORE_B);
+                    if (fb & rqX) no |= shelf.get(SHELF_CORE_R);
                     line = (between(sq, f) | past) & safe & ~no;
                     if (fb & pinned_x) line &= line_through(f, xk);
                 }

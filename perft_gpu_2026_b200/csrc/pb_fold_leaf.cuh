@@ -14,24 +14,31 @@
 //
 // Measured on B200 against the leaf that makes and counts every move
 // (balanced, listed pieces; the benchmark's 27.2 M edges, 774 M moves):
-// 20.09 -> 7.72 ms (k_fold 6.58, k_fold_count 1.14); 5.2 M edges of 6-40 ply
-// playouts 5.33 -> 2.41 ms; 4.2 M edges of 60-140 ply playouts 4.26 -> 2.18 ms.
+// 20.09 -> 7.20 ms (k_fold 6.05, k_fold_count 1.14); 5.2 M edges of 6-40 ply
+// playouts 5.33 -> 2.27 ms; 4.2 M edges of 60-140 ply playouts 4.26 -> 2.05 ms.
 #pragma once
 #include "pb_fold.cuh"
 #include "pb_kernels.cuh"
 
 namespace pb {
 
-// k_fold's CTA: 96 registers a thread, 20 warps per SM.  On the benchmark's
-// leaves 20 warps ran 6.69 ms, 24 (80 registers, spills) 7.13, 32 (64 registers)
-// 7.94.  The code is long and straight, so warps that start together share its
-// instruction fetches: at the same 20 warps CTAs of 128 threads ran 7.83 ms
-// (barriers between the stages gained nothing more).  Small launches use 64
-// threads so that they reach every SM.
-constexpr int FOLD_THREADS = 320;
+// k_fold's CTA: 80 registers a thread, 24 warps per SM, with the values read
+// seldom on a shelf in shared memory (120 B a thread).  On the benchmark's leaves
+// 20 warps (96 registers) without the shelf ran 6.49 ms and with it 6.40, 24 warps
+// with it 6.07, 32 warps (64 registers, spills) 6.47; without the shelf 24 and 32
+// warps had lost to 20.  The code is long and straight, so warps that start
+// together share its instruction fetches: at the same 24 warps CTAs of 256
+// threads ran 9 % slower (barriers between the stages gained nothing more).
+// Warps of a CTA in multiples of four, one for each scheduler: 22 warps in CTAs
+// of 11 ran 6.73 ms.  Small launches use 64 threads so that they reach every SM.
+constexpr int FOLD_THREADS = 384;
 constexpr int FOLD_SMALL_THREADS = 64;
-constexpr int FOLD_THREADS_PER_SM = 640;
-constexpr int FOLD_STAGE = 12;  // staged moves per thread of a warp
+constexpr int FOLD_THREADS_PER_SM = 768;
+// Staged moves per thread of a warp: with the shelf a CTA's 64.6 KB fill the 132 KB
+// shared-memory split twice.  9 lose 5 to 17 % on playouts (the queue's atomics),
+// 16 take 32 KB from the L1 cache and lose 1.5 % on the benchmark's leaves.
+constexpr int FOLD_STAGE = 12;
+constexpr int FOLD_SHELF_BYTES = SHELF_SLOTS * 8;  // dynamic shared memory per thread
 
 enum : u32 { DEVERR_QUEUE = 8u };  // a queue was too short for its chunk: the leaf runs again in smaller chunks
 
@@ -120,6 +127,7 @@ __global__ void __launch_bounds__(T, FOLD_THREADS_PER_SM / T)
     constexpr int W = T / 32;
     __shared__ u32 s_stage[W][FOLD_STAGE * 32];
     __shared__ u32 s_used[W][2];
+    extern __shared__ u64 s_shelf[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     u64 n = e.n, nparents = e.nparents;
     if (e.n_dev) {
@@ -142,7 +150,7 @@ __global__ void __launch_bounds__(T, FOLD_THREADS_PER_SM / T)
         u32 st = e.states[p];
         make_move<C>(b, st, e.moves[i]);
         StagedSink sink{s_stage[warp], s_used[warp], (u32)lane << 16, i, queue};
-        total = fold_child<1 - C, STRICT>(b, st, sink, &simple);
+        total = fold_child<1 - C, STRICT>(b, st, sink, &simple, Shelf{s_shelf + threadIdx.x, T});
     }
     __syncwarp();
     const u32 used = min(s_used[warp][0], s_used[warp][1]);

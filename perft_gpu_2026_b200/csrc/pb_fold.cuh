@@ -13,17 +13,19 @@
 // a piece p is SIMPLE when it leaves Y's castling, pins and checks alone and
 // what it does to the king's moves is plain:
 //   - p attacks no core square from f or from t; X-rays through Y's first
-//     blocker towards the king count as attacks (a slider there would pin).
-//     Pawns attack no ring square either;
+//     blocker towards the king count as attacks (a slider there would pin);
 //   - f is not an X piece that shields a core or ring square from an X slider,
 //     nor one of two blockers with a Y piece between an X slider and the king;
 //   - t is not on a line from an X slider to a core or ring square it attacks,
 //     nor between a pinned Y piece's pinner and the king;
 //   - neither f nor t is on such a castling path;
 //   - a piece captured on t is not next to the king, pinned, on a castling
-//     corner or a pawn about to promote, is not a slider that sees f along
-//     the line of the capture, and is not a pawn that bears on f (unless a
-//     pawn takes it, where the overlap is one known move).
+//     corner or a pawn about to promote, is not a pawn that bears on f (unless
+//     a pawn takes it, where the overlap is one known move), and is not a
+//     slider that the king takes;
+//   - no en-passant capture of it is in question: each of Y's pawns beside a
+//     double push has one, unless one of them is pinned or the king shares
+//     their rank.
 // After a simple move
 //   - Y's pinned-piece and castling moves are as before; its king moves too,
 //     unless p attacks ring squares from f or t: those moves are counted again
@@ -34,16 +36,17 @@
 //     t), less one if X slides between the two squares in front of an unmoved
 //     pawn;
 //   - a Y slider that sees t loses the squares beyond t, and one that sees f
-//     gains those beyond f; moves of f along that same line are corrected one
-//     by one.
+//     gains those beyond f; moves of f along that same line, the slider's own
+//     capture included, are corrected one by one.
 // Weights of t are summed over all simple moves at once: the number of simple
 // moves onto each square is kept in bit-sliced planes (at most 16 pieces can
 // reach one square: eight lines and eight knight jumps).
 //
-// Promotions, en passant, castling and double pushes that allow an en-passant
-// capture go to the sink.  On the benchmark's leaves 4.2 % of the moves do, on
-// middle-game playouts 14 %, late in a game 21 %; without the recounted king
-// moves it was 7.5 %, 21 % and 37 %.
+// Promotions, en passant and castling go to the sink.  On the benchmark's leaves
+// 2.5 % of the moves do, on middle-game playouts 11 %, late in a game 17 %; with
+// pawns next to the ring, captured sliders and double pushes beside a pawn it was
+// 4.2 %, 14 % and 21 %, without the recounted king moves 7.5 %, 21 % and 37 %.
+// What is left is mostly checks and pins made or lifted.
 #pragma once
 #include "pb_core.cuh"
 
@@ -62,7 +65,7 @@ enum ShelfSlot {
     SHELF_MOVED0,
     SHELF_MOVED1,
     SHELF_MOVED2,
-    SHELF_FLAGGED,
+    SHELF_NO_EP,
     SHELF_OK_TO,
     SHELF_RING_B,
     SHELF_RING_R,
@@ -322,22 +325,25 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple, Shelf shel
     // moved0..2: the number of simple moves of each pawn, bit-sliced.
     u64 moved0 = 0, moved1 = 0, moved2 = 0;
     const u64 pawns = s.pawns & mine;
-    const u64 flagged = east1(s.pawns & them) | west1(s.pawns & them);  // a double push here allows en passant
-    const u64 reach_p = cap_west<Y>(ring | core) | cap_east<Y>(ring | core);
+    // a double push onto `flagged` allows en passant: one move for each pawn
+    // beside it, unless one is pinned or the king is on their rank
+    const u64 yp = s.pawns & them, flagged = east1(yp) | west1(yp);
+    const u64 no_ep = ykb & push1<X>(DP_X) ? flagged : east1(yp & pinned_y) | west1(yp & pinned_y);
+    const u64 reach_p = cap_west<Y>(core) | cap_east<Y>(core);
     const u64 ok_to = ~(reach_p | stay | PROMO_RANKS);
-    shelf.set(SHELF_FLAGGED, flagged);
+    shelf.set(SHELF_NO_EP, no_ep);
     shelf.set(SHELF_OK_TO, ok_to);
     {
         // pinned pawns push along their king's file and capture along its
         // diagonals; all their moves go to the sink
         const u64 free_p = pawns & ~pinned_x, held = pawns & pinned_x, diag = bishop_empty(xk);
-        const u64 ok = free_p & ~(reach_p | keep), ok_cap = them & ~bY & ok_to;
+        const u64 ok = free_p & ~(reach_p | keep), ok_cap = them & ok_to;
         const u64 d1 = push1<X>(free_p | (held & (FILEA << (xk & 7)))) & empty, d2 = push1<X>(d1 & DP_X) & empty & safe;
         const u64 target = them & safe;
         const u64 xw = (cap_west<X>(free_p) | (cap_west<X>(held & diag) & diag)) & target;
         const u64 xe = (cap_east<X>(free_p) | (cap_east<X>(held & diag) & diag)) & target;
         const u64 s1 = d1 & safe & ok_to & push1<X>(ok);
-        const u64 s2 = d2 & ~flagged & ok_to & push1<X>(push1<X>(ok));
+        const u64 s2 = d2 & ~no_ep & ok_to & push1<X>(push1<X>(ok));
         const u64 sw = cap_west<X>(ok) & xw & ok_cap;
         const u64 se = cap_east<X>(ok) & xe & ok_cap;
         to.add(s1);
@@ -348,6 +354,26 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple, Shelf shel
         // capture of a pawn that attacks f: its lost capture of f is in both
         // its own loss and f's weight
         if ((sw | se) & fp) corr = popc(sw & fp) + popc(se & fp);
+        if (s2 & flagged) corr += popc(s2 & east1(yp)) + popc(s2 & west1(yp));
+        // ring squares attacked from f or t: Y's king moves are counted again
+        const u64 reach_r = cap_west<Y>(ring) | cap_east<Y>(ring);
+        if ((ok | s1 | s2 | sw | se) & reach_r) {
+            u64 n1 = s1 & (reach_r | push1<X>(reach_r)), n2 = s2 & (reach_r | push1<X>(push1<X>(reach_r)));
+            u64 nw = sw & (reach_r | cap_west<X>(reach_r)), ne = se & (reach_r | cap_east<X>(reach_r));
+            while (n1 | n2 | nw | ne) {
+                u64 tb, fb;
+                if (n1)
+                    tb = n1 & (0 - n1), n1 ^= tb, fb = push1<Y>(tb);
+                else if (n2)
+                    tb = n2 & (0 - n2), n2 ^= tb, fb = push1<Y>(push1<Y>(tb));
+                else if (nw)
+                    tb = nw & (0 - nw), nw ^= tb, fb = cap_east<Y>(tb);
+                else
+                    tb = ne & (0 - ne), ne ^= tb, fb = cap_west<Y>(tb);
+                const u64 left = (cap_west<X>(fb) | cap_east<X>(fb)) & ~multi;
+                corr += popc(ring & ~((threat & ~left) | cap_west<X>(tb) | cap_east<X>(tb))) - kings;
+            }
+        }
         const u64 f1 = push1<Y>(s1), f2 = push1<Y>(push1<Y>(s2)), fw = cap_east<Y>(sw), fe = cap_west<Y>(se);
         const u64 x = f1 ^ f2 ^ fw, c = (f1 & f2) | (fw & (f1 ^ f2)), c2 = x & fe;
         moved0 = x ^ fe;
@@ -485,7 +511,6 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple, Shelf shel
         const u64 fb = sl & (0 - sl);
         const bool diag = (fb & bqX) != 0;
         u64 a = magic_lookup((diag ? PB_TAB.bishop : PB_TAB.rook) + f, occ), core_f = 0, ring_f = 0;
-        u64 seen = a & (diag ? bY : rY);
         if (diag) {
             core_f = shelf.get(SHELF_CORE_B);
             ring_f = shelf.get(SHELF_RING_B);
@@ -495,14 +520,13 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple, Shelf shel
             ring_f |= shelf.get(SHELF_RING_R);
             if (diag) {
                 const u64 c = rook_att(f, occ);
-                seen |= c & rY;
                 a |= c;
             }
         }
         u64 t = a & safe & ~us;
         if (fb & pinned_x) t &= line_through(f, xk);
         if (!t) continue;
-        const u64 no = stay | core_f | seen | (fp & (king_att(f) | push1<X>(push1<X>(fb))));
+        const u64 no = stay | core_f | (fp & (king_att(f) | push1<X>(push1<X>(fb))));
         const u64 sm = ((fb & (keep | core_f)) || popc(pieces & (fb - 1)) >= 12) ? 0 : t & ~no;
         u64 near = sm & ring_f, left = 0;
         if (fb & ring_f) {
@@ -614,27 +638,27 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple, Shelf shel
                 const u64 past = opened & beyond(sq, f);
                 const int ext = popc(past & ~them);
                 corr += ext * n;
-                // moves of f along the same line
+                // moves of f along the same line, up to the capture of the slider
                 if (!(fb & (s.pawns | alike))) continue;
                 u64 line = 0;
                 if (fb & s.pawns) {
                     if (diag) {
-                        line = (cap_west<X>(fb) | cap_east<X>(fb)) & past & them & ~bY;
+                        line = (cap_west<X>(fb) | cap_east<X>(fb)) & (past | bit) & them;
                     } else if (((sq ^ f) & 7) == 0) {
                         const u64 d = push1<X>(fb) & empty;
-                        line = d | (push1<X>(d & DP_X) & empty & ~shelf.get(SHELF_FLAGGED));
+                        line = d | (push1<X>(d & DP_X) & empty & ~shelf.get(SHELF_NO_EP));
                     }
                     line &= safe & shelf.get(SHELF_OK_TO);
                 } else {
-                    u64 no = stay | us | (past & y_alike) | (fp & (king_att(f) | push1<X>(push1<X>(fb))));
+                    u64 no = stay | us | (fp & (king_att(f) | push1<X>(push1<X>(fb))));
                     if (fb & bqX) no |= shelf.get(SHELF_CORE_B);
                     if (fb & rqX) no |= shelf.get(SHELF_CORE_R);
-                    line = (between(sq, f) | past) & safe & ~no;
+                    line = (between(sq, f) | past | bit) & safe & ~no;
                     if (fb & pinned_x) line &= line_through(f, xk);
                 }
                 if (line) {
                     corr -= ext * popc(line & ~past);
-                    corr += popc(line & them);
+                    corr += popc(line & past & them);
                     for (u64 t = line & past & empty; t; t &= t - 1) corr -= popc(past & beyond(sq, lsb(t)) & ~them);
                 }
             }

@@ -5,8 +5,8 @@
 // simple moves (fold_child) and appends its other moves to a queue in device
 // memory; k_fold_count makes the queued moves and counts each of them in full,
 // one per thread.  Both are bound by integer issue.  The queue between them
-// costs 16 B of traffic per queued move (one per child on the benchmark's
-// leaves, five on middle-game playouts) and buys full warps in both halves, no
+// costs 16 B of traffic per queued move (0.7 per child on the benchmark's
+// leaves, 3.6 on middle-game playouts) and buys full warps in both halves, no
 // barriers, and 55 + 20 KB of code instead of one kernel whose warps fetch from
 // both at once (one kernel with a shared-memory queue and a barrier between the
 // halves: 10.9 ms against 8.15 ms for the first form of these two on the
@@ -14,8 +14,8 @@
 //
 // Measured on B200 against the leaf that makes and counts every move
 // (balanced, listed pieces; the benchmark's 27.2 M edges, 774 M moves):
-// 20.09 -> 7.20 ms (k_fold 6.05, k_fold_count 1.14); 5.2 M edges of 6-40 ply
-// playouts 5.33 -> 2.27 ms; 4.2 M edges of 60-140 ply playouts 4.26 -> 2.05 ms.
+// 20.09 -> 6.78 ms (k_fold 6.09, k_fold_count 0.69); 5.2 M edges of 6-40 ply
+// playouts 5.33 -> 2.10 ms; 4.2 M edges of 60-140 ply playouts 4.26 -> 1.90 ms.
 #pragma once
 #include "pb_fold.cuh"
 #include "pb_kernels.cuh"

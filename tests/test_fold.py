@@ -50,6 +50,28 @@ def test_fold_equals_counting_on_constructed_positions(fen):
     assert bad == 0 and checked > 0
 
 
+@pytest.mark.parametrize("fen", [
+    # double pushes beside pawns: free, pinned on a file and a diagonal, the king
+    # and a rook on their rank, two capturers
+    "4k3/8/8/8/2p1p3/8/3P4/4K3 w - - 0 1",
+    "4k3/8/8/8/4p3/8/3P4/4RK2 w - - 0 1",
+    "8/8/6k1/8/4p3/8/2BP4/6K1 w - - 0 1",
+    "8/8/8/8/k1p4R/8/1P1P4/4K3 w - - 0 1",
+    "5k2/R3p3/8/1p1P1P1q/2P1P1P1/8/1P1P1P1P/4K3 w - - 0 1",
+    # sliders that take and are taken along their own lines, with more behind
+    "3r3k/3q4/3r4/8/3R4/3Q4/3R4/K7 w - - 0 1",
+    "k6b/6q1/5b2/8/3B4/2Q5/1B6/K7 w - - 0 1",
+    "7k/8/2b1q3/3P4/2r1b3/1P3P2/8/K7 w - - 0 1",
+    "1k6/8/1q1q1q2/2Q1Q3/1b1R1b2/2Q1Q3/1r3r2/K7 w - - 0 1",
+    # pawns beside the squares next to the king
+    "8/8/3k4/8/1PPPPP2/8/PPP1PPP1/K7 w - - 0 1",
+    "8/2p1p3/8/2PkP3/P1p1p1P1/2P1P3/1P1P1P2/K7 w - - 0 1",
+])
+def test_fold_pawns_beside_and_captured_sliders(fen):
+    checked, made, bad = pg.selftest_fold(_walk(fen, 2000, 8, seed=11))
+    assert bad == 0 and checked > 0
+
+
 def test_fold_equals_counting_on_playouts():
     checked, made, bad = pg.selftest_fold(pg.random_playouts(99, 60000, 0, 160, packed=True))
     assert bad == 0

@@ -9,10 +9,11 @@ that produced them.
 
 leaf    the bench position (4 random plies from the initial array, splitmix64
         seed 1) at perft --depth without tables, --reps times: each pass is
-        one two-ply leaf launch over the position's perft(depth-2) edges, so
-        `-k regex:k_leaf2 -s <reps-1> -c 1` captures the last pass's leaf
-        launch, the same launch the benchmark times.  Prints the count, the
-        CUDA-event leaf time and the move-count calls of that launch.
+        one two-ply leaf over the position's perft(depth-2) edges: with the
+        default kernel 6 pairs of k_fold and k_fold_count (`-k regex:k_fold`),
+        one pair per chunk of edges; with the others one launch, the last
+        pass's by `-k regex:k_leaf2 -s <reps-1> -c 1`.  Prints the count, the
+        CUDA-event leaf time and the counted moves of that leaf.
 levels  one batched perft over --roots playout positions (0..60 plies, seed
         3): large BFS levels for the HBM-bound level kernels (make+count,
         scan, staged generation).

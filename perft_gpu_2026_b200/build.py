@@ -62,7 +62,7 @@ def build_cli(force: bool = False) -> str:
 
 
 def build_oracle(reference_dir: str | None = None) -> None:
-    """The checker: oracle/liboracle.so, and oracle/_ref/perft_gpu_ref when a
+    """The oracle: oracle/liboracle.so, and oracle/_ref/perft_gpu_ref when a
     directory holding the reference sources is given (argument, else the
     PERFT_REFERENCE_DIR environment variable)."""
     subprocess.run(["make", "-s", "-C", os.path.join(ROOT, "oracle")], check=True)

@@ -67,24 +67,31 @@ struct __align__(32) Magic {
 
 // Attack and geometry tables.  One copy lives in device global memory
 // (g_tab, read with the non-coherent path) and one on the host (h_tab).
+//
+// Index 64 is the square of a king that is not on the board (bit_index of an
+// empty set): it attacks nothing, nothing bears on it and nothing lies between
+// it and a square.  A king can be captured in positions that parse_fen accepts:
+// an en-passant capture that uncovers a slider behind the captured pawn is
+// generated, as in the reference.  The side without a king then has no moves.
 struct Tables {
-    Magic rook[64];
-    Magic bishop[64];
-    u64 knight[64];
-    u64 king[64];
-    u64 rook_empty[64];
-    u64 bishop_empty[64];
-    u64 between[64][64];
+    Magic rook[65];
+    Magic bishop[65];
+    u64 knight[65];
+    u64 king[65];
+    u64 rook_empty[65];
+    u64 bishop_empty[65];
+    u64 between[66][64];  // rows 64 and 65 (the end of [64][64]) are empty
     u64 line[64][64];
     u64 beyond[64][64];  // [s][t]: the squares past t on the ray from s through t
     // Squares from which a rook / bishop on an empty board attacks the zone
     // of a king on that square: its 3x3 block and, for e1/e8, the castling
     // squares c..g of its back rank.
-    u64 rook_reach[64];
-    u64 bishop_reach[64];
-    u64 knight_reach[64];  // squares from which a knight attacks that zone
+    u64 rook_reach[65];
+    u64 bishop_reach[65];
+    u64 knight_reach[65];  // squares from which a knight attacks that zone
 };
-constexpr int ATTACK_TABLE_SIZE = 107648;  // sum over squares of 2^bits (rook 102400 + bishop 5248)
+constexpr int ATTACK_SLICES = 107648;                // sum over squares of 2^bits (rook 102400 + bishop 5248)
+constexpr int ATTACK_TABLE_SIZE = ATTACK_SLICES + 1;  // and the empty set, for square 64
 
 extern Tables h_tab;
 extern u64 h_attacks[ATTACK_TABLE_SIZE];
@@ -102,7 +109,7 @@ PB_HD int popc(u64 x)
     return __builtin_popcountll(x);
 #endif
 }
-// Index of the lowest set bit (x != 0).  On the GPU this is a population
+// Index of the lowest set bit, 64 if there is none.  On the GPU this is a population
 // count of the bits below it: POPC issues on the XU pipe, which leaves the
 // ALU pipe (the leaf kernel's bottleneck) free.
 PB_HD int lsb(u64 x)
@@ -110,16 +117,16 @@ PB_HD int lsb(u64 x)
 #ifdef __CUDA_ARCH__
     return __popcll((x - 1) & ~x);
 #else
-    return __builtin_ctzll(x);
+    return x ? __builtin_ctzll(x) : 64;
 #endif
 }
-// Index of a single set bit.
+// Index of a single set bit, 64 if there is none.
 PB_HD int bit_index(u64 single)
 {
 #ifdef __CUDA_ARCH__
     return __popcll(single - 1);
 #else
-    return __builtin_ctzll(single);
+    return single ? __builtin_ctzll(single) : 64;
 #endif
 }
 PB_HD bool more_than_one(u64 x) { return (x & (x - 1)) != 0; }
@@ -165,7 +172,7 @@ PB_HD u64 rook_att(int sq, u64 occ) { return magic_lookup(&PB_TAB.rook[sq], occ)
 PB_HD u64 bishop_att(int sq, u64 occ) { return magic_lookup(&PB_TAB.bishop[sq], occ); }
 PB_HD u64 knight_att(int sq) { return ldg64(&PB_TAB.knight[sq]); }
 PB_HD u64 king_att(int sq) { return ldg64(&PB_TAB.king[sq]); }
-PB_HD u64 between(int a, int b) { return ldg64(&PB_TAB.between[a][b]); }
+PB_HD u64 between(int a, int b) { return ldg64(&PB_TAB.between[0][0] + a * 64 + b); }
 PB_HD u64 line_through(int a, int b) { return ldg64(&PB_TAB.line[a][b]); }
 PB_HD u64 rook_empty(int sq) { return ldg64(&PB_TAB.rook_empty[sq]); }
 PB_HD u64 bishop_empty(int sq) { return ldg64(&PB_TAB.bishop_empty[sq]); }
@@ -369,7 +376,7 @@ struct ListedView {
 template <int C, bool STRICT>
 PB_HD u32 count_evasions(const Sets &s, u32 state, u64 pinned, u64 threat, int ksq)
 {
-    u64 king = 1ULL << ksq;
+    u64 king = s.kings & s.us;
     u64 checkers = (cap_west<C>(king) | cap_east<C>(king)) & s.pawns & s.them;
     checkers |= knight_att(ksq) & s.knights & s.them;
     checkers |= bishop_att(ksq, s.occ) & s.bq & s.them;
@@ -495,20 +502,23 @@ PB_HD u32 count_quiet(const Sets &s, u32 state, u64 pinned, u64 threat, int ksq,
 // and the enemy attack map (findPinnedPieces + findAttackedSquares).
 struct CountPrep {
     Sets s;
-    u64 pinned, threat;
+    u64 king, pinned, threat;
     int ksq;
 };
 template <int C> PB_HD CountPrep count_prep(const Board &b)
 {
     CountPrep p;
     p.s = derive<C>(b);
-    u64 my_king = p.s.kings & p.s.us;
-    p.ksq = bit_index(my_king);
+    p.king = p.s.kings & p.s.us;
+    p.ksq = bit_index(p.king);
     p.pinned = pinned_set(p.ksq, p.s.bq & p.s.them, p.s.rq & p.s.them, p.s.occ);
-    p.threat = enemy_attacks<C>(p.s, my_king, p.ksq);
+    p.threat = enemy_attacks<C>(p.s, p.king, p.ksq);
     return p;
 }
-template <int C> PB_HD bool prep_in_check(const CountPrep &p) { return (p.threat >> p.ksq) & 1; }
+// In check; a side without a king counts as in a check that no move answers
+// (no checkers, and `safe` is empty).
+PB_HD bool king_in_check(u64 king, u64 threat) { return (king & ~threat) == 0; }
+template <int C> PB_HD bool prep_in_check(const CountPrep &p) { return king_in_check(p.king, p.threat); }
 
 // Number of legal moves (countMoves, MoveGeneratorBitboard.h:1700-1943, and
 // countMovesOutOfCheck, :1564-1694, for a side in check).
@@ -529,8 +539,8 @@ PB_HD u32 count_moves(const Board &b, u32 state, const Own &own = Own())
     const CountPrep p = count_prep<C>(b);
     const Sets &s = p.s;
     const int ksq = p.ksq;
-    const u64 king = 1ULL << ksq;
-    const bool check = (p.threat & king) != 0;
+    const u64 king = p.king;
+    const bool check = prep_in_check<C>(p);
 #ifdef __CUDA_ARCH__
     // no lane of the converged group in check: the leaner not-in-check path
     if (!__any_sync(__activemask(), check)) return count_quiet<C, STRICT>(s, state, p.pinned, p.threat, ksq, own);
@@ -649,7 +659,7 @@ template <class Sink> PB_HD void emit_pawn(Sink &sink, int from, int to, int fla
 template <int C, class Sink>
 PB_HD void gen_evasions(const Sets &s, u32 state, u64 pinned, u64 threat, int ksq, Sink &sink)
 {
-    u64 king = 1ULL << ksq;
+    u64 king = s.kings & s.us;
     u64 checkers = (cap_west<C>(king) | cap_east<C>(king)) & s.pawns & s.them;
     checkers |= knight_att(ksq) & s.knights & s.them;
     checkers |= bishop_att(ksq, s.occ) & s.bq & s.them;
@@ -716,7 +726,7 @@ template <int C, class Sink> PB_HD void gen_moves(const Board &b, u32 state, Sin
     u64 eb = s.bq & s.them, er = s.rq & s.them;
     u64 pinned = pinned_set(ksq, eb, er, s.occ);
     u64 threat = enemy_attacks<C>(s, my_king, ksq);
-    if (threat & my_king) {
+    if (king_in_check(my_king, threat)) {
         gen_evasions<C>(s, state, pinned, threat, ksq, sink);
         return;
     }

@@ -263,7 +263,7 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple, Shelf shel
     const u64 pinned_x = pinned_set(xk, s.bq & them, s.rq & them, occ);
     const u64 threat_y = enemy_attacks<X>(s, xkb, xk);
     u64 safe = ~0ULL, checkers = 0, mine = us;
-    if (threat_y & xkb) {
+    if (king_in_check(xkb, threat_y)) {
         checkers = (cap_west<X>(xkb) | cap_east<X>(xkb)) & s.pawns & them;
         checkers |= knight_att(xk) & s.knights & them;
         checkers |= bishop_att(xk, occ) & s.bq & them;
@@ -398,11 +398,11 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple, Shelf shel
         const u64 ept = ep_target<X>(st);
         if (ept) {
             const u64 victim = push1<Y>(ept);
-            if (!checkers || victim == checkers) {
+            if (safe == ~0ULL || victim == checkers) {
                 for (u64 src = (east1(victim) | west1(victim)) & pawns; src; src &= src - 1) {
                     const u64 p = src & (0 - src);
                     bool legal = true;
-                    if (!checkers) {
+                    if (safe == ~0ULL) {
                         if (p & pinned_x)
                             legal = (ept & line_through(lsb(src), xk)) != 0;
                         else
@@ -439,7 +439,7 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple, Shelf shel
         }
     }
 
-    if (!checkers) {
+    if (safe == ~0ULL) {
         const u32 castle_x = X == WHITE ? (st & 3) : ((st >> 2) & 3);
         constexpr int K0 = X == WHITE ? 4 : 60;
         if ((castle_x & 1) && !(KS_X & (occ | threat_y))) sink.one(make_move_code(K0, K0 + 2, MF_KING_CASTLE), false);

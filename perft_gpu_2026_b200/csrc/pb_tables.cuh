@@ -75,7 +75,7 @@ static bool fill_magic(Magic &m, int sq, u64 mul, const int (*dirs)[2], u32 offs
 inline Tables device_tables(const u64 *dev_attacks)
 {
     Tables t = h_tab;
-    for (int sq = 0; sq < 64; sq++) {
+    for (int sq = 0; sq <= 64; sq++) {
         t.rook[sq].base = (u64)(uintptr_t)(dev_attacks + h_tab.rook[sq].base);
         t.bishop[sq].base = (u64)(uintptr_t)(dev_attacks + h_tab.bishop[sq].base);
     }
@@ -168,7 +168,10 @@ inline bool build_host_tables()
         ok = ok && fill_magic(h_tab.bishop[sq], sq, kBishopMagic[sq], kBishopDirs, offset);
         offset += 1u << (64 - h_tab.bishop[sq].shift);
     }
-    ok = ok && offset == (u32)ATTACK_TABLE_SIZE;
+    ok = ok && offset == (u32)ATTACK_SLICES;
+    // square 64: every lookup ends at the table's last entry, the empty set
+    h_attacks[ATTACK_SLICES] = 0;
+    h_tab.rook[64] = h_tab.bishop[64] = Magic{0, 0, ATTACK_SLICES, 31, 63};
     built = true;
     return ok;
 }

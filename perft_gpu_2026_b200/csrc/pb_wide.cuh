@@ -37,7 +37,7 @@ template <int C> PB_HD MovePrep<C> move_prep(const Board &b, u32 st)
     p.ksq = bit_index(king);
     p.pinned = pinned_set(p.ksq, s.bq & s.them, s.rq & s.them, s.occ);
     p.threat = enemy_attacks<C>(s, king, p.ksq);
-    p.check = (p.threat & king) != 0;
+    p.check = king_in_check(king, p.threat);
     p.only_king = false;
     p.safe = ~0ULL;
     u64 checkers = 0;

@@ -42,6 +42,10 @@
 // moves onto each square is kept in bit-sliced planes (at most 16 pieces can
 // reach one square: eight lines and eight knight jumps).
 //
+// All of this counts Y's moves from a position in which Y is not in check.  Y has
+// just moved, so it is not, except after an en-passant capture that uncovered its
+// king (pb_core.cuh, Tables); there no move is simple.
+//
 // Promotions, en passant and castling go to the sink.  On the benchmark's leaves
 // 2.5 % of the moves do, on middle-game playouts 11 %, late in a game 17 %; with
 // pawns next to the ring, captured sliders and double pushes beside a pawn it was
@@ -220,10 +224,12 @@ PB_HD u32 fold_child(const Board &b, u32 st, Sink &sink, u32 *simple, Shelf shel
         multi = two;
     }
     {
-        u64 a = bishop_att(yk, occ);
+        u64 a = bishop_att(yk, occ), checkers_y = (threat & ykb) | (a & bqX);
         core_b = a | bishop_att(yk, occ & ~(a & them));
         a = rook_att(yk, occ);
+        checkers_y |= a & rqX;
         core_r = a | rook_att(yk, occ & ~(a & them));
+        if (checkers_y) lines = ~0ULL;  // Y in check
     }
     for (u64 sn = (bishop_empty(yk) & bqX) | (rook_empty(yk) & rqX); sn; sn &= sn - 1) {
         const u64 bw = between(lsb(sn), yk), bt = bw & occ, rest = bt & (bt - 1);

@@ -82,3 +82,50 @@ def test_side_without_king_has_no_moves():
             found += 1
             assert pg.generate_moves(p) == [] and pg.count_moves(p) == 0 and pg.count_moves(p, strict=True) == 0
     assert found > 20
+
+
+def test_folded_counts_of_a_king_left_in_check():
+    """Folding starts from the position with no check on the side that has just
+    moved; here it is in check."""
+    # perft 2 of the child after f5e6: black to move, the bishop on b8 checks f4
+    p = pg.parse_fen(FENS[0])
+    child = next(q for q in (pg.make_move(p, m) for m in pg.generate_moves(p))
+                 if pg.to_fen(q).startswith("1b6/5k2/4P3/8/5K2"))
+    assert sum(pg.count_moves(pg.make_move(child, m)) for m in pg.generate_moves(child)) == 43
+    checked, made, bad = pg.selftest_fold([child])
+    assert bad == 0 and made == checked
+    # such children, what follows them, and their neighbours
+    positions = []
+    for fen in FENS + drawn(60, seed=5):
+        for q in (pg.make_move(pg.parse_fen(fen), m) for m in pg.generate_moves(pg.parse_fen(fen))):
+            positions.append(q)
+            positions += [pg.make_move(q, m) for m in pg.generate_moves(q)]
+    checked, made, bad = pg.selftest_fold(positions)
+    assert bad == 0 and checked > 100000
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("strict", [False, True])
+def test_every_path_matches_oracle(strict, oracle):
+    """The same positions through the small kernels, the folded leaf (a batch of
+    more than 8,192 leaf edges), the table leaf, the listed leaf and the host."""
+    fens = FENS + drawn(24, seed=6)
+    roots = [pg.parse_fen(f) for f in fens]
+    want = {d: [oracle.perft(f, d, strict) for f in fens] for d in (3, 4)}
+    with pg.Engine(device=0, use_tt=False, strict=strict, arena_bytes=1 << 30) as eng:
+        for leaf in (6, 5):
+            eng.set_tuning(leaf_kernel=leaf)
+            for d in (3, 4):
+                assert [eng.perft_position(p, d) for p in roots] == want[d], (leaf, d)
+                many = roots * 40
+                assert eng.perft_batch(many, d) == want[d] * 40, (leaf, d)
+                assert eng.last_stats().leaf_edges > 8192
+    with pg.Engine(device=0, use_tt=True, strict=strict, arena_bytes=1 << 30, device_tt_mb=1024, host_tt_mb=64) as eng:
+        for d in (3, 4):
+            for _ in range(2):
+                assert [eng.perft_position(p, d) for p in roots] == want[d], d
+    deep = [p for p, w in zip(roots, want[4]) if w < 200000]
+    assert len(deep) > 3
+    with pg.Engine(device=0, use_tt=True, strict=strict, arena_bytes=1 << 30, device_tt_mb=1024, host_tt_mb=64) as eng:
+        for p in deep:  # a king captured above the leaf
+            assert eng.perft_position(p, 5) == oracle.perft(pg.to_fen(p), 5, strict)

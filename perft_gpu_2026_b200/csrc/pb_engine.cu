@@ -1456,20 +1456,15 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
         }
     }
     u64 *d_n0 = g.sizes;  // [0] = roots, [k] = edges of level k
-    std::vector<u64> init(nlev + 4, 0);
-    init[0] = n;
-    PB_CUDA(cudaMemcpy(g.sizes, init.data(), sizeof(u64) * init.size(), cudaMemcpyHostToDevice));
-    {
-        std::vector<u32> iota(n);
-        for (u64 i = 0; i < n; i++) iota[i] = (u32)i;
-        PB_CUDA(cudaMemcpy(g.r0, iota.data(), sizeof(u32) * n, cudaMemcpyHostToDevice));
-    }
     cudaGraph_t graph = nullptr;
     PB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(g.rc, 0, sizeof(unsigned long long) * n, s);
     cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s);
     reset_counters(ctx);
     cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), s);
+    // Everything the kernels read is written by the graph itself or, like b0 and
+    // s0, before each run: other calls use the same arena in between.
+    k_plan_roots<<<grid_for(std::max<u64>(n, nlev + 4), 256), 256, 0, s>>>(g.r0, n, g.sizes, nlev + 4);
     // level 0: root move counts -> E_1
     k_count_positions<WHITE, true><<<grid_for(n, 256), 256, 0, s>>>(g.b0, g.s0, n, cnt0);
     cudaMemsetAsync(status0, 0, sizeof(u64) * tiles0, s);

@@ -905,6 +905,15 @@ __device__ __forceinline__ bool plan_overflowed(const u32 *err)
     return __syncthreads_or((*reinterpret_cast<const volatile u32 *>(err) & DEVERR_OVERFLOW) != 0) != 0;
 }
 
+// Start of a planned batch: every root's index and the number of roots; the
+// levels' sizes are then written by their scans.
+__global__ void __launch_bounds__(256) k_plan_roots(u32 *__restrict__ root, u64 n, u64 *__restrict__ sizes, int nsizes)
+{
+    const u64 i = (u64)blockIdx.x * 256 + threadIdx.x;
+    if (i < n) root[i] = (u32)i;
+    if (i < (u64)nsizes) sizes[i] = i ? 0 : n;
+}
+
 // The same leaf with the level sizes in device memory, for captured graphs:
 // the grid covers the planned capacity and the CTAs past the level's actual
 // size leave at once (a whole CTA at a time, so the ranking's barriers are

@@ -23,7 +23,8 @@ LIB = os.path.join(PKG, "libperftb200.so")
 CLI = os.path.join(PKG, "perft_gpu")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-shared"] + ARCH
+# a dropped [[nodiscard]] error (the launch helpers) does not build
+NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-Werror=unused-result", "-shared"] + ARCH
 
 
 def _nvcc() -> str:

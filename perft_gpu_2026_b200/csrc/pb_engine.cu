@@ -238,11 +238,11 @@ inline unsigned fold_count_grid(const pb_ctx *ctx, u64 m)
 }
 
 // Zeroes the counters and the first chunk's queue cursor (one 64-byte block).
-inline cudaError_t reset_counters(pb_ctx *ctx) { return cudaMemsetAsync(ctx->d_counter, 0, 64, ctx->stream); }
+[[nodiscard]] inline cudaError_t reset_counters(pb_ctx *ctx) { return cudaMemsetAsync(ctx->d_counter, 0, 64, ctx->stream); }
 
 // k_fold over edges [first, first + m) in CTAs of T threads.
 template <int C, bool S, int T, FoldOut OUT>
-cudaError_t launch_fold_kernel(pb_ctx *ctx, const LeafEdges &e, u64 first, u64 m, const FoldQueue &q,
+[[nodiscard]] cudaError_t launch_fold_kernel(pb_ctx *ctx, const LeafEdges &e, u64 first, u64 m, const FoldQueue &q,
                                unsigned long long *rc)
 {
     constexpr int SHELF = T * FOLD_SHELF_BYTES;
@@ -256,7 +256,7 @@ cudaError_t launch_fold_kernel(pb_ctx *ctx, const LeafEdges &e, u64 first, u64 m
 // The folded leaf over e.n edges; `overflow` is the error bit of a queue that
 // was too short.  The caller has reset the counters.
 template <int C, bool S, FoldOut OUT>
-cudaError_t launch_fold_t(pb_ctx *ctx, const LeafEdges &e, const FoldQueue &q, bool careful, unsigned long long *rc,
+[[nodiscard]] cudaError_t launch_fold_t(pb_ctx *ctx, const LeafEdges &e, const FoldQueue &q, bool careful, unsigned long long *rc,
                           u32 overflow)
 {
     cudaStream_t s = ctx->stream;
@@ -275,7 +275,7 @@ cudaError_t launch_fold_t(pb_ctx *ctx, const LeafEdges &e, const FoldQueue &q, b
     return cudaGetLastError();
 }
 template <FoldOut OUT>
-cudaError_t launch_fold(pb_ctx *ctx, int c, bool strict, const LeafEdges &e, const FoldQueue &q, bool careful,
+[[nodiscard]] cudaError_t launch_fold(pb_ctx *ctx, int c, bool strict, const LeafEdges &e, const FoldQueue &q, bool careful,
                         unsigned long long *rc, u32 overflow)
 {
     if (c == WHITE) return strict ? launch_fold_t<WHITE, true, OUT>(ctx, e, q, careful, rc, overflow)
@@ -686,7 +686,7 @@ bool plan_tt_fold(const pb_ctx *ctx, Arena ar, u64 n, TTFold *f)
     return f->q.cap / MAX_MOVES >= f->chunk;
 }
 template <int C, bool S>
-cudaError_t launch_tt_fold_t(pb_ctx *ctx, const TTFold &f, const Board *b, const uint8_t *st, const Hash128 *h,
+[[nodiscard]] cudaError_t launch_tt_fold_t(pb_ctx *ctx, const TTFold &f, const Board *b, const uint8_t *st, const Hash128 *h,
                              const u32 *pi, const uint16_t *mv, u64 n, u64 npar, TTView tv, u32 *out)
 {
     cudaStream_t s = ctx->stream;
@@ -711,7 +711,7 @@ cudaError_t launch_tt_fold_t(pb_ctx *ctx, const TTFold &f, const Board *b, const
     }
     return cudaGetLastError();
 }
-cudaError_t launch_tt_fold(pb_ctx *ctx, int c, bool strict, const TTFold &f, const Board *b, const uint8_t *st,
+[[nodiscard]] cudaError_t launch_tt_fold(pb_ctx *ctx, int c, bool strict, const TTFold &f, const Board *b, const uint8_t *st,
                            const Hash128 *h, const u32 *pi, const uint16_t *mv, u64 n, u64 npar, TTView tv, u32 *out)
 {
     if (c == WHITE) return strict ? launch_tt_fold_t<WHITE, true>(ctx, f, b, st, h, pi, mv, n, npar, tv, out)
@@ -1460,7 +1460,8 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
     PB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(g.rc, 0, sizeof(unsigned long long) * n, s);
     cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s);
-    reset_counters(ctx);
+    // what fails in between is returned after the capture has ended
+    cudaError_t ce = reset_counters(ctx);
     cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), s);
     // Everything the kernels read is written by the graph itself or, like b0 and
     // s0, before each run: other calls use the same arena in between.
@@ -1518,7 +1519,9 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
     } else if (g.mode == 3 && !g.queue && fold_fits(fold_queue(ctx, ar))) {
         // a queue too short counts as an outgrown plan
         const LeafEdges e{pb_, ps, pr, L[nlev].pi, L[nlev].mv, lcap, npar_cap, d_n0 + nlev, npar, nullptr, nullptr, nullptr};
-        launch_fold<FOLD_ROOTED>(ctx, c, g.strict, e, fold_queue(ctx, ar), false, g.rc, DEVERR_OVERFLOW);
+        const cudaError_t fe =
+            launch_fold<FOLD_ROOTED>(ctx, c, g.strict, e, fold_queue(ctx, ar), false, g.rc, DEVERR_OVERFLOW);
+        if (ce == cudaSuccess) ce = fe;
     } else if (c == WHITE) {
         if (g.strict)
             launch_leaf_queue<WHITE, true>(g.mode, g.queue, s, ctx->num_sms, pb_, ps, pr, L[nlev].pi, L[nlev].mv, d_n0 + nlev, lcap, npar,
@@ -1534,8 +1537,13 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
             launch_leaf_queue<BLACK, false>(g.mode, g.queue, s, ctx->num_sms, pb_, ps, pr, L[nlev].pi, L[nlev].mv, d_n0 + nlev, lcap,
                                             npar, npar_cap, cursor, g.rc, ctx->d_counter, ctx->d_err);
     }
-    cudaError_t ce = cudaStreamEndCapture(s, &graph);
-    if (ce != cudaSuccess) return cuda_fail(ctx, ce, "end capture");
+    if (ce == cudaSuccess) ce = cudaGetLastError();
+    const cudaError_t ende = cudaStreamEndCapture(s, &graph);
+    if (ce == cudaSuccess) ce = ende;
+    if (ce != cudaSuccess) {
+        if (graph) cudaGraphDestroy(graph);
+        return cuda_fail(ctx, ce, "graph capture");
+    }
     if (g.exec) cudaGraphExecDestroy(g.exec);
     g.exec = nullptr;
     ce = cudaGraphInstantiate(&g.exec, graph, 0);

@@ -459,8 +459,18 @@ void launch_leaf_wide(pb_ctx *ctx, int c, bool strict, const Board *b, const uin
     }
 }
 
+// A pass that gave up may have left its upload from the staging area, and kernels
+// that read it on the device, in flight: the next pass refills that area.
+int passed(pb_ctx *ctx, int rc, int bfs_status)
+{
+    if (rc == PB_OK && bfs_status == BFS_OK) return PB_OK;
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    if (rc == PB_OK) PB_CUDA(e);
+    return rc;
+}
+
 // One GPU breadth-first perft; status BFS_TOO_BIG when a level would not fit.
-int bfs_perft(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth, u64 *out, int *bfs_status)
+int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth, u64 *out, int *bfs_status)
 {
     NvtxRange nvtx_pass("bfs_perft");
     *bfs_status = BFS_OK;
@@ -635,6 +645,12 @@ int bfs_perft(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth,
         stats.leaf_ms += b2;
     }
     return PB_OK;
+}
+
+int bfs_perft(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth, u64 *out, int *bfs_status)
+{
+    const int rc = bfs_perft_pass(ctx, root, root_st, color, depth, out, bfs_status);
+    return passed(ctx, rc, *bfs_status);
 }
 
 // Device tables for remaining depths 2..max_r (allocated on first use, kept
@@ -1105,7 +1121,7 @@ inline void to_white_to_move(const pb_pos &p, Board &b, uint8_t &st)
 
 // Batched breadth-first perft of n white-to-move roots at one depth;
 // out[i] = perft(depth) of root i.  BFS_TOO_BIG when a level does not fit.
-int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth, u64 *out, int *bfs_status)
+int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth, u64 *out, int *bfs_status)
 {
     NvtxRange nvtx_pass("bfs_batch");
     *bfs_status = BFS_OK;
@@ -1327,6 +1343,12 @@ int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth,
         stats.leaf_ms += b2;
     }
     return PB_OK;
+}
+
+int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth, u64 *out, int *bfs_status)
+{
+    const int rc = bfs_batch_pass(ctx, rb, rs, n, depth, out, bfs_status);
+    return passed(ctx, rc, *bfs_status);
 }
 
 // Batched perft with automatic halving when a level does not fit.

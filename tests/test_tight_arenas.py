@@ -1,0 +1,27 @@
+"""Calls in arenas that hold only part of their levels: passes that give up and
+the smaller passes that follow them."""
+import pytest
+
+import perft_gpu_2026_b200 as pg
+
+pytestmark = pytest.mark.gpu
+
+KIWI = "r3k2r/p1ppqpb1/bn2pnp1/3PN3/1p2P3/2N2Q1p/PPPBBPPP/R3K2R w KQkq - 0 1"
+
+
+@pytest.fixture(scope="module")
+def wanted():
+    roots = [pg.parse_fen(f) for f in (pg.START_FEN, KIWI, "8/2p5/3p4/KP5r/1R3p1k/8/4P1P1/8 w - - 0 1")]
+    batch = pg.random_playouts(17, 300, 0, 60, packed=True)
+    with pg.Engine(device=0, use_tt=False, arena_bytes=2 << 30) as eng:
+        return roots, [eng.perft_position(p, 5) for p in roots], batch, eng.perft_batch(batch, 4)
+
+
+@pytest.mark.parametrize("arena_kb", [8, 16, 64, 256, 512, 1024, 1500, 4096, 20000])
+def test_passes_that_give_up_and_their_successors(arena_kb, wanted):
+    """Each pass that gives up is followed at once by one on other positions."""
+    roots, counts, batch, batch_counts = wanted
+    with pg.Engine(device=0, use_tt=False, arena_bytes=arena_kb << 10) as eng:
+        assert [eng.perft_position(p, 5) for p in roots] == counts
+        if arena_kb >= 64:
+            assert eng.perft_batch(batch, 4) == batch_counts

@@ -86,7 +86,7 @@ struct pb_ctx {
     bool timing = false;
     pb_tuning tuning{6, 0, 1024, 128, 2, 1, 1, 1, 2};
     int num_sms = 0;
-    uint16_t *spill = nullptr;  // cooperative-leaf spill area (device)
+    uint16_t *spill = nullptr;  // cooperative-leaf spill area, behind the arena in its allocation
     size_t spill_blocks = 0;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // call start, leaf start, leaf end, call end
     pb_stats stats{};
@@ -348,8 +348,6 @@ int launch_leaf_t(pb_ctx *ctx, const Board *b, const uint8_t *st, const u32 *pi,
     }
     u64 grid = std::min<u64>(nchunks, (u64)ctx->num_sms * per_sm);
     if (grid > ctx->spill_blocks) return fail(ctx, PB_ERR_NOMEM, "leaf spill area too small");
-    if (!ctx->spill)  // 130 MB that only this leaf uses
-        PB_CUDA(cudaMalloc(&ctx->spill, ctx->spill_blocks * LEAF_T * LEAF_OVF * sizeof(uint16_t)));
     k_leaf2_coop<C, S><<<(unsigned)grid, LEAF_T, 0, s>>>(b, st, pi, mv, n, npar, ctx->spill, ctx->d_counter);
     PB_CUDA(cudaGetLastError());
     return PB_OK;
@@ -2221,13 +2219,19 @@ int pb_create(int device, const pb_opts *opts, pb_ctx **out)
             ctx->spill_blocks = (size_t)ctx->num_sms * 8;
             size_t freeb = 0, totalb = 0;
             cudaMemGetInfo(&freeb, &totalb);
+            const size_t spill = ctx->spill_blocks * LEAF_T * LEAF_OVF * sizeof(uint16_t);
+            freeb -= std::min(freeb, spill);
             size_t want = ctx->opts.arena_bytes;
             if (!want) {
                 // no TT: half of free memory up to 32 GiB; TT mode keeps room for the tables
                 size_t cap = ctx->opts.use_tt ? (16ULL << 30) : (32ULL << 30);
                 want = std::min(freeb / 2, cap);
             }
-            if ((e = cudaMalloc(&ctx->arena, want)) != cudaSuccess) { rc = cuda_fail(ctx, e, "arena"); break; }
+            // the cooperative leaf's 130 MB with it: a later call must not need memory
+            // that other users of the GPU may have taken by then
+            const size_t spill_at = (want + 255) & ~(size_t)255;
+            if ((e = cudaMalloc(&ctx->arena, spill_at + spill)) != cudaSuccess) { rc = cuda_fail(ctx, e, "arena"); break; }
+            ctx->spill = reinterpret_cast<uint16_t *>(ctx->arena + spill_at);
             ctx->arena_bytes = want;
             build_zobrist();
             if ((e = cudaMemcpyToSymbol(g_zob, &h_zob, sizeof(Zobrist))) != cudaSuccess) { rc = cuda_fail(ctx, e, "upload keys"); break; }
@@ -2258,7 +2262,6 @@ void pb_destroy(pb_ctx *ctx)
             if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
         if (ctx->arena) cudaFree(ctx->arena);
         if (ctx->d_counter) cudaFree(ctx->d_counter);
-        if (ctx->spill) cudaFree(ctx->spill);
         if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
         if (ctx->stream) cudaStreamDestroy(ctx->stream);
     }

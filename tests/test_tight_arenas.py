@@ -25,3 +25,19 @@ def test_passes_that_give_up_and_their_successors(arena_kb, wanted):
         assert [eng.perft_position(p, 5) for p in roots] == counts
         if arena_kb >= 64:
             assert eng.perft_batch(batch, 4) == batch_counts
+
+
+def test_leaf_kernels_need_no_memory_after_creation():
+    """The cooperative leaf's spill area is there from the start: a call with it
+    takes no device memory."""
+    import torch
+
+    torch.cuda.set_device(0)
+    p = pg.parse_fen(KIWI)
+    with pg.Engine(device=0, use_tt=False, arena_bytes=256 << 20) as eng:
+        want = eng.perft_position(p, 5)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info(0)[0]
+        eng.set_tuning(leaf_kernel=2)
+        assert eng.perft_position(p, 5) == want
+        assert free - torch.cuda.mem_get_info(0)[0] < 64 << 20

@@ -294,7 +294,9 @@ struct NvtxRange {
     NvtxRange &operator=(const NvtxRange &) = delete;
 };
 
-enum { BFS_OK = 0, BFS_TOO_BIG = 1 };
+// BFS_WHOLE_TOO_BIG: a level did not fit, in a pass whose small levels took whole
+// kernels and with them more room than their moves need.
+enum { BFS_OK = 0, BFS_TOO_BIG = 1, BFS_WHOLE_TOO_BIG = 2 };
 
 template <int C, bool S>
 int launch_leaf_t(pb_ctx *ctx, const Board *b, const uint8_t *st, const u32 *pi, const uint16_t *mv, u64 n, u64 npar)
@@ -457,18 +459,30 @@ void launch_leaf_wide(pb_ctx *ctx, int c, bool strict, const Board *b, const uin
     }
 }
 
+// Runs a breadth-first pass, where its whole-level kernels' lists (256 moves for
+// each position) left too little room once more without them: what fits with
+// lists of exact size is not split.
+//
 // A pass that gave up may have left its upload from the staging area, and kernels
 // that read it on the device, in flight: the next pass refills that area.
-int passed(pb_ctx *ctx, int rc, int bfs_status)
+template <class Pass> int run_passes(pb_ctx *ctx, int *bfs_status, Pass pass)
 {
-    if (rc == PB_OK && bfs_status == BFS_OK) return PB_OK;
-    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
-    if (rc == PB_OK) PB_CUDA(e);
-    return rc;
+    const u32 levels = ctx->stats.levels;
+    for (const bool whole_levels : {true, false}) {
+        const int rc = pass(whole_levels);
+        if (rc == PB_OK && *bfs_status == BFS_OK) return PB_OK;
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        if (rc != PB_OK) return rc;
+        PB_CUDA(e);
+        if (*bfs_status != BFS_WHOLE_TOO_BIG) break;
+        ctx->stats.levels = levels;
+    }
+    return PB_OK;
 }
 
 // One GPU breadth-first perft; status BFS_TOO_BIG when a level would not fit.
-int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth, u64 *out, int *bfs_status)
+int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth, bool whole_levels, u64 *out,
+                   int *bfs_status)
 {
     NvtxRange nvtx_pass("bfs_perft");
     *bfs_status = BFS_OK;
@@ -477,6 +491,11 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
         *out = host_perft(root, root_st, color, depth, strict);
         return PB_OK;
     }
+    int wide_levels = 0;
+    auto too_big = [&] {
+        *bfs_status = wide_levels ? BFS_WHOLE_TOO_BIG : BFS_TOO_BIG;
+        return PB_OK;
+    };
     uint16_t root_moves[MAX_MOVES];
     int n0 = host_gen(root, root_st, color, root_moves);
     if (n0 == 0) {
@@ -490,10 +509,7 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
     uint8_t *ps = ar.take<uint8_t>(1);
     uint16_t *emv = ar.take<uint16_t>(n0);
     u32 *epi = ar.take<u32>(n0);
-    if (!pb_ || !ps || !emv || !epi) {
-        *bfs_status = BFS_TOO_BIG;
-        return PB_OK;
-    }
+    if (!pb_ || !ps || !emv || !epi) return too_big();
     // root, state, moves and parent indices (zero) in one copy, laid out as in
     // the arena; error word, counters and totals cleared in one memset
     {
@@ -518,45 +534,32 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
     int c = color;
     const int fuse = ctx->tuning.leaf_fuse == 1 ? 1 : 2;
     const unsigned long long *n_dev = nullptr;  // the leaf's edges, where the host does not wait for their number
-    int wide_levels = 0;
     for (int rem = depth - 1; rem > fuse; rem--) {
         Board *cb = ar.take<Board>(n);
         uint8_t *cs = ar.take<uint8_t>(n);
-        if (!cb || !cs) {
-            *bfs_status = BFS_TOO_BIG;
-            return PB_OK;
-        }
+        if (!cb || !cs) return too_big();
         uint16_t *nmv = nullptr;
         u32 *npi = nullptr;
         u64 *offs = nullptr;
-        const bool whole = wide_level(ctx, n) && wide_levels < WIDE_LEVELS;
+        const bool whole = whole_levels && wide_level(ctx, n) && wide_levels < WIDE_LEVELS;
         unsigned long long *total = reinterpret_cast<unsigned long long *>(ctx->d_total);
         if (whole) {
             total += 1 + wide_levels++;
             nmv = ar.take<uint16_t>(n * MAX_MOVES);
             npi = ar.take<u32>(n * MAX_MOVES);
-            if (!nmv || !npi) {
-                *bfs_status = BFS_TOO_BIG;
-                return PB_OK;
-            }
+            if (!nmv || !npi) return too_big();
             launch_level_wide(ctx, c, cur_b, cur_s, nullptr, epi, emv, n, n_par, cb, cs, nullptr, nmv, npi, total);
             PB_CUDA(cudaGetLastError());
             if (rem - 1 == fuse && fuse == 2 && n <= WIDE_UNREAD && ctx->tuning.leaf_kernel == 6) n_dev = total;
         } else {
             u32 *cnt = ar.take<u32>(n);
             offs = ar.take<u64>(n);
-            if (!cnt || !offs) {
-                *bfs_status = BFS_TOO_BIG;
-                return PB_OK;
-            }
+            if (!cnt || !offs) return too_big();
             if (c == WHITE)
                 k_expand_count<WHITE><<<grid_for(n, 256), 256, 0, s>>>(cur_b, cur_s, epi, emv, n, n_par, cb, cs, cnt, ctx->d_err);
             else
                 k_expand_count<BLACK><<<grid_for(n, 256), 256, 0, s>>>(cur_b, cur_s, epi, emv, n, n_par, cb, cs, cnt, ctx->d_err);
-            if (!launch_scan(ctx, ar, cnt, n, offs)) {
-                *bfs_status = BFS_TOO_BIG;
-                return PB_OK;
-            }
+            if (!launch_scan(ctx, ar, cnt, n, offs)) return too_big();
             PB_CUDA(cudaGetLastError());
         }
         stats.kernels += 2;
@@ -573,18 +576,12 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
                 *out = 0;
                 return PB_OK;
             }
-            if (next > 0xFFFFFFFFULL) {  // parent indices are u32
-                *bfs_status = BFS_TOO_BIG;
-                return PB_OK;
-            }
+            if (next > 0xFFFFFFFFULL) return too_big();  // parent indices are u32
         }
         if (!whole) {
             nmv = ar.take<uint16_t>(next);
             npi = ar.take<u32>(next);
-            if (!nmv || !npi) {
-                *bfs_status = BFS_TOO_BIG;
-                return PB_OK;
-            }
+            if (!nmv || !npi) return too_big();
             launch_generate(ctx, 1 - c, cb, cs, offs, n, nmv, npi);
             PB_CUDA(cudaGetLastError());
         }
@@ -647,8 +644,9 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
 
 int bfs_perft(pb_ctx *ctx, const Board &root, u32 root_st, int color, int depth, u64 *out, int *bfs_status)
 {
-    const int rc = bfs_perft_pass(ctx, root, root_st, color, depth, out, bfs_status);
-    return passed(ctx, rc, *bfs_status);
+    return run_passes(ctx, bfs_status, [&](bool whole_levels) {
+        return bfs_perft_pass(ctx, root, root_st, color, depth, whole_levels, out, bfs_status);
+    });
 }
 
 // Device tables for remaining depths 2..max_r (allocated on first use, kept
@@ -1119,7 +1117,8 @@ inline void to_white_to_move(const pb_pos &p, Board &b, uint8_t &st)
 
 // Batched breadth-first perft of n white-to-move roots at one depth;
 // out[i] = perft(depth) of root i.  BFS_TOO_BIG when a level does not fit.
-int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth, u64 *out, int *bfs_status)
+int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth, bool whole_levels, u64 *out,
+                   int *bfs_status)
 {
     NvtxRange nvtx_pass("bfs_batch");
     *bfs_status = BFS_OK;
@@ -1129,6 +1128,11 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         for (u64 i = 0; i < n; i++) out[i] = 1;
         return PB_OK;
     }
+    int wide_levels = 0;
+    auto too_big = [&] {
+        *bfs_status = wide_levels ? BFS_WHOLE_TOO_BIG : BFS_TOO_BIG;
+        return PB_OK;
+    };
     cudaStream_t s = ctx->stream;
     pb_stats &stats = ctx->stats;
     Arena ar{ctx->arena, ctx->arena_bytes};
@@ -1138,10 +1142,7 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
     u32 *cnt0 = ar.take<u32>(n);
     u64 *off0 = ar.take<u64>(n);
     unsigned long long *rc = ar.take<unsigned long long>(n);
-    if (!b0 || !s0 || !r0 || !cnt0 || !off0 || !rc) {
-        *bfs_status = BFS_TOO_BIG;
-        return PB_OK;
-    }
+    if (!b0 || !s0 || !r0 || !cnt0 || !off0 || !rc) return too_big();
     const bool few = n <= WIDE_MAX;  // boards, states and counts fit the pinned staging area
     if (few) {
         const size_t at = (size_t)(reinterpret_cast<char *>(s0) - ctx->arena);
@@ -1176,7 +1177,7 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
     uint16_t *emv = nullptr;
     u32 *epi = nullptr;
     u64 ne = n, n_par = n;
-    int c = WHITE, wide_levels = 0;
+    int c = WHITE;
     std::vector<u32> iota;
     // One level: the children of the current edges (at first the roots as they
     // are) and their moves as the next edges.
@@ -1189,20 +1190,14 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         u64 *offs = off0;
         uint16_t *nmv = nullptr;
         u32 *npi = nullptr;
-        const bool whole = wide_level(ctx, m) && wide_levels < WIDE_LEVELS;
+        const bool whole = whole_levels && wide_level(ctx, m) && wide_levels < WIDE_LEVELS;
         unsigned long long *total = reinterpret_cast<unsigned long long *>(ctx->d_total);
-        if (!cb || !cs || !cr) {
-            *bfs_status = BFS_TOO_BIG;
-            return PB_OK;
-        }
+        if (!cb || !cs || !cr) return too_big();
         if (whole) {
             total += 1 + wide_levels++;
             nmv = ar.take<uint16_t>(m * MAX_MOVES);
             npi = ar.take<u32>(m * MAX_MOVES);
-            if (!nmv || !npi) {
-                *bfs_status = BFS_TOO_BIG;
-                return PB_OK;
-            }
+            if (!nmv || !npi) return too_big();
             launch_level_wide(ctx, c, cur_b, cur_s, cur_r, roots ? nullptr : epi, emv, m, n_par, cb, cs, cr, nmv, npi,
                               total);
         } else {
@@ -1215,20 +1210,14 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
             } else {
                 cnt = ar.take<u32>(m);
                 offs = ar.take<u64>(m);
-                if (!cnt || !offs) {
-                    *bfs_status = BFS_TOO_BIG;
-                    return PB_OK;
-                }
+                if (!cnt || !offs) return too_big();
                 const unsigned g = grid_for(m, 256);
                 if (c == WHITE)
                     k_expand_count_rooted<WHITE><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, m, n_par, cb, cs, cr, cnt, ctx->d_err);
                 else
                     k_expand_count_rooted<BLACK><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, m, n_par, cb, cs, cr, cnt, ctx->d_err);
             }
-            if (!launch_scan(ctx, ar, cnt, m, offs)) {
-                *bfs_status = BFS_TOO_BIG;
-                return PB_OK;
-            }
+            if (!launch_scan(ctx, ar, cnt, m, offs)) return too_big();
         }
         PB_CUDA(cudaGetLastError());
         PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, SCRATCH_BYTES, cudaMemcpyDeviceToHost, s));
@@ -1244,17 +1233,11 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         cur_r = cr;
         n_par = m;
         if (!roots) c = 1 - c;
-        if (next > 0xFFFFFFFFULL) {
-            *bfs_status = BFS_TOO_BIG;
-            return PB_OK;
-        }
+        if (next > 0xFFFFFFFFULL) return too_big();
         if (!whole) {
             nmv = ar.take<uint16_t>(next ? next : 1);
             npi = ar.take<u32>(next ? next : 1);
-            if (!nmv || !npi) {
-                *bfs_status = BFS_TOO_BIG;
-                return PB_OK;
-            }
+            if (!nmv || !npi) return too_big();
             if (next) launch_generate(ctx, c, cb, cs, offs, m, nmv, npi);
             PB_CUDA(cudaGetLastError());
         }
@@ -1345,8 +1328,9 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
 
 int bfs_batch(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int depth, u64 *out, int *bfs_status)
 {
-    const int rc = bfs_batch_pass(ctx, rb, rs, n, depth, out, bfs_status);
-    return passed(ctx, rc, *bfs_status);
+    return run_passes(ctx, bfs_status, [&](bool whole_levels) {
+        return bfs_batch_pass(ctx, rb, rs, n, depth, whole_levels, out, bfs_status);
+    });
 }
 
 // Batched perft with automatic halving when a level does not fit.

@@ -41,3 +41,28 @@ def test_leaf_kernels_need_no_memory_after_creation():
         eng.set_tuning(leaf_kernel=2)
         assert eng.perft_position(p, 5) == want
         assert free - torch.cuda.mem_get_info(0)[0] < 64 << 20
+
+
+def exact_bytes(edges, positions):
+    """Arena bytes of a call whose levels have `edges` edges and materialise
+    `positions` positions, every array of the size it needs (multiples of 256)."""
+    up = lambda b: (b + 255) // 256 * 256
+    total = 2 * 256 + up(2 * edges[0]) + up(4 * edges[0])
+    for n, nxt in zip(positions, edges[1:]):
+        total += sum(up(n * k) for k in (32, 1, 4, 8)) + up(8 * ((n + 4095) // 4096 + 1)) + up(2 * nxt) + up(4 * nxt)
+    return total
+
+
+def test_an_arena_of_exact_size_is_enough():
+    """The whole-level kernels' wider lists do not make a call split that fits
+    without them (perft 7: levels of 20, 400, 8,902, 197,281 and 4,865,609 edges)."""
+    edges = [20, 400, 8902, 197281, 4865609]
+    p = pg.parse_fen(pg.START_FEN)
+    with pg.Engine(device=0, use_tt=False, arena_bytes=exact_bytes(edges, edges[:-1]) + 8192) as eng:
+        assert eng.perft_position(p, 7) == 3195901860
+        st = eng.last_stats()
+        assert st.levels == 4 and list(st.level_sizes[:5]) == edges
+        assert eng.perft_batch([p], 7) == [3195901860]
+    with pg.Engine(device=0, use_tt=False, arena_bytes=exact_bytes(edges, edges[:-1]) - 65536) as eng:
+        assert eng.perft_position(p, 7) == 3195901860
+        assert eng.last_stats().levels > 4  # a little less, and it is split

@@ -162,7 +162,7 @@ u64 host_perft(const Board &b, u32 st, int c, int depth, bool strict)
 {
     if (depth <= 0) return 1;
     if (depth == 1) return host_count(b, st, c, strict);
-    uint16_t mv[MAX_MOVES];
+    uint16_t mv[HOST_MOVES];
     int n = host_gen(b, st, c, mv);
     u64 total = 0;
     for (int i = 0; i < n; i++) {
@@ -496,7 +496,7 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
         *bfs_status = wide_levels ? BFS_WHOLE_TOO_BIG : BFS_TOO_BIG;
         return PB_OK;
     };
-    uint16_t root_moves[MAX_MOVES];
+    uint16_t root_moves[HOST_MOVES];
     int n0 = host_gen(root, root_st, color, root_moves);
     if (n0 == 0) {
         *out = 0;
@@ -569,7 +569,9 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
             PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, SCRATCH_BYTES, cudaMemcpyDeviceToHost, s));
             PB_CUDA(cudaStreamSynchronize(s));
             stats.d2h_bytes += SCRATCH_BYTES;
-            if ((u32)ctx->h_pinned[SCRATCH_ERR]) return fail(ctx, PB_ERR_DEVICE, "a BFS level reported a device error");
+            const u32 err = (u32)ctx->h_pinned[SCRATCH_ERR];
+            if (err == DEVERR_CAPACITY && wide_levels) return too_big();  // more than MAX_MOVES each
+            if (err) return fail(ctx, PB_ERR_DEVICE, "a BFS level reported a device error");
             next = ctx->h_pinned[total - ctx->d_counter];
             if (stats.levels < 16) stats.level_sizes[stats.levels] = next;
             if (next == 0) {
@@ -622,7 +624,9 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
         if ((u32)ctx->h_pinned[SCRATCH_ERR] != DEVERR_QUEUE || attempt > 0) break;
         PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));  // a queue was too short
     }
-    if ((u32)ctx->h_pinned[SCRATCH_ERR]) return fail(ctx, PB_ERR_DEVICE, "kernel reported a device error");
+    const u32 err = (u32)ctx->h_pinned[SCRATCH_ERR];
+    if (n_dev && err == DEVERR_CAPACITY) return too_big();  // its level was not read
+    if (err) return fail(ctx, PB_ERR_DEVICE, "kernel reported a device error");
     if (n_dev) {
         n = ctx->h_pinned[n_dev - ctx->d_counter];
         if (stats.levels < 16) stats.level_sizes[stats.levels] = n;
@@ -826,7 +830,7 @@ int bfs_tt_roots(pb_ctx *ctx, const Board *rb, const uint8_t *rs, const Hash128 
     u32 *epi = nullptr;
     u64 n = 0;
     if (nroots == 1) {
-        uint16_t root_moves[MAX_MOVES];
+        uint16_t root_moves[HOST_MOVES];
         int n0 = host_gen(rb[0], rs[0], color, root_moves);
         n = (u64)n0;
         emv = ar.take<uint16_t>(n ? n : 1);
@@ -1083,7 +1087,7 @@ int gpu_perft(pb_ctx *ctx, const Board &b, u32 st, int c, int depth, u64 *out)
     if (rc != PB_OK) return rc;
     if (status == BFS_OK) return PB_OK;
     if (depth <= 3) return fail(ctx, PB_ERR_NOMEM, "BFS arena too small for a depth-3 perft");
-    uint16_t mv[MAX_MOVES];
+    uint16_t mv[HOST_MOVES];
     int n = host_gen(b, st, c, mv);
     u64 total = 0;
     for (int i = 0; i < n; i++) {
@@ -1224,7 +1228,9 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         PB_CUDA(cudaStreamSynchronize(s));
         stats.kernels += 2;
         stats.d2h_bytes += SCRATCH_BYTES;
-        if ((u32)ctx->h_pinned[SCRATCH_ERR]) return fail(ctx, PB_ERR_DEVICE, "batched level reported a device error");
+        const u32 err = (u32)ctx->h_pinned[SCRATCH_ERR];
+        if (err == DEVERR_CAPACITY && wide_levels) return too_big();  // more than MAX_MOVES each
+        if (err) return fail(ctx, PB_ERR_DEVICE, "batched level reported a device error");
         const u64 next = ctx->h_pinned[total - ctx->d_counter];
         if (!roots) stats.levels++;
         if (stats.levels < 16) stats.level_sizes[stats.levels] = next;
@@ -1687,7 +1693,7 @@ int plan_and_run(pb_ctx *ctx, const pb_pos *roots, const int *depths, int n, uin
             it.bytes = level_bytes(it.lv, plan_levels(it.depth));
             if (it.depth >= 4 && it.bytes > budget) {
                 // too big for any batch: split into children one ply down
-                uint16_t mv[MAX_MOVES];
+                uint16_t mv[HOST_MOVES];
                 int m = host_gen(it.b, it.s, WHITE, mv);
                 for (int j = 0; j < m; j++) {
                     PlanItem c;
@@ -1791,7 +1797,7 @@ int playout(u64 *st, int plies, pb_pos *out)
     u32 s = out->state;
     int c = WHITE, played = 0;
     for (int i = 0; i < plies; i++) {
-        uint16_t mv[MAX_MOVES];
+        uint16_t mv[HOST_MOVES];
         int n = host_gen(b, s, c, mv);
         if (n <= 0) break;
         std::sort(mv, mv + n, [](uint16_t a, uint16_t z) { return uci_key(a) < uci_key(z); });
@@ -1855,7 +1861,7 @@ int launch_recurse(pb_ctx *ctx, const Board &b, u32 st, int c, int depth, const 
         if (!ctx->gpu) v = host_perft(b, st, c, depth, ctx->opts.strict != 0);
         total.lo = v;
     } else {
-        uint16_t mv[MAX_MOVES];
+        uint16_t mv[HOST_MOVES];
         int n = host_gen(b, st, c, mv);
         for (int i = 0; i < n; i++) {
             Board cb = b;
@@ -1949,7 +1955,7 @@ int launch_breadth_first(pb_ctx *ctx, const Board &root, u32 root_st, int c, int
         std::vector<HostNode> next;
         std::unordered_map<Hash128, u32, KeyHash, KeyEq> index;
         for (const HostNode &nd : level) {
-            uint16_t mv[MAX_MOVES];
+            uint16_t mv[HOST_MOVES];
             int m = host_gen(nd.b, nd.s, col, mv);
             for (int k = 0; k < m; k++) {
                 HostNode ch{nd.b, nd.s, Hash128{0, 0}, nd.paths};
@@ -2041,7 +2047,7 @@ u64 check_listed_t(const Board &y, u32 ys, u64 *checked)
     *checked = 0;
     if (!ListedPieces::build<C>(y, lists, &listed)) return 0;
     const ListedView own{lists, &listed};
-    uint16_t mv[MAX_MOVES];
+    uint16_t mv[HOST_MOVES];
     ArraySink sink{mv, 0};
     gen_moves<Z>(y, ys, sink);
     u64 bad = 0;
@@ -2097,7 +2103,7 @@ u64 check_fold_t(const Board &y, u32 ys, u64 *checked, u64 *made)
 {
     u64 bad = 0;
     for (int strict = 0; strict < 2; strict++) {
-        uint16_t mv[MAX_MOVES];
+        uint16_t mv[HOST_MOVES];
         ArraySink all{mv, 0};
         gen_moves<Z>(y, ys, all);
         CountSink want{y, ys, strict != 0, 0, 0};
@@ -2279,7 +2285,10 @@ int pb_generate_moves(const pb_pos *pos, uint16_t *moves)
 {
     if (!pos || !moves) return PB_ERR_ARG;
     build_host_tables();
-    return host_gen(to_board(*pos), pos->state, pos->color, moves);
+    uint16_t all[HOST_MOVES];
+    const int n = std::min<int>(host_gen(to_board(*pos), pos->state, pos->color, all), MAX_MOVES);
+    memcpy(moves, all, sizeof(uint16_t) * n);
+    return n;
 }
 
 int pb_position_hash(const pb_pos *pos, pb_u128 *out)

@@ -162,7 +162,8 @@ __device__ __forceinline__ int warp_targets(const MovePrep<C> &p, u32 st, u64 (&
 // EDGES, takes n positions as they are), stores them and appends their moves to
 // the next level's edges.  A CTA's positions take their place from *total in
 // one piece, in order; the order of the pieces varies from run to run, and no
-// result depends on it.  `cap` edges have room (n * MAX_MOVES always do).  The
+// result depends on it.  `cap` edges have room, n * MAX_MOVES; positions past that
+// set the error word and the driver takes the kernels with exact sizes.  The
 // next kernels read sibling edges in neighbouring threads, so the larger levels
 // use pieces of W = 16 positions (200 roots at perft 4: the folded leaf ran 78 us
 // on ordered edges, 100 on pieces of one position); the smallest use more CTAs.
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(32 * WIDE_WARPS)
 {
     __shared__ uint16_t s_mv[WIDE_WARPS][MAX_MOVES];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (n_dev) n = (u32)*n_dev;
+    if (n_dev) n = (u32)min(*n_dev, (unsigned long long)n);  // a level that ran out of room lists fewer
     for (u32 i = blockIdx.x * WIDE_WARPS + warp; i < n; i += gridDim.x * WIDE_WARPS) {
         const u32 p = pidx[i];
         if (p >= nparents) continue;
@@ -246,26 +247,31 @@ __global__ void __launch_bounds__(32 * WIDE_WARPS)
         u32 st = pstates[p];
         make_move<C>(b, st, moves[i]);
         int cnt;
-        {
-            const MovePrep<1 - C> prep = move_prep<1 - C>(b, st);
-            u64 t[2];
-            int at;
-            cnt = warp_targets<1 - C>(prep, st, t, &at);
-#pragma unroll
-            for (int h = 0; h < 2; h++)
-                put_moves<1 - C>(prep, lane + 32 * h, t[h], [&](uint16_t m) {
-                    if (at < MAX_MOVES) s_mv[warp][at] = m;
-                    at++;
-                });
-        }
-        __syncwarp();
-        cnt = min(cnt, (int)MAX_MOVES);
         u32 total = 0;
-        for (int k = lane; k < cnt; k += 32) {
-            Board g = b;
-            u32 gs = st;
-            make_move<1 - C>(g, gs, s_mv[warp][k]);
-            total += count_moves<C, STRICT>(g, gs);
+        for (int done = 0;; done += MAX_MOVES) {  // once: hardly a position has more
+            {
+                const MovePrep<1 - C> prep = move_prep<1 - C>(b, st);
+                u64 t[2];
+                int at;
+                cnt = warp_targets<1 - C>(prep, st, t, &at);
+                at -= done;
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    put_moves<1 - C>(prep, lane + 32 * h, t[h], [&](uint16_t m) {
+                        if ((u32)at < MAX_MOVES) s_mv[warp][at] = m;
+                        at++;
+                    });
+            }
+            __syncwarp();
+            const int listed = min(cnt - done, (int)MAX_MOVES);
+            for (int k = lane; k < listed; k += 32) {
+                Board g = b;
+                u32 gs = st;
+                make_move<1 - C>(g, gs, s_mv[warp][k]);
+                total += count_moves<C, STRICT>(g, gs);
+            }
+            if (cnt - done <= MAX_MOVES) break;
+            __syncwarp();
         }
         total = __reduce_add_sync(0xffffffffu, total);
         if (lane == 0 && cnt) {

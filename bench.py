@@ -524,7 +524,7 @@ def main():
     def step():
         total = run_once()
         st = eng.last_stats()
-        return total, st.device_ms, st.leaf_ms, st.leaf_positions, st.kernels, st.h2d_bytes, st.d2h_bytes
+        return total, st.device_ms, st.leaf_ms, st.leaf_positions, st.launches, st.h2d_bytes, st.d2h_bytes
 
     for _ in range(args.warmup):
         step()

@@ -174,12 +174,15 @@ typedef struct {
     uint64_t leaf_edges;       /* edges the leaf kernel took (one perft(2) each) */
     uint64_t leaf_positions;   /* positions the leaf kernel counted (move-count calls) */
     uint64_t nodes;            /* the perft result of the call */
-    uint32_t kernels;          /* kernel launches of the call: three per BFS level and one per leaf,
-                                  however few or many kernels a level or leaf took */
+    uint32_t kernels;          /* steps of the call: three per BFS level and one per leaf, however few or
+                                  many kernels a level or leaf took (`launches` counts those) */
     uint32_t levels;           /* BFS expand levels */
     uint64_t level_sizes[16];  /* edges per level, level 0 = root moves */
     uint64_t h2d_bytes;        /* host-to-device bytes copied */
     uint64_t d2h_bytes;        /* device-to-host bytes copied */
+    uint32_t launches;         /* kernels launched, those of captured graphs included (without the
+                                  planner's network) */
+    uint32_t leaf_reruns;      /* leaves counted again because a queue was too short */
 } pb_stats;
 
 /* Launch parameters of the GPU path (no reference counterpart: the

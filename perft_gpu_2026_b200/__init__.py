@@ -79,6 +79,8 @@ class Stats(ctypes.Structure):
         ("level_sizes", ctypes.c_uint64 * 16),
         ("h2d_bytes", ctypes.c_uint64),
         ("d2h_bytes", ctypes.c_uint64),
+        ("launches", ctypes.c_uint32),
+        ("leaf_reruns", ctypes.c_uint32),
     ]
 
 

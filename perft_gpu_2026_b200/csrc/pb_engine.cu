@@ -46,6 +46,7 @@ struct GraphPlan {
     bool queue = false;  // persistent work-queue leaf instead of the grid leaf
     std::vector<u64> caps;
     cudaGraphExec_t exec = nullptr;
+    u32 launches = 0;  // kernels in it
     // device buffers inside the arena (fixed for the captured graph)
     Board *b0 = nullptr;
     uint8_t *s0 = nullptr;
@@ -271,6 +272,7 @@ template <int C, bool S, FoldOut OUT>
                                             : launch_fold_kernel<C, S, FOLD_THREADS, OUT>(ctx, e, first, m, q, rc);
         if (fe != cudaSuccess) return fe;
         k_fold_count<C, S, OUT><<<fold_count_grid(ctx, m), 256, 0, s>>>(e, q, rc, ctx->d_counter, overflow, ctx->d_err);
+        ctx->stats.launches += 2;
     }
     return cudaGetLastError();
 }
@@ -358,6 +360,7 @@ int launch_leaf_t(pb_ctx *ctx, const Board *b, const uint8_t *st, const u32 *pi,
 int launch_leaf(pb_ctx *ctx, int c, bool strict, const Board *b, const uint8_t *st, const u32 *pi,
                 const uint16_t *mv, u64 n, u64 npar)
 {
+    ctx->stats.launches++;
     if (c == WHITE) return strict ? launch_leaf_t<WHITE, true>(ctx, b, st, pi, mv, n, npar)
                                   : launch_leaf_t<WHITE, false>(ctx, b, st, pi, mv, n, npar);
     return strict ? launch_leaf_t<BLACK, true>(ctx, b, st, pi, mv, n, npar)
@@ -379,6 +382,7 @@ void launch_generate(pb_ctx *ctx, int c, const Board *b, const uint8_t *st, cons
                      u32 *pi)
 {
     cudaStream_t s = ctx->stream;
+    ctx->stats.launches++;
     if (ctx->tuning.gen_threads == 64) {
         if (c == WHITE) k_generate<WHITE, 64><<<grid_for(n, 64), 64, 0, s>>>(b, st, offs, ctx->d_total, n, mv, pi, ctx->d_err);
         else k_generate<BLACK, 64><<<grid_for(n, 64), 64, 0, s>>>(b, st, offs, ctx->d_total, n, mv, pi, ctx->d_err);
@@ -396,6 +400,7 @@ void launch_level_wide(pb_ctx *ctx, int c, const Board *pb_, const uint8_t *ps, 
 {
     cudaStream_t s = ctx->stream;
     const u64 cap = n * MAX_MOVES;
+    ctx->stats.launches++;
 #define PB_LEVEL_W(CC, EE, RR, WW)                                                                                    \
     k_level_wide<CC, EE, RR, WW><<<grid_for(n, WW), 32 * WW, 0, s>>>(pb_, ps, pr, pi, mv, (u32)n, npar, cb, cs, cr, nmv, \
                                                                      npi, cap, total, ctx->d_err)
@@ -428,6 +433,7 @@ bool launch_scan(pb_ctx *ctx, Arena &ar, const u32 *cnt, u64 n, u64 *offs)
     const u64 tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     u64 *status = ar.take<u64>(tiles + 1);  // and the tile ticket
     if (!status) return false;
+    ctx->stats.launches++;
     cudaMemsetAsync(status, 0, sizeof(u64) * (tiles + 1), ctx->stream);
     k_scan<<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(cnt, n, offs, status, reinterpret_cast<u32 *>(status + tiles),
                                                              ctx->d_total, ctx->d_err);
@@ -450,6 +456,7 @@ void launch_leaf_wide_t(pb_ctx *ctx, const Board *b, const uint8_t *st, const u3
 void launch_leaf_wide(pb_ctx *ctx, int c, bool strict, const Board *b, const uint8_t *st, const u32 *r, const u32 *pi,
                       const uint16_t *mv, u64 n, const unsigned long long *n_dev, u64 npar, unsigned long long *rc)
 {
+    ctx->stats.launches++;
     if (c == WHITE) {
         if (strict) launch_leaf_wide_t<WHITE, true>(ctx, b, st, r, pi, mv, n, n_dev, npar, rc);
         else launch_leaf_wide_t<WHITE, false>(ctx, b, st, r, pi, mv, n, n_dev, npar, rc);
@@ -521,9 +528,9 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
         memcpy(stage + (reinterpret_cast<char *>(ps) - ctx->arena), &st8, 1);
         memcpy(stage + (reinterpret_cast<char *>(emv) - ctx->arena), root_moves, sizeof(uint16_t) * n0);
         PB_CUDA(cudaMemcpyAsync(ctx->arena, stage, bytes, cudaMemcpyHostToDevice, s));
+        stats.h2d_bytes += bytes;
     }
     PB_CUDA(cudaMemsetAsync(ctx->d_counter, 0, SCRATCH_BYTES, s));
-    stats.h2d_bytes += sizeof(Board) + 1 + sizeof(uint16_t) * n0;
     if (stats.levels < 16) stats.level_sizes[stats.levels] = (u64)n0;
     if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[0], s));
 
@@ -559,6 +566,7 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
                 k_expand_count<WHITE><<<grid_for(n, 256), 256, 0, s>>>(cur_b, cur_s, epi, emv, n, n_par, cb, cs, cnt, ctx->d_err);
             else
                 k_expand_count<BLACK><<<grid_for(n, 256), 256, 0, s>>>(cur_b, cur_s, epi, emv, n, n_par, cb, cs, cnt, ctx->d_err);
+            stats.launches++;
             if (!launch_scan(ctx, ar, cnt, n, offs)) return too_big();
             PB_CUDA(cudaGetLastError());
         }
@@ -623,6 +631,7 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
         PB_CUDA(cudaStreamSynchronize(s));
         if ((u32)ctx->h_pinned[SCRATCH_ERR] != DEVERR_QUEUE || attempt > 0) break;
         PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));  // a queue was too short
+        stats.leaf_reruns++;
     }
     const u32 err = (u32)ctx->h_pinned[SCRATCH_ERR];
     if (n_dev && err == DEVERR_CAPACITY) return too_big();  // its level was not read
@@ -724,6 +733,7 @@ template <int C, bool S>
         k_fold_count<C, S, FOLD_EACH><<<fold_count_grid(ctx, m), 256, 0, s>>>(e, f.q, nullptr, ctx->d_counter, DEVERR_QUEUE, ctx->d_err);
         k_tt_keep<<<grid_for(m, 256), 256, 0, s>>>(f.ch, first, (u32)m, out, tv);
         if (gen == (1u << (32 - TT_AT_BITS)) - 1) gen = 0;
+        ctx->stats.launches += 5;
     }
     return cudaGetLastError();
 }
@@ -867,6 +877,7 @@ int bfs_tt_roots(pb_ctx *ctx, const Board *rb, const uint8_t *rs, const Hash128 
         PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_total, sizeof(u64), cudaMemcpyDeviceToHost, s));
         PB_CUDA(cudaStreamSynchronize(s));
         stats.kernels += 2;
+        stats.launches += 2;
         stats.d2h_bytes += 8;
         n = ctx->h_pinned[0];
         if (n > 0xFFFFFFFFULL) {
@@ -936,6 +947,7 @@ int bfs_tt_roots(pb_ctx *ctx, const Board *rb, const uint8_t *rs, const Hash128 
         PB_CUDA(cudaMemcpyAsync(ctx->h_pinned + 1, ctx->d_err, sizeof(u32), cudaMemcpyDeviceToHost, s));
         PB_CUDA(cudaStreamSynchronize(s));
         stats.kernels += 4;
+        stats.launches += 4;
         stats.d2h_bytes += 12;
         if ((u32)ctx->h_pinned[1]) return fail(ctx, PB_ERR_DEVICE, "TT level reported a device error");
         u64 next = ctx->h_pinned[0];
@@ -969,6 +981,7 @@ int bfs_tt_roots(pb_ctx *ctx, const Board *rb, const uint8_t *rs, const Hash128 
                                                                                    nmv, npi, ctx->d_err);
         PB_CUDA(cudaGetLastError());
         stats.kernels += 1;
+        stats.launches += 1;
         emv = nmv;
         epi = npi;
         n = next;
@@ -992,6 +1005,7 @@ int bfs_tt_roots(pb_ctx *ctx, const Board *rb, const uint8_t *rs, const Hash128 
                                  n_par, ctx->dtt.at(2), leafcnt, cursor);
         if (rc2 != PB_OK) return rc2;
         stats.kernels += 1;
+        stats.launches += 1;
     } else if (n > 0) {
         TTView tv = ctx->dtt.at(2);
         unsigned g = grid_for(n, PB_LEAF_THREADS);
@@ -1022,6 +1036,7 @@ int bfs_tt_roots(pb_ctx *ctx, const Board *rb, const uint8_t *rs, const Hash128 
 #undef PB_TT_LEAF
         PB_CUDA(cudaGetLastError());
         stats.kernels += 1;
+        stats.launches += 1;
     }
     if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[2], s));
     // upsweep, deepest level first, then the roots (their counts are not
@@ -1039,6 +1054,7 @@ int bfs_tt_roots(pb_ctx *ctx, const Board *rb, const uint8_t *rs, const Hash128 
         k_resolve_dups<<<g, 256, 0, s>>>(L.flags, L.redirect, L.n, L.vals);
         PB_CUDA(cudaGetLastError());
         stats.kernels += 2;
+        stats.launches += 2;
         child64 = L.vals;
     }
     const TTView none{nullptr, 0, TT_NONE, 0};
@@ -1048,6 +1064,7 @@ int bfs_tt_roots(pb_ctx *ctx, const Board *rb, const uint8_t *rs, const Hash128 
         k_upsweep<u32><<<grid_for(nroots, 256), 256, 0, s>>>(child32, roff, rcnt, rflags, ph, nroots, none, rvals);
     PB_CUDA(cudaGetLastError());
     stats.kernels += 1;
+    stats.launches += 1;
     if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[3], s));
     std::vector<u64> tmp(nroots);
     PB_CUDA(cudaMemcpyAsync(tmp.data(), rvals, sizeof(u64) * nroots, cudaMemcpyDeviceToHost, s));
@@ -1153,13 +1170,14 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         memcpy(ctx->h_stage, rb, sizeof(Board) * n);
         memcpy(ctx->h_stage + at, rs, n);
         PB_CUDA(cudaMemcpyAsync(ctx->arena, ctx->h_stage, at + n, cudaMemcpyHostToDevice, s));
+        stats.h2d_bytes += at + n;
     } else {
         PB_CUDA(cudaMemcpyAsync(b0, rb, sizeof(Board) * n, cudaMemcpyHostToDevice, s));
         PB_CUDA(cudaMemcpyAsync(s0, rs, n, cudaMemcpyHostToDevice, s));
+        stats.h2d_bytes += (sizeof(Board) + 1) * n;
     }
     PB_CUDA(cudaMemsetAsync(rc, 0, sizeof(unsigned long long) * n, s));
     PB_CUDA(cudaMemsetAsync(ctx->d_counter, 0, SCRATCH_BYTES, s));
-    stats.h2d_bytes += (sizeof(Board) + 1 + 4) * n;
     if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[0], s));
     if (depth == 1) {
         if (strict)
@@ -1172,6 +1190,7 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         PB_CUDA(cudaStreamSynchronize(s));
         for (u64 i = 0; i < n; i++) out[i] = tmp[i];
         stats.kernels += 1;
+        stats.launches += 1;
         stats.d2h_bytes += 4 * n;
         return PB_OK;
     }
@@ -1210,6 +1229,7 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
                 iota.resize(n);
                 for (u64 i = 0; i < n; i++) iota[i] = (u32)i;
                 PB_CUDA(cudaMemcpyAsync(r0, iota.data(), sizeof(u32) * n, cudaMemcpyHostToDevice, s));
+                stats.h2d_bytes += sizeof(u32) * n;
                 k_count_positions<WHITE, true><<<grid_for(n, 256), 256, 0, s>>>(b0, s0, n, cnt0);
             } else {
                 cnt = ar.take<u32>(m);
@@ -1221,6 +1241,7 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
                 else
                     k_expand_count_rooted<BLACK><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, m, n_par, cb, cs, cr, cnt, ctx->d_err);
             }
+            stats.launches++;
             if (!launch_scan(ctx, ar, cnt, m, offs)) return too_big();
         }
         PB_CUDA(cudaGetLastError());
@@ -1261,6 +1282,7 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[1], s));
         if (ne) {
             if (depth == 2) {
+                stats.launches++;
                 unsigned g = grid_for(ne, 256);
                 if (c == WHITE) {
                     if (strict) k_leaf1_rooted<WHITE, true><<<g, 256, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc);
@@ -1277,6 +1299,7 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
             } else {
                 unsigned g = grid_for(ne, PB_LEAF_THREADS);
                 const int mode = std::min(leaf_mode(ctx), 2);
+                stats.launches++;
 #define PB_ROOTED_LEAF(CC, SS)                                                                                   \
         if (mode == 2)                                                                                               \
             k_leaf2_rooted<CC, SS, 2><<<g, PB_LEAF_THREADS, 0, s>>>(cur_b, cur_s, cur_r, epi, emv, ne, n_par, rc,    \
@@ -1315,13 +1338,14 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         // a queue was too short: the leaf again, in chunks that always fit
         PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));
         PB_CUDA(cudaMemsetAsync(rc, 0, sizeof(unsigned long long) * n, s));
+        stats.leaf_reruns++;
     }
     if ((u32)ctx->h_pinned[SCRATCH_ERR]) return fail(ctx, PB_ERR_DEVICE, "batched leaf reported a device error");
     if (ne) stats.kernels += 1;
     for (u64 i = 0; i < n; i++) out[i] = tmp[i];
     stats.leaf_edges += ne;
     stats.leaf_positions += ctx->h_pinned[1];
-    stats.d2h_bytes += 8 * n + 20;
+    stats.d2h_bytes += 8 * n + SCRATCH_BYTES;
     if (ctx->timing) {
         float a = 0, b2 = 0;
         PB_CUDA(cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[3]));
@@ -1470,6 +1494,8 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
     PB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(g.rc, 0, sizeof(unsigned long long) * n, s);
     cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s);
+    const u32 launched = ctx->stats.launches;  // counted anew at each run
+    ctx->stats.launches += 4;  // the roots' kernels
     // what fails in between is returned after the capture has ended
     cudaError_t ce = reset_counters(ctx);
     cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), s);
@@ -1491,6 +1517,7 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
     u64 npar_cap = n;
     int c = WHITE;
     for (int k = 1; k < nlev; k++) {
+        ctx->stats.launches += 3;
         u64 cap = g.caps[k - 1];
         unsigned ge = (unsigned)std::min<u64>((cap + 255) / 256, (u64)ctx->num_sms * 16);
         if (c == WHITE)
@@ -1518,6 +1545,8 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
     }
     // leaf over E_nlev
     const u64 lcap = g.caps[nlev - 1];
+    const bool fold = depth > 2 && g.mode == 3 && !g.queue && fold_fits(fold_queue(ctx, ar));
+    if (!fold) ctx->stats.launches += 1;
     if (depth == 2) {
         unsigned gl = (unsigned)std::min<u64>((lcap + 255) / 256, (u64)ctx->num_sms * 16);
         if (g.strict)
@@ -1526,7 +1555,7 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
         else
             k_leaf1_rooted_dev<WHITE, false><<<gl, 256, 0, s>>>(pb_, ps, pr, L[1].pi, L[1].mv, d_n0 + 1, lcap, npar,
                                                                 npar_cap, g.rc, ctx->d_err);
-    } else if (g.mode == 3 && !g.queue && fold_fits(fold_queue(ctx, ar))) {
+    } else if (fold) {
         // a queue too short counts as an outgrown plan
         const LeafEdges e{pb_, ps, pr, L[nlev].pi, L[nlev].mv, lcap, npar_cap, d_n0 + nlev, npar, nullptr, nullptr, nullptr};
         const cudaError_t fe =
@@ -1547,6 +1576,8 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
             launch_leaf_queue<BLACK, false>(g.mode, g.queue, s, ctx->num_sms, pb_, ps, pr, L[nlev].pi, L[nlev].mv, d_n0 + nlev, lcap,
                                             npar, npar_cap, cursor, g.rc, ctx->d_counter, ctx->d_err);
     }
+    g.launches = ctx->stats.launches - launched;
+    ctx->stats.launches = launched;
     if (ce == cudaSuccess) ce = cudaGetLastError();
     const cudaError_t ende = cudaStreamEndCapture(s, &graph);
     if (ce == cudaSuccess) ce = ende;
@@ -1599,6 +1630,7 @@ int run_planned_batch(pb_ctx *ctx, GraphPlan &g, const Board *rb, const uint8_t 
     PB_CUDA(cudaStreamSynchronize(s));
     u32 err = (u32)ctx->h_pinned[2];
     ctx->stats.kernels += 3 * (u32)std::max(depth - 3, 0) + 3 + 1;
+    ctx->stats.launches += g.launches;
     ctx->stats.h2d_bytes += (sizeof(Board) + 1) * n;
     ctx->stats.d2h_bytes += 8 * n + 20;
     if (ctx->timing) {

@@ -362,10 +362,9 @@ __global__ void __launch_bounds__(PB_LEAF_THREADS, PB_LEAF_MIN_BLOCKS)
     }
     if (miss) {
         uint16_t mv[MAX_MOVES];
-        ArraySink sink{mv, 0};
-        gen_moves<1 - C>(b, st, sink);
-        total = grandchild_counts<C, STRICT, MODE >= 2, PB_LEAF_THREADS>(b, st, mv, sink.n);
-        counted = sink.n;
+        counted = in_rounds<1 - C>(b, st, mv, [&](int listed) {
+            total += grandchild_counts<C, STRICT, MODE >= 2, PB_LEAF_THREADS>(b, st, mv, listed);
+        });
         tt_store(tt, h, total);
         out[i] = total;
     }
@@ -473,10 +472,10 @@ __global__ void __launch_bounds__(PB_LEAF_THREADS, PB_LEAF_MIN_BLOCKS)
                     u32 st = pstates[p];
                     make_move<C>(b, st, moves[i]);
                     uint16_t mv[MAX_MOVES];
-                    ArraySink sink{mv, 0};
-                    gen_moves<1 - C>(b, st, sink);
-                    const u32 total = grandchild_counts<C, STRICT, MODE >= 2, T>(b, st, mv, sink.n);
-                    counted += sink.n;
+                    u32 total = 0;
+                    counted += in_rounds<1 - C>(b, st, mv, [&](int listed) {
+                        total += grandchild_counts<C, STRICT, MODE >= 2, T>(b, st, mv, listed);
+                    });
                     tt_store(tt, h, total);
                     out[i] = total;
                 }

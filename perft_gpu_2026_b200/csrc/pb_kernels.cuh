@@ -324,6 +324,29 @@ __global__ void __launch_bounds__(GT) k_generate(const Board *__restrict__ board
 }
 
 // ---------------------------------------------------------------- leaves
+// The moves of `b` (side Z) in rounds of MAX_MOVES from the first'th on: `count`
+// takes each round's number of moves in mv.  One round, but for placements that
+// no game reaches.  Returns the number of all moves.
+struct RoundSink {
+    uint16_t *p;
+    int n;  // of the round; starts at minus the moves before it
+    PB_HD void put(uint16_t m)
+    {
+        if ((u32)n < MAX_MOVES) p[n] = m;
+        n++;
+    }
+};
+template <int Z, class Count>
+__device__ __forceinline__ u32 in_rounds(const Board &b, u32 st, uint16_t *mv, Count count, int first = 0)
+{
+    for (;; first += MAX_MOVES) {
+        RoundSink sink{mv, -first};
+        gen_moves<Z>(b, st, sink);
+        count(min(sink.n, (int)MAX_MOVES));
+        if (sink.n <= MAX_MOVES) return (u32)(first + sink.n);
+    }
+}
+
 // Sum over the moves mv[0..n) of child b of their grandchildren's move counts
 // (each move made on a copy of b, then counted).  With LISTED the counts
 // iterate the child's own-piece lists (ListedPieces, read back through
@@ -403,15 +426,14 @@ __global__ void __launch_bounds__(T, 1024 / T) k_leaf2(const Board *__restrict__
         u32 st = pstates[p];
         make_move<C>(b, st, moves[i]);
         uint16_t mv[MAX_MOVES];
-        ArraySink sink{mv, 0};
-        gen_moves<1 - C>(b, st, sink);
-        for (int k = 0; k < sink.n; k++) {
-            Board g = b;
-            u32 gs = st;
-            make_move<1 - C>(g, gs, mv[k]);
-            total += count_moves<C, STRICT>(g, gs);
-        }
-        counted = sink.n;
+        counted = in_rounds<1 - C>(b, st, mv, [&](int listed) {
+            for (int k = 0; k < listed; k++) {
+                Board g = b;
+                u32 gs = st;
+                make_move<1 - C>(g, gs, mv[k]);
+                total += count_moves<C, STRICT>(g, gs);
+            }
+        });
     }
     total = __reduce_add_sync(0xffffffffu, total);
     counted = __reduce_add_sync(0xffffffffu, counted);
@@ -520,15 +542,14 @@ __global__ void __launch_bounds__(T, 1024 / T) k_leaf2_sorted(const Board *__res
         b = s_b[tid];
         st = s_st[tid];
         uint16_t mv[MAX_MOVES];
-        ArraySink sink{mv, 0};
-        gen_moves<1 - C>(b, st, sink);
-        for (int k = 0; k < sink.n; k++) {
-            Board g = b;
-            u32 gs = st;
-            make_move<1 - C>(g, gs, mv[k]);
-            total += count_moves<C, STRICT>(g, gs);
-        }
-        counted = sink.n;
+        counted = in_rounds<1 - C>(b, st, mv, [&](int listed) {
+            for (int k = 0; k < listed; k++) {
+                Board g = b;
+                u32 gs = st;
+                make_move<1 - C>(g, gs, mv[k]);
+                total += count_moves<C, STRICT>(g, gs);
+            }
+        });
     }
     total = __reduce_add_sync(0xffffffffu, total);
     counted = __reduce_add_sync(0xffffffffu, counted);
@@ -580,10 +601,8 @@ __global__ void __launch_bounds__(T, PB_LISTED_WARPS_PER_SM * 32 / T) k_leaf2_li
         b = s_b[tid];
         st = s_st[tid];
         uint16_t mv[MAX_MOVES];
-        ArraySink sink{mv, 0};
-        gen_moves<1 - C>(b, st, sink);
-        total = grandchild_counts<C, STRICT, true, T>(b, st, mv, sink.n);
-        counted = sink.n;
+        counted = in_rounds<1 - C>(
+            b, st, mv, [&](int listed) { total += grandchild_counts<C, STRICT, true, T>(b, st, mv, listed); });
     }
     total = __reduce_add_sync(0xffffffffu, total);
     counted = __reduce_add_sync(0xffffffffu, counted);
@@ -620,7 +639,7 @@ struct ColumnSink {
     {
         if (n < LEAF_CAP)
             col[n * LEAF_T] = m;
-        else
+        else if (n < MAX_MOVES)
             ovf[n - LEAF_CAP] = m;
         n++;
     }
@@ -658,7 +677,14 @@ __global__ void __launch_bounds__(LEAF_T, 4) k_leaf2_coop(const Board *__restric
             s_cst[tid] = (uint8_t)st;
             ColumnSink sink{s_mv + tid, my_spill, 0};
             gen_moves<1 - C>(b, st, sink);
-            cnt = sink.n;
+            cnt = min(sink.n, (int)MAX_MOVES);
+            if (sink.n > MAX_MOVES) {  // what the table has no room for, here
+                uint16_t mv[MAX_MOVES];
+                in_rounds<1 - C>(
+                    b, st, mv, [&](int listed) { total += grandchild_counts<C, STRICT, false, LEAF_T>(b, st, mv, listed); },
+                    MAX_MOVES);
+                counted += (u32)(sink.n - MAX_MOVES);
+            }
         }
         // ---- block exclusive scan of cnt
         u32 x = (u32)cnt;
@@ -832,10 +858,9 @@ __device__ __forceinline__ void leaf2_rooted_cta(const Board *__restrict__ pboar
     if (MODE >= 1) rank_children<C, PB_LEAF_THREADS>(b, st, root, valid);
     if (valid) {
         uint16_t mv[MAX_MOVES];
-        ArraySink sink{mv, 0};
-        gen_moves<1 - C>(b, st, sink);
-        total = grandchild_counts<C, STRICT, MODE >= 2, PB_LEAF_THREADS>(b, st, mv, sink.n);
-        counted = sink.n;
+        counted = in_rounds<1 - C>(b, st, mv, [&](int listed) {
+            total += grandchild_counts<C, STRICT, MODE >= 2, PB_LEAF_THREADS>(b, st, mv, listed);
+        });
     }
     add_by_key(root_counts, root, total, valid);
     counted = __reduce_add_sync(0xffffffffu, counted);
@@ -1081,10 +1106,9 @@ __global__ void __launch_bounds__(PB_LEAF_THREADS, PB_LEAF_MIN_BLOCKS)
         if (MODE >= 1) rank_children<C, PB_LEAF_THREADS>(b, st, root, valid);
         if (valid) {
             uint16_t mv[MAX_MOVES];
-            ArraySink sink{mv, 0};
-            gen_moves<1 - C>(b, st, sink);
-            total = grandchild_counts<C, STRICT, MODE >= 2, PB_LEAF_THREADS>(b, st, mv, sink.n);
-            counted += sink.n;
+            counted += in_rounds<1 - C>(b, st, mv, [&](int listed) {
+                total += grandchild_counts<C, STRICT, MODE >= 2, PB_LEAF_THREADS>(b, st, mv, listed);
+            });
         }
         add_by_key(root_counts, root, total, valid);
     }
@@ -1147,57 +1171,64 @@ __global__ void __launch_bounds__(T, 1024 / T) k_leaf2_defer(const Board *__rest
     __shared__ uint8_t q_st[T / 32][DEFER_CAP];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u64 i = (u64)blockIdx.x * T + threadIdx.x;
-    u32 total = 0;
-    int nm = 0;
+    u32 total = 0, counted = 0;
     Board b;
     u32 st = 0;
     uint16_t mv[MAX_MOVES];
-    if (i < n && pidx[i] < nparents) {
+    const bool valid = i < n && pidx[i] < nparents;
+    if (valid) {
         u32 p = pidx[i];
         b = load_board(pboards + p);
         st = pstates[p];
         make_move<C>(b, st, moves[i]);
-        ArraySink sink{mv, 0};
-        gen_moves<1 - C>(b, st, sink);
-        nm = sink.n;
     }
-    const u32 counted = (u32)nm;
-    const int kmax = (int)__reduce_max_sync(0xffffffffu, (u32)nm);
     int qn = 0;
-    for (int k = 0; k < kmax; k++) {
-        bool check = false;
-        Board g;
-        u32 gs = 0;
-        CountPrep pr;
-        if (k < nm) {
-            g = b;
-            gs = st;
-            make_move<1 - C>(g, gs, mv[k]);
-            pr = count_prep<C>(g);
-            check = prep_in_check<C>(pr);
-            if (!check) total += count_quiet<C, STRICT>(pr.s, gs, pr.pinned, pr.threat, pr.ksq);
+    for (int first = 0;; first += MAX_MOVES) {  // rounds of the warp's longest list
+        int left = 0;
+        if (valid) {
+            RoundSink sink{mv, -first};
+            gen_moves<1 - C>(b, st, sink);
+            left = sink.n;
         }
-        const unsigned dm = __ballot_sync(0xffffffffu, check);
-        if (dm) {
-            if (check) {
-                const int slot = qn + __popc(dm & ((1u << lane) - 1u));
-                q_b[warp][slot] = g;
-                q_pin[warp][slot] = pr.pinned;
-                q_thr[warp][slot] = pr.threat;
-                q_st[warp][slot] = (uint8_t)gs;
+        const int nm = max(min(left, (int)MAX_MOVES), 0);
+        counted += (u32)nm;
+        const int kmax = (int)__reduce_max_sync(0xffffffffu, (u32)nm);
+        for (int k = 0; k < kmax; k++) {
+            bool check = false;
+            Board g;
+            u32 gs = 0;
+            CountPrep pr;
+            if (k < nm) {
+                g = b;
+                gs = st;
+                make_move<1 - C>(g, gs, mv[k]);
+                pr = count_prep<C>(g);
+                check = prep_in_check<C>(pr);
+                if (!check) total += count_quiet<C, STRICT>(pr.s, gs, pr.pinned, pr.threat, pr.ksq);
             }
-            qn += __popc(dm);
-            __syncwarp();
-            if (qn >= 32) {
-                const int slot = qn - 32 + lane;
-                const Board e = q_b[warp][slot];
-                const Sets es = derive<C>(e);
-                total += count_evasions<C, STRICT>(es, q_st[warp][slot], q_pin[warp][slot], q_thr[warp][slot],
-                                                   bit_index(es.kings & es.us));
-                qn -= 32;
+            const unsigned dm = __ballot_sync(0xffffffffu, check);
+            if (dm) {
+                if (check) {
+                    const int slot = qn + __popc(dm & ((1u << lane) - 1u));
+                    q_b[warp][slot] = g;
+                    q_pin[warp][slot] = pr.pinned;
+                    q_thr[warp][slot] = pr.threat;
+                    q_st[warp][slot] = (uint8_t)gs;
+                }
+                qn += __popc(dm);
                 __syncwarp();
+                if (qn >= 32) {
+                    const int slot = qn - 32 + lane;
+                    const Board e = q_b[warp][slot];
+                    const Sets es = derive<C>(e);
+                    total += count_evasions<C, STRICT>(es, q_st[warp][slot], q_pin[warp][slot], q_thr[warp][slot],
+                                                       bit_index(es.kings & es.us));
+                    qn -= 32;
+                    __syncwarp();
+                }
             }
         }
+        if (!__any_sync(0xffffffffu, left > MAX_MOVES)) break;
     }
     if (lane < qn) {
         const Board e = q_b[warp][lane];

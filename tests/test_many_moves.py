@@ -89,3 +89,28 @@ def test_every_path(use_tt):
         assert eng.perft_batch([p] * 3 + [b] * 3 + [start], 3) == [w3] * 3 + [b3] * 3 + [8902]
         assert eng.perft_batch([b] * 2500, 3) == [b3] * 2500  # more than 8,192 edges: the folded leaf
         assert eng.perft_position(start, 5) == 4865609
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("leaf", [1, 2, 3, 4, 5])
+def test_leaf_kernels_that_list_moves(leaf):
+    """Among other positions, so that warps and CTAs hold both."""
+    b, start = pg.parse_fen(BLACK), pg.parse_fen(pg.START_FEN)
+    b3 = pg.Engine(device=-1).perft_cpu(b, 3)
+    with pg.Engine(device=0, use_tt=False, arena_bytes=1 << 30) as eng:
+        eng.set_tuning(leaf_kernel=leaf)
+        assert eng.perft_position(b, 3) == b3
+        assert eng.perft_batch([b, start] * 200, 3) == [b3, 8902] * 200
+        eng.mlp_init(seed=5, out_bias=[5.5, 11.0, 16.5, 22.0])
+        params = eng.mlp_params()
+        params[:-4] = 0.0
+        eng.mlp_set_params(params)
+        for planned in (1, 2):
+            eng.set_tuning(planned_leaf=planned)
+            got, st = eng.perft_batch_planned([b, start] * 200, 3)
+            assert got == [b3, 8902] * 200 and st.graph_batches == 1 and st.retries == 0
+    for tt_leaf in (1, 2):
+        with pg.Engine(device=0, use_tt=True, arena_bytes=1 << 30, device_tt_mb=512, host_tt_mb=64) as eng:
+            eng.set_tuning(leaf_kernel=leaf, tt_leaf=tt_leaf)
+            for _ in range(2):
+                assert eng.perft_position(b, 3) == b3 and eng.perft_position(start, 5) == 4865609

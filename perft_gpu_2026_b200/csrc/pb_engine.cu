@@ -205,9 +205,6 @@ inline int leaf_mode(const pb_ctx *ctx)
 }
 
 // The folded leaf's queue is what the arena has left behind the levels.
-// Without this much (a few full chunks even at 256 queued moves per edge) the
-// leaf counts every move on the spot (the listed leaf), which needs no memory.
-constexpr u64 FOLD_MIN_ITEMS = 256 * 1024;
 inline FoldQueue fold_queue(const pb_ctx *ctx, const Arena &ar)
 {
     FoldQueue q{};
@@ -215,17 +212,26 @@ inline FoldQueue fold_queue(const pb_ctx *ctx, const Arena &ar)
     q.cursor = ctx->d_counter + 4;
     return q;
 }
-inline bool fold_fits(const FoldQueue &q) { return q.cap >= FOLD_MIN_ITEMS; }
-
 // Edges per chunk: all of them if the queue holds 64 moves per edge (2 to 12
 // are queued on playouts, 24 in endgames of pieces alone), else that many, but
 // at 16 per edge still chunks that fill the GPU.  A chunk whose queue turns
-// out too short makes the leaf run again with `careful`: 256 moves per edge,
-// the size of every move list, always fit.
+// out too short makes the leaf run again with `careful`: 256 moves per edge
+// always fit.
 inline u64 fold_chunk(const FoldQueue &q, u64 n, bool careful)
 {
-    if (careful) return q.cap / MAX_MOVES;
+    if (careful) return std::min(n, q.cap / MAX_MOVES);
     return std::min(n, std::max(q.cap / 64, std::min<u64>(q.cap / 16, 1u << 20)));
+}
+// Chunks much smaller than the GPU cost more than folding saves: below this many
+// edges (unless the leaf has no more) the leaf counts every move on the spot (the
+// listed leaf), which needs no memory. On 27.2 M opening edges chunks of 32 K ran
+// 45.9 ms, of 64 K 20.0, the listed leaf 21.4; on 4.1 M middle-game edges 6.86,
+// 4.24 and 5.79; a leaf run again in chunks of 1,100 to 4,100 edges took 9 to 32
+// times the listed leaf's 1.95 ms.
+constexpr u64 FOLD_MIN_CHUNK = 1u << 16;
+inline bool fold_fits(const FoldQueue &q, u64 n, bool careful)
+{
+    return fold_chunk(q, n, careful) >= std::min(n, FOLD_MIN_CHUNK);
 }
 
 // Below one wave of edges k_fold runs small CTAs, which reach every SM (up to two
@@ -606,8 +612,8 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
     }
     const FoldQueue queue = fold_queue(ctx, ar);
     const bool wide = n_dev || (ctx->tuning.leaf_kernel == 6 && fuse == 2 && n <= WIDE_MAX);
-    const bool fold = ctx->tuning.leaf_kernel == 6 && fuse == 2 && fold_fits(queue);
     for (int attempt = 0;; attempt++) {
+        const bool fold = ctx->tuning.leaf_kernel == 6 && fuse == 2 && fold_fits(queue, n, attempt > 0);
         if (attempt) PB_CUDA(reset_counters(ctx));
         if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[1], s));
         {
@@ -1274,10 +1280,10 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         ne = next;
     }
     const FoldQueue queue = fold_queue(ctx, ar);
-    const bool fold = leaf_mode(ctx) == 3 && depth > 2 && fold_fits(queue);
     std::vector<unsigned long long> many(few ? 0 : n);
     unsigned long long *tmp = few ? reinterpret_cast<unsigned long long *>(ctx->h_stage) : many.data();
     for (int attempt = 0;; attempt++) {
+        const bool fold = leaf_mode(ctx) == 3 && depth > 2 && fold_fits(queue, ne, attempt > 0);
         if (attempt) PB_CUDA(reset_counters(ctx));
         if (ctx->timing) PB_CUDA(cudaEventRecord(ctx->ev[1], s));
         if (ne) {
@@ -1335,7 +1341,7 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         PB_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_counter, SCRATCH_BYTES, cudaMemcpyDeviceToHost, s));
         PB_CUDA(cudaStreamSynchronize(s));
         if ((u32)ctx->h_pinned[SCRATCH_ERR] != DEVERR_QUEUE || attempt > 0) break;
-        // a queue was too short: the leaf again, in chunks that always fit
+        // a queue was too short: the leaf again, in chunks that always fit or listed
         PB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(u32), s));
         PB_CUDA(cudaMemsetAsync(rc, 0, sizeof(unsigned long long) * n, s));
         stats.leaf_reruns++;
@@ -1545,7 +1551,7 @@ int capture_batch_graph(pb_ctx *ctx, GraphPlan &g)
     }
     // leaf over E_nlev
     const u64 lcap = g.caps[nlev - 1];
-    const bool fold = depth > 2 && g.mode == 3 && !g.queue && fold_fits(fold_queue(ctx, ar));
+    const bool fold = depth > 2 && g.mode == 3 && !g.queue && fold_fits(fold_queue(ctx, ar), lcap, false);
     if (!fold) ctx->stats.launches += 1;
     if (depth == 2) {
         unsigned gl = (unsigned)std::min<u64>((lcap + 255) / 256, (u64)ctx->num_sms * 16);

@@ -40,7 +40,7 @@ constexpr int FOLD_THREADS_PER_SM = 768;
 constexpr int FOLD_STAGE = 12;
 constexpr int FOLD_SHELF_BYTES = SHELF_SLOTS * 8;  // dynamic shared memory per thread
 
-enum : u32 { DEVERR_QUEUE = 8u };  // a queue was too short for its chunk: the leaf runs again in smaller chunks
+enum : u32 { DEVERR_QUEUE = 8u };  // a queue was too short for its chunk: the leaf runs again
 
 // The edges of a leaf.  With n_dev the sizes are in device memory (captured
 // graphs): n and nparents are then the planned capacities.

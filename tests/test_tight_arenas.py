@@ -66,3 +66,79 @@ def test_an_arena_of_exact_size_is_enough():
     with pg.Engine(device=0, use_tt=False, arena_bytes=exact_bytes(edges, edges[:-1]) - 65536) as eng:
         assert eng.perft_position(p, 7) == 3195901860
         assert eng.last_stats().levels > 4  # a little less, and it is split
+
+
+ROOKS = "3qk3/8/8/8/8/8/8/QRBNKBRQ w - - 0 1"
+CROWD = "4k3/qqqqqqqq/8/8/8/8/QQQQQQQQ/4K3 w - - 0 1"
+QUEENS = "1k6/ppp5/8/1Q1Q1Q1Q/Q1Q1Q1Q1/1Q1Q1Q1Q/Q1Q1Q1Q1/K7 b - - 0 1"
+
+
+@pytest.mark.parametrize("fen,depth", [(KIWI, 5), (ROOKS, 6)])
+@pytest.mark.parametrize("room_mb", [1, 4, 8.25, 64])
+def test_short_queues_do_not_make_tiny_chunks(fen, depth, room_mb):
+    """An arena with `room_mb` left for the folded leaf's queue: chunks of 64 K
+    edges at least, or the listed leaf."""
+    p = pg.parse_fen(fen)
+    with pg.Engine(device=0, use_tt=False, arena_bytes=2 << 30) as eng:
+        want = eng.perft_position(p, depth)
+        st = eng.last_stats()
+        edges = list(st.level_sizes[:st.levels + 1])
+    with pg.Engine(device=0, use_tt=False, arena_bytes=exact_bytes(edges, edges[:-1]) + int(room_mb * (1 << 20))) as eng:
+        assert eng.perft_position(p, depth) == want
+        st = eng.last_stats()
+        assert list(st.level_sizes[:st.levels + 1]) == edges
+        # levels (twice, where the whole-level kernels' lists left too little
+        # room), chunks, and a leaf counted again
+        assert st.launches <= 2 * 3 * st.levels + 2 * (2 * (edges[-1] // 65536 + 1) + 1)
+
+
+def test_queue_too_short_in_a_single_position():
+    """Room for 16 to 20 queued moves per edge where a sample of them queues 23:
+    the leaf runs again."""
+    p = pg.parse_fen(CROWD)
+    kids = [pg.make_move(p, m) for m in pg.generate_moves(p)]
+    leaves = pg.pack_positions([pg.make_move(k, m) for k in kids for m in pg.generate_moves(k)])
+    _, made, bad = pg.selftest_fold(leaves)
+    queued, n = made // 2, len(leaves)  # both conventions
+    assert bad == 0 and n > 8192 and queued > 21 * n
+    with pg.Engine(device=0, use_tt=False, arena_bytes=1 << 30) as eng:
+        want = eng.perft_position(p, 4)
+        st = eng.last_stats()
+        assert st.leaf_edges == n and st.leaf_reruns == 0
+        counted = st.leaf_positions
+    arena = exact_bytes([len(kids), n], [len(kids)]) + 8 * 18 * n
+    with pg.Engine(device=0, use_tt=False, arena_bytes=arena) as eng:
+        for _ in range(2):
+            assert eng.perft_position(p, 4) == want
+            st = eng.last_stats()
+            assert st.leaf_reruns == 1 and st.leaf_positions == counted
+
+
+@pytest.mark.parametrize("n,arena_mb", [
+    (2000, 3),      # 350 K items for 12,000 edges that queue 57 each: then the listed leaf
+    (175000, 160),  # 17.9 M items for 1.05 M edges: then chunks of 70 K edges that always fit
+])
+def test_queue_too_short_in_a_batch(n, arena_mb):
+    roots = [pg.parse_fen(QUEENS), pg.parse_fen(KIWI)]
+    with pg.Engine(device=0, use_tt=False, arena_bytes=1 << 30) as eng:
+        want = [eng.perft_position(r, 3) for r in roots]
+    batch = pg.pack_positions([roots[0]] * (n - 2) + [roots[1], roots[0]])
+    with pg.Engine(device=0, use_tt=False, arena_bytes=arena_mb << 20) as eng:
+        assert eng.perft_batch(batch, 3) == [want[0]] * (n - 2) + [want[1], want[0]]
+        assert eng.last_stats().leaf_reruns == 1
+
+
+def test_queue_too_short_in_a_planned_batch():
+    """12,000 edges that queue 57 moves each, a planned leaf of 22 K edges at 16
+    to 30: the plan counts as outgrown and the batch runs exactly."""
+    root = pg.parse_fen(QUEENS)
+    with pg.Engine(device=0, use_tt=False, arena_bytes=1 << 30) as eng:
+        want = eng.perft_position(root, 3)
+    with pg.Engine(device=0, use_tt=False, arena_bytes=5 << 20) as eng:
+        eng.mlp_init(seed=5, out_bias=[3.0, 9.0, 13.0, 18.0])
+        params = eng.mlp_params()
+        params[:-4] = 0.0
+        eng.mlp_set_params(params)
+        for _ in range(2):
+            got, st = eng.perft_batch_planned([root] * 2000, 3)
+            assert got == [want] * 2000 and st.graph_batches == 1 and st.retries == 1

@@ -41,7 +41,7 @@ struct Mlp {
     static constexpr size_t WORK_ELEMS = (size_t)tc::MAX_SPLITS * MLP_H * MLP_H;
     __nv_bfloat16 *h1b = nullptr, *dh2b = nullptr;
     PosBytes *pos = nullptr;
-    // The training set of the last mlp_train (positions, feature indices,
+    // The training set of the last mlp_train (a piece of positions, feature indices,
     // targets, order, losses of an epoch's steps), kept for the next one unless
     // larger than TRAIN_KEEP: allocating and freeing it took 0.4 ms per call.
     char *train = nullptr;
@@ -68,7 +68,7 @@ struct Mlp {
     cudaError_t alloc_train(size_t n, size_t steps, TrainSet *set)
     {
         size_t off[6] = {0};
-        const size_t bytes[5] = {n * sizeof(PosBytes), n * MLP_MAX_ACTIVE * sizeof(int16_t),
+        const size_t bytes[5] = {std::min<size_t>(n, FEATURE_PIECE) * sizeof(PosBytes), n * MLP_MAX_ACTIVE * sizeof(int16_t),
                                  n * MLP_OUT * sizeof(float), n * sizeof(int), steps * sizeof(float)};
         for (int k = 0; k < 5; k++) off[k + 1] = off[k] + ((bytes[k] + 255) & ~(size_t)255);
         if (off[5] > train_bytes) {
@@ -115,7 +115,7 @@ struct Mlp {
         PB_MLP_ALLOC(y, (size_t)B * MLP_OUT * 4);
         PB_MLP_ALLOC(dy, (size_t)B * MLP_OUT * 4);
         PB_MLP_ALLOC(t, (size_t)B * MLP_OUT * 4);
-        PB_MLP_ALLOC(pos, (size_t)B * sizeof(PosBytes));
+        PB_MLP_ALLOC(pos, (size_t)std::min(B, FEATURE_PIECE) * sizeof(PosBytes));
 #undef PB_MLP_ALLOC
         max_batch = B;
         return cudaSuccess;
@@ -167,15 +167,25 @@ struct Mlp {
         return cudaGetLastError();
     }
 
-    // Feature indices of n positions into rows [0, n) of `out`, by way of `dev`;
-    // rows up to `rows` get none.
+    // Feature indices of n positions into rows [0, n) of `out`, by way of `dev`
+    // (room for n or FEATURE_PIECE positions) a piece at a time; rows up to `rows`
+    // get none.  The pieces bound the device memory that positions take and keep
+    // the kernel's 32-bit thread index (32 threads a row) in range.
+    static constexpr int FEATURE_PIECE = 1 << 20;
+    static_assert((u64)FEATURE_PIECE * 32 + 256 <= 0xFFFFFFFFu, "thread indices of a piece fit 32 bits");
     cudaError_t features_to(const pb_pos *from, PosBytes *dev, int n, int rows, int16_t *out, cudaStream_t s)
     {
         static_assert(sizeof(pb_pos) == sizeof(PosBytes), "positions are copied as they are");
-        cudaError_t e = cudaMemcpyAsync(dev, from, sizeof(PosBytes) * n, cudaMemcpyHostToDevice, s);
-        if (e != cudaSuccess) return e;
-        k_features<<<(unsigned)(((size_t)rows * 32 + 255) / 256), 256, 0, s>>>(dev, n, rows, out);
-        return cudaGetLastError();
+        for (size_t first = 0; first < (size_t)rows; first += FEATURE_PIECE) {
+            const int r = (int)std::min<size_t>((size_t)rows - first, FEATURE_PIECE);
+            const int k = (int)std::min<size_t>(r, (size_t)n - std::min((size_t)n, first));
+            cudaError_t e = cudaSuccess;
+            if (k) e = cudaMemcpyAsync(dev, from + first, sizeof(PosBytes) * k, cudaMemcpyHostToDevice, s);
+            if (e != cudaSuccess) return e;
+            k_features<<<(unsigned)(((size_t)r * 32 + 255) / 256), 256, 0, s>>>(dev, k, r, out + first * MLP_MAX_ACTIVE);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
+        return cudaSuccess;
     }
 
     // A batch: feature indices and targets by row, the batch's samples by `order`

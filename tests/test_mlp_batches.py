@@ -81,3 +81,21 @@ def test_training_steps_through_the_order(eng):
     # six steps of at most about lr each; orders of summation may flip the sign of a step of a near-zero gradient
     assert np.abs(got - p).max() <= 12 * lr
     assert np.linalg.norm(got - p) <= 0.02 * np.linalg.norm(got - p0)
+
+
+def test_training_sets_of_several_pieces(eng):
+    """Positions go to the device 1 M at a time.  1.5 M samples, the last third
+    other positions than the first two, with the network's own predictions as
+    targets: the loss of an epoch that changes no weight is zero (to the rounding
+    of the predictions' last bits) only if every sample has its own features."""
+    eng.mlp_init(seed=5, out_bias=[4.0, 9.0, 14.0, 19.0])
+    a, b = pg.random_playouts(51, 64, 0, 60, packed=True), pg.random_playouts(52, 64, 0, 60, packed=True)
+    n_a, n_b = (1 << 20) // 64, (1 << 19) // 64
+    pos = (pg.Pos * (64 * (n_a + n_b))).from_buffer_copy(bytes(a) * n_a + bytes(b) * n_b)
+    t = np.concatenate([np.tile(eng.mlp_predict(a), (n_a, 1)), np.tile(eng.mlp_predict(b), (n_b, 1))])
+    apart = float(((eng.mlp_predict(a) - eng.mlp_predict(b)) ** 2).mean())
+    assert apart > 1e-3  # the loss of a third of the samples, had they the others' features
+    assert eng.mlp_train(pos, t, epochs=1, batch=65536, lr=0.0) < 1e-8
+    # one position per sample wrong on purpose, in the last piece
+    t[-1] += 64.0
+    assert abs(eng.mlp_train(pos, t, epochs=1, batch=65536, lr=0.0) - 64.0 ** 2 / len(pos)) < 1e-6

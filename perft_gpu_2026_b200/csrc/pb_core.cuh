@@ -137,6 +137,16 @@ PB_HD int bit_index(u64 single)
 }
 PB_HD bool more_than_one(u64 x) { return (x & (x - 1)) != 0; }
 
+// x as a value the compiler does not recognise, so that what is computed from
+// it is computed again instead of kept in registers across a loop.
+PB_HD u64 fresh(u64 x)
+{
+#ifdef __CUDA_ARCH__
+    asm volatile("" : "+l"(x));
+#endif
+    return x;
+}
+
 PB_HD u64 north(u64 x) { return x << 8; }
 PB_HD u64 south(u64 x) { return x >> 8; }
 PB_HD u64 east1(u64 x) { return (x << 1) & ~FILEA; }

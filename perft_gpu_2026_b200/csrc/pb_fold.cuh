@@ -131,16 +131,6 @@ struct TargetPlanes {
 
 PB_HD u64 beyond(int s, int t) { return ldg64(&PB_TAB.beyond[s][t]); }
 
-// x as a value the compiler does not recognise, so that what is computed from
-// it is computed again instead of kept in registers across the piece loops.
-PB_HD u64 fresh(u64 x)
-{
-#ifdef __CUDA_ARCH__
-    asm volatile("" : "+l"(x));
-#endif
-    return x;
-}
-
 // What Y's unpinned pawns `fp` add to its count, by square: pushes (p1 single,
 // dbl double), captures (cw, cc: squares attacked; on the promotion rank a
 // square counts once unless STRICT).  And what an X piece that leaves f gives

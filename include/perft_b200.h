@@ -193,8 +193,8 @@ typedef struct {
  * ranked by move count first, 5 = as 4 with each child's own-piece squares
  * listed once for all of its grandchild counts, 6 = folded counting: most
  * grandchildren are summed by set arithmetic, the rest made and counted one
- * per thread from a queue in the BFS arena (default; an arena without room for
- * the queue runs 5 instead); batched, planned and table leaves follow 4 to 6;
+ * per thread from a queue in the BFS arena (default; an arena with room
+ * for chunks of fewer than 65,536 edges runs 5 instead); batched, planned and table leaves follow 4 to 6;
  * leaf_blocks_per_sm: persistent grid of the cooperative leaf. */
 typedef struct {
     int leaf_kernel;

@@ -39,9 +39,8 @@ enum {
     MF_QUIET = 0, MF_DOUBLE_PUSH = 1, MF_KING_CASTLE = 2, MF_QUEEN_CASTLE = 3,
     MF_CAPTURE = 4, MF_EP = 5, MF_PROMO = 8
 };
-// Room for a position's moves in the kernels' lists, of which the small levels and
-// the folded leaf take none for granted: 218 is the most a game can reach, but a
-// FEN with two dozen queens has more.
+// Room for a position's moves in a kernel's list.  218 is the most a game can
+// reach; a FEN with two dozen queens has more, and is listed in rounds.
 enum { MAX_MOVES = 256 };
 // More than any position has: a square is entered along eight lines and by eight
 // knights, on the promotion rank by three pawns in four ways each; castling.

@@ -13,9 +13,11 @@
 // benchmark's leaves).
 //
 // Measured on B200 against the leaf that makes and counts every move
-// (balanced, listed pieces; the benchmark's 27.2 M edges, 774 M moves):
+// (children balanced across warps, listed pieces; the benchmark's 27.2 M edges, 774 M moves):
 // 20.09 -> 6.78 ms (k_fold 6.09, k_fold_count 0.69); 5.2 M edges of 6-40 ply
 // playouts 5.33 -> 2.10 ms; 4.2 M edges of 60-140 ply playouts 4.26 -> 1.90 ms.
+// The test for a side left in check and the defined square of a missing king
+// cost 0.3 to 0.9 % of that.
 #pragma once
 #include "pb_fold.cuh"
 #include "pb_kernels.cuh"

@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_leaf2(const Board *__restrict__
 
 namespace pb {
 
-// ---------------------------------------------------------------- balanced leaf
+// ---------------------------------------------------------------- ranked leaf
 // Fused two-ply leaf with the CTA's children handed to threads in order of
 // their move counts.  In k_leaf2 a warp runs as many grandchild iterations as
 // its longest move list, so lanes with short lists idle (about 11 % of the

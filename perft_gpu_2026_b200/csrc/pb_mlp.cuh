@@ -74,9 +74,9 @@ __global__ void __launch_bounds__(256) k_features(const PosBytes *__restrict__ p
 // h1 = relu(b1 + sum of active rows of W1), in the order of the row's indices;
 // BF16 (GEMM operand) and with h1f FP32 (for backward).  64 threads per sample,
 // four columns each, four samples per CTA; a training batch names its samples
-// by `order` (null: sample s is row s).  Bound by the W1 rows read from L1 and
-// L2 (16 KB per position): 2-byte loads of one column per thread ran 21.5 us for
-// 4096 positions, 8-byte loads 9.9 us.
+// by `order` (null: sample s is row s).  Bound by the loads of the W1 rows (16 KB
+// per position; L1 45 % busy, 12 cycles' wait per issue): 2-byte loads of one column
+// per thread ran 21.5 us for 4096 positions, 8-byte loads 9.9 us.
 constexpr int L1_SAMPLES = 4;
 __global__ void __launch_bounds__(64 * L1_SAMPLES)
     k_mlp_layer1(const int16_t *__restrict__ idx, const int *__restrict__ order, const __nv_bfloat16 *__restrict__ w1,
@@ -459,7 +459,7 @@ inline cudaError_t gemm_tc(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 
 // h2 = relu(z2 + b2) and y = b3 + h2 . W3, one warp per sample (two in turn, so
 // that the weights are read once); with targets t (rows by `order`) also h2 in
 // FP32, the loss gradient dy = 2 (y - t) / (n * 4) and the squared error sum,
-// one atomic per CTA.  Bound by reading z2.
+// one atomic per CTA.  Bound by the latency of reading z2 (DRAM 7 %, L2 8 %).
 constexpr int OUT_SAMPLES = 2;  // per warp
 __global__ void __launch_bounds__(256)
     k_mlp_out(const float *__restrict__ z2, const float *__restrict__ b2, const __nv_bfloat16 *__restrict__ w3,
@@ -588,9 +588,11 @@ __global__ void __launch_bounds__(256) k_sum_parts(const float *__restrict__ par
 // dh1 (FP32, from the GEMM) masked by relu'(h1), then scattered into the
 // active rows of dW1 with four-wide FP32 reductions and summed into db1.  64
 // threads per sample, four columns each; a thread keeps its part of db1 over
-// BACK1_SAMPLES samples.  Bound by the reductions in L2 (128 K rows of 1 KB per
-// 4096 samples): one-wide atomics and one db1 atomic per sample and column ran
-// 64 us, this 56 (2.4 TB/s of additions into L2).
+// BACK1_SAMPLES samples.  128 K rows of 1 KB per 4096 samples go to L2: one-wide
+// atomics and one db1 atomic per sample and column ran 64 us, this 56 (2.4 TB/s of
+// additions).  12 % of the warp slots are active, waiting on memory for 42 cycles
+// per issue, with L2 at 22 % of its throughput: latency, of the loads or of the
+// additions to rows that many samples share.
 constexpr int BACK1_SAMPLES = 8;
 __device__ __forceinline__ void red_add4(float *p, const float4 &v)
 {

@@ -5,6 +5,7 @@ that produced them.
     python profile_workloads.py leaf   [--depth 7] [--arena-gb 2] [--reps 3] [--leaf-kernel K] [--leaf-threads T]
     python profile_workloads.py levels [--roots 16384] [--depth 5] [--arena-gb 6]
     python profile_workloads.py tt     [--depth 8] [--dtt-mb 2000] [--arena-gb 2]
+    python profile_workloads.py train  [--n 8192] [--batch 4096] [--reps 2]
     python profile_workloads.py gemm   [--m 4096] [--n 256] [--k 256] [--ta 0] [--tb 0] [--reps 20]
 
 leaf    the bench position (4 random plies from the initial array, splitmix64
@@ -20,6 +21,8 @@ levels  one batched perft over --roots playout positions (0..60 plies, seed
 tt      the start position with device tables: perft depth-1 (fills the
         tables), then perft depth (the launch to capture: skip the first
         table-leaf launch).  Counts are checked against the known totals.
+train   the scheduler network: --reps training calls of one epoch over --n
+        playouts (0..60 plies, seed 3), then a prediction of them.
 gemm    the scheduler network's tcgen05 GEMM on random BF16 operands: one
         checked launch, then --reps timed launches (CUDA events); prints the
         mean time and TFLOP/s.  The network's three products at a 4096-sample
@@ -90,6 +93,20 @@ def tt(args):
     eng.close()
 
 
+def train(args):
+    import numpy as np
+
+    pos = pg.random_playouts(3, args.n, 0, 60, packed=True)
+    t = np.random.default_rng(3).uniform(0, 20, size=(args.n, 4)).astype(np.float32)
+    eng = pg.Engine(device=0, use_tt=False, arena_bytes=1 << 28)
+    eng.mlp_init(seed=1, out_bias=[4.5, 9.0, 13.5, 18.0])
+    for _ in range(args.reps):
+        loss = eng.mlp_train(pos, t, epochs=1, batch=args.batch)
+    y = eng.mlp_predict(pos)
+    print(json.dumps({"workload": "train", "n": args.n, "batch": args.batch, "loss": loss, "mean": float(y.mean())}))
+    eng.close()
+
+
 def gemm(args):
     import numpy as np
 
@@ -128,6 +145,10 @@ def main(argv=None):
     a.add_argument("--depth", type=int, default=8)
     a.add_argument("--dtt-mb", type=int, default=2000)
     a.add_argument("--arena-gb", type=int, default=2)
+    a = sub.add_parser("train")
+    a.add_argument("--n", type=int, default=8192)
+    a.add_argument("--batch", type=int, default=4096)
+    a.add_argument("--reps", type=int, default=2)
     a = sub.add_parser("gemm")
     a.add_argument("--m", type=int, default=4096)
     a.add_argument("--n", type=int, default=256)
@@ -136,7 +157,7 @@ def main(argv=None):
     a.add_argument("--tb", type=int, default=0)
     a.add_argument("--reps", type=int, default=20)
     args = ap.parse_args(argv)
-    {"leaf": leaf, "levels": levels, "tt": tt, "gemm": gemm}[args.which](args)
+    {"leaf": leaf, "levels": levels, "tt": tt, "train": train, "gemm": gemm}[args.which](args)
     return 0
 
 

@@ -175,14 +175,11 @@ typedef struct {
     uint64_t leaf_positions;   /* positions the leaf kernel counted (move-count calls) */
     uint64_t nodes;            /* the perft result of the call */
     uint32_t kernels;          /* steps of the call: three per BFS level and one per leaf, however few or
-                                  many kernels a level or leaf took (`launches` counts those) */
+                                  many kernels a level or leaf took (pb_last_launches) */
     uint32_t levels;           /* BFS expand levels */
     uint64_t level_sizes[16];  /* edges per level, level 0 = root moves */
     uint64_t h2d_bytes;        /* host-to-device bytes copied */
     uint64_t d2h_bytes;        /* device-to-host bytes copied */
-    uint32_t launches;         /* kernels launched, those of captured graphs included (without the
-                                  planner's network) */
-    uint32_t leaf_reruns;      /* leaves counted again because a queue was too short */
 } pb_stats;
 
 /* Launch parameters of the GPU path (no reference counterpart: the
@@ -226,6 +223,11 @@ int pb_get_tuning(const pb_ctx *ctx, pb_tuning *t);
 /* Turns per-call event timing on or off (off by default). */
 int pb_set_timing(pb_ctx *ctx, int enable);
 int pb_last_stats(const pb_ctx *ctx, pb_stats *out);
+
+/* Of the same call: kernels launched, those of captured graphs included
+ * (without the planner's network), and leaves counted again because a queue
+ * was too short.  Either pointer may be null. */
+int pb_last_launches(const pb_ctx *ctx, uint32_t *launches, uint32_t *leaf_reruns);
 
 /* n playouts at once (threads): position i uses the generator state drawn
  * i-th from a splitmix64 stream seeded with `seed`; from that state it draws

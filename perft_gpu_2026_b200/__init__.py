@@ -79,9 +79,9 @@ class Stats(ctypes.Structure):
         ("level_sizes", ctypes.c_uint64 * 16),
         ("h2d_bytes", ctypes.c_uint64),
         ("d2h_bytes", ctypes.c_uint64),
-        ("launches", ctypes.c_uint32),
-        ("leaf_reruns", ctypes.c_uint32),
     ]
+    launches = 0  # of pb_last_launches
+    leaf_reruns = 0
 
 
 class Tuning(ctypes.Structure):
@@ -146,6 +146,7 @@ def _load() -> ctypes.CDLL:
         "pb_set_tuning": (ctypes.c_int, [ctypes.c_void_p, P(Tuning)]),
         "pb_get_tuning": (ctypes.c_int, [ctypes.c_void_p, P(Tuning)]),
         "pb_last_stats": (ctypes.c_int, [ctypes.c_void_p, P(Stats)]),
+        "pb_last_launches": (ctypes.c_int, [ctypes.c_void_p, P(ctypes.c_uint32), P(ctypes.c_uint32)]),
         "pb_mlp_param_count": (ctypes.c_size_t, []),
         "pb_mlp_init": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint64, P(ctypes.c_float)]),
         "pb_mlp_get_params": (ctypes.c_int, [ctypes.c_void_p, P(ctypes.c_float), ctypes.c_size_t]),
@@ -526,6 +527,9 @@ class Engine:
     def last_stats(self) -> Stats:
         st = Stats()
         self._check(lib.pb_last_stats(self._h, ctypes.byref(st)))
+        launches, reruns = ctypes.c_uint32(), ctypes.c_uint32()
+        self._check(lib.pb_last_launches(self._h, ctypes.byref(launches), ctypes.byref(reruns)))
+        st.launches, st.leaf_reruns = launches.value, reruns.value
         return st
 
     def prepare(self, p: Pos, max_depth: int) -> int:

@@ -69,6 +69,11 @@ constexpr int SCRATCH_ERR = 8;
 constexpr int WIDE_LEVELS = 7;
 constexpr size_t STAGE_BYTES = 512 * 1024;  // uploads and readbacks of calls with few roots
 
+// pb_stats, whose layout callers are compiled with, and what came later.
+struct CallStats : pb_stats {
+    uint32_t launches = 0, leaf_reruns = 0;
+};
+
 struct pb_ctx {
     int device = -1;
     bool gpu = false;
@@ -90,7 +95,7 @@ struct pb_ctx {
     uint16_t *spill = nullptr;  // cooperative-leaf spill area, behind the arena in its allocation
     size_t spill_blocks = 0;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // call start, leaf start, leaf end, call end
-    pb_stats stats{};
+    CallStats stats{};
     HostTT htt;
     DeviceTT dtt;
     Mlp mlp;
@@ -516,7 +521,7 @@ int bfs_perft_pass(pb_ctx *ctx, const Board &root, u32 root_st, int color, int d
         return PB_OK;
     }
     cudaStream_t s = ctx->stream;
-    pb_stats &stats = ctx->stats;
+    CallStats &stats = ctx->stats;
     Arena ar{ctx->arena, ctx->arena_bytes};
     Board *pb_ = ar.take<Board>(1);
     uint8_t *ps = ar.take<uint8_t>(1);
@@ -818,7 +823,7 @@ int bfs_tt_roots(pb_ctx *ctx, const Board *rb, const uint8_t *rs, const Hash128 
     int rc = ensure_dtt(ctx, depth - 1);
     if (rc != PB_OK) return rc;
     cudaStream_t s = ctx->stream;
-    pb_stats &stats = ctx->stats;
+    CallStats &stats = ctx->stats;
     Arena ar{ctx->arena, ctx->arena_bytes};
     Board *pb_ = ar.take<Board>(nroots);
     uint8_t *ps = ar.take<uint8_t>(nroots);
@@ -1161,7 +1166,7 @@ int bfs_batch_pass(pb_ctx *ctx, const Board *rb, const uint8_t *rs, u64 n, int d
         return PB_OK;
     };
     cudaStream_t s = ctx->stream;
-    pb_stats &stats = ctx->stats;
+    CallStats &stats = ctx->stats;
     Arena ar{ctx->arena, ctx->arena_bytes};
     Board *b0 = ar.take<Board>(n);
     uint8_t *s0 = ar.take<uint8_t>(n);
@@ -2424,7 +2429,7 @@ int pb_perft_position(pb_ctx *ctx, const pb_pos *pos, int depth, uint64_t *count
     if (!ctx || !pos || !count || depth < 0 || depth > 20) return PB_ERR_ARG;
     if (!ctx->gpu) return fail(ctx, PB_ERR_NODEVICE, "context has no GPU");
     PB_CUDA(cudaSetDevice(ctx->device));
-    memset(&ctx->stats, 0, sizeof(ctx->stats));
+    ctx->stats = CallStats{};
     int rc = gpu_perft(ctx, to_board(*pos), pos->state, pos->color, depth, reinterpret_cast<u64 *>(count));
     ctx->stats.nodes = *count;
     return rc;
@@ -2493,6 +2498,14 @@ int pb_get_tuning(const pb_ctx *ctx, pb_tuning *t)
 {
     if (!ctx || !t) return PB_ERR_ARG;
     *t = ctx->tuning;
+    return PB_OK;
+}
+
+int pb_last_launches(const pb_ctx *ctx, uint32_t *launches, uint32_t *leaf_reruns)
+{
+    if (!ctx) return PB_ERR_ARG;
+    if (launches) *launches = ctx->stats.launches;
+    if (leaf_reruns) *leaf_reruns = ctx->stats.leaf_reruns;
     return PB_OK;
 }
 
@@ -2630,7 +2643,7 @@ int pb_perft_batch(pb_ctx *ctx, const pb_pos *roots, const int *depths, int n, u
     if (!ctx || !roots || !depths || !counts || n < 0) return PB_ERR_ARG;
     if (!ctx->gpu) return fail(ctx, PB_ERR_NODEVICE, "context has no GPU");
     PB_CUDA(cudaSetDevice(ctx->device));
-    memset(&ctx->stats, 0, sizeof(ctx->stats));
+    ctx->stats = CallStats{};
     // all at one depth: in the caller's order, counts straight to the caller
     if (n > 0 && std::all_of(depths, depths + n, [&](int d) { return d == depths[0]; })) {
         if (depths[0] < 0 || depths[0] > 20) return PB_ERR_ARG;
@@ -3043,7 +3056,7 @@ int pb_perft_batch_planned(pb_ctx *ctx, const pb_pos *roots, const int *depths, 
     for (int i = 0; i < n; i++)
         if (depths[i] < 0 || depths[i] > 12) return PB_ERR_ARG;
     PB_CUDA(cudaSetDevice(ctx->device));
-    memset(&ctx->stats, 0, sizeof(ctx->stats));
+    ctx->stats = CallStats{};
     if (stats) memset(stats, 0, sizeof(*stats));
     int rc = plan_and_run(ctx, roots, depths, n, counts, stats);
     for (int i = 0; i < n && rc == PB_OK; i++) ctx->stats.nodes += counts[i];
